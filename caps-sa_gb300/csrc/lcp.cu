@@ -1,5 +1,4 @@
-// lcp.cu — LCP-based kernels: LCP arrays, batched LcpDispatch::lcp /
-// suffix_cmp_with, the bounded-context run flags, and the merge-path
+// lcp.cu — LCP-based kernels: batched LcpDispatch::lcp / suffix_cmp_with, the bounded-context run flags, and the merge-path
 // version of the reference's LCP-enhanced two-way merge.
 #include <algorithm>
 
@@ -37,26 +36,6 @@ __device__ int thread_suffix_cmp(const void *text, int sym, const DevLimits &L, 
         return (a > b) - (a < b);
     }
     return dev_boundary_order(L, p, lp, q, lq);
-}
-
-template <typename OT>
-__global__ void __launch_bounds__(kWarpBlock)
-    lcp_array_kernel(const void *__restrict__ text, int sym, DevLimits L, uint64_t max_ctx,
-                     const uint32_t *__restrict__ sa, uint64_t m, OT *__restrict__ out) {
-    const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
-    const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    const uint32_t lane = threadIdx.x & 31;
-    for (uint64_t i = warp; i < m; i += nwarps) {
-        uint64_t r = 0;
-        if (i > 0) {
-            uint64_t a = sa[i - 1], b = sa[i];
-            uint64_t cap = min(dev_lim_at(L, a), dev_lim_at(L, b));
-            if (max_ctx < cap) cap = max_ctx;
-            const uint64_t k = (uint64_t)sym;
-            r = warp_lcp_bytes((const uint8_t *)text, a * k, b * k, cap * k) / k;
-        }
-        if (lane == 0) out[i] = (OT)r;
-    }
 }
 
 __global__ void __launch_bounds__(kWarpBlock)
@@ -305,21 +284,6 @@ unsigned warp_grid(Ctx &c, uint64_t items) {
 }
 
 }  // namespace
-
-capssa_status lcp_array_sa(Ctx &c, const void *text, int sym_bytes, uint64_t n,
-                           const DevLimits &L, uint64_t max_ctx, const uint32_t *sa, uint64_t m,
-                           void *out_lcp, int out_bytes) {
-    (void)n;
-    if (m == 0) return CAPSSA_OK;
-    if (out_bytes == 4)
-        lcp_array_kernel<uint32_t><<<warp_grid(c, m), kWarpBlock, 0, c.stream>>>(
-            text, sym_bytes, L, max_ctx, sa, m, (uint32_t *)out_lcp);
-    else
-        lcp_array_kernel<uint64_t><<<warp_grid(c, m), kWarpBlock, 0, c.stream>>>(
-            text, sym_bytes, L, max_ctx, sa, m, (uint64_t *)out_lcp);
-    CAPSSA_LAUNCHED(c);
-    return CAPSSA_OK;
-}
 
 capssa_status lcp_pairs(Ctx &c, const void *text, int sym_bytes, uint64_t n, const uint64_t *p,
                         const uint64_t *q, uint64_t count, uint64_t max_ctx, uint64_t *out) {

@@ -104,9 +104,6 @@ __device__ __forceinline__ uint64_t warp_sym_lcp(const void *text, int sym_bytes
 }
 
 // Host-side entry points implemented in lcp.cu.
-capssa_status lcp_array_sa(Ctx &c, const void *text, int sym_bytes, uint64_t n,
-                           const DevLimits &L, uint64_t max_ctx, const uint32_t *sa, uint64_t m,
-                           void *out_lcp, int out_bytes);
 capssa_status lcp_pairs(Ctx &c, const void *text, int sym_bytes, uint64_t n, const uint64_t *p,
                         const uint64_t *q, uint64_t count, uint64_t max_ctx, uint64_t *out);
 capssa_status suffix_cmp_pairs(Ctx &c, const void *text, int sym_bytes, const DevLimits &L,

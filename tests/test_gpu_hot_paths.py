@@ -44,3 +44,35 @@ def test_batched_positions_local_to_their_text(ctx, shape, index):
     out = torch.empty(len(cat) + 1, dtype=dt, device="cuda")[1:]
     ctx.build_batched(cat, offs, out=out)
     assert np.array_equal(out.cpu().numpy().view(index), got)
+
+
+# ---------------------------------------------------------------- LCP array
+
+@pytest.mark.parametrize("dtype,sigma", [(np.uint8, 2), (np.uint8, 4), (np.uint8, 6),
+                                         (np.uint8, 100), (np.uint16, 3000),
+                                         (np.uint32, 1 << 20)])
+@pytest.mark.parametrize("max_ctx", [orc.UNBOUNDED, 511, 513])
+def test_lcp_array_short_long_and_bounded(ctx, dtype, sigma, max_ctx):
+    """Neighbours that part inside the first windows, after the four bursts a
+    thread reads alone, and after several warp-wide steps; repeats that reach
+    the text's end, segment ends, and context bounds inside a window.  The
+    whole text and a subset sorted on its own."""
+    rng = np.random.default_rng(sigma % 1000)
+    n = 60011
+    t = rng.integers(0, sigma, n).astype(dtype)
+    t[30000:50000] = t[5000:25000]      # one long repeat
+    t[n - 700:] = t[100:800]            # one that the text's end cuts
+    t[26000:26400] = t[0]               # a run
+    ends = np.array([9000, 9001, 21003, 40000, n])
+    for lp, lo in ((capssa.PlainText(n), orc.Limits(n)),
+                   (capssa.SegmentedText(n, ends, capssa.BoundaryRank.LONGER_FIRST),
+                    orc.Limits(n, ends, True))):
+        opts = capssa.Opts(max_context=max_ctx)
+        sa, lcp = ctx.build_in_memory_lcp(t, None, lp, opts)
+        wsa, wlcp = orc.build_in_memory(t, None, lo, max_ctx, with_lcp=True)
+        assert np.array_equal(sa, wsa) and np.array_equal(lcp, wlcp)
+        pos = np.unique(np.concatenate([rng.integers(0, n, 2000), np.arange(30000, 33000),
+                                        np.arange(5000, 7000), [n]])).astype(np.uint64)
+        sa, lcp = ctx.build_in_memory_lcp(t, pos, lp, opts, index=np.uint64)
+        wsa, wlcp = orc.build_in_memory(t, pos, lo, max_ctx, index=np.uint64, with_lcp=True)
+        assert np.array_equal(sa, wsa) and np.array_equal(lcp, wlcp)
