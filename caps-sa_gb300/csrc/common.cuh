@@ -150,7 +150,7 @@ struct Ctx {
     uint64_t launches = 0;
     // side streams: the independent kernels of one refinement round run
     // concurrently, forked from and joined back to `stream` by events
-    static constexpr int kSide = 4;
+    static constexpr int kSide = 5;
     cudaStream_t side[kSide] = {};
     cudaEvent_t fork_ev = nullptr;
     cudaEvent_t join_ev[kSide] = {};

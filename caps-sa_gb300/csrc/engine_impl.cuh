@@ -1696,115 +1696,293 @@ __global__ void direct_warp_kernel(const uint4 *__restrict__ groups, uint32_t co
     }
 }
 
-// One block sorts one medium tied group (17..kMediumMax members, all
-// agreeing on h symbols) with a bitonic network over direct comparisons,
-// then splits it into subgroups like direct_warp_kernel.
-constexpr int kMedThreads = 256;
+// Tied groups of kLo + 1 .. MAXM members (33 .. kMediumMax over the two
+// instantiations): one block per group, window by window.  Each step reads
+// the next window of every member still tied (one round trip for the group:
+// bound by those random L2 reads), orders each tied subgroup by it inside
+// shared memory, and splits the subgroups where windows differ; a window that
+// every subgroup agrees on costs no ordering.  A suffix that ends inside its
+// window is padded low (ShorterFirst) or high (LongerFirst) and ordered by
+// the symbols it still had, as the key records are.  The group leaves once it
+// is settled, or when its subgroups agree on twice the round's depth (what
+// rank doubling needs), and the subgroups then queue by their own size.
+// Ordering: by counting inside 32 slots, then merges of doubling runs by
+// binary search, in which only subgroups that span both runs take part (a
+// bitonic network over the same windows: 20 ms where the large instantiation now
+// takes 2.3 ms, all rounds of the text below).
+// Groups of up to 256 members, nearly all of them, run 128 threads and 9 KB
+// of shared memory, so many share an SM.  The bitonic network over direct text
+// comparisons that stood here before read the text again at each of its
+// log2(m)^2 / 2 compare steps: round 1 of a 50 M-symbol word text (134,949
+// groups, 8-symbol keys) took 26.4 ms, 5.8 ms now with the smaller groups.
+constexpr uint32_t kMedSmall = 256;  // members the small instantiation holds
 
-__global__ void __launch_bounds__(kMedThreads)
+template <uint32_t kLo, uint32_t MAXM, int THREADS>
+__global__ void __launch_bounds__(THREADS)
     direct_medium_kernel(const uint4 *__restrict__ groups, uint32_t count,
                          uint32_t *__restrict__ sa, uint32_t *__restrict__ hd,
                          uint32_t *__restrict__ rank, DevLimits L, Packed P, int lf,
-                         GroupLists G, int nxt) {
-    __shared__ uint32_t spos[kMediumMax];
-    __shared__ uint64_t slim[kMediumMax];
-    __shared__ int8_t rel[kMediumMax];
-    __shared__ uint32_t shead[kMediumMax];
-    __shared__ uint32_t wmax[kMedThreads / 32];
+                         uint64_t round_h, GroupLists G, int nxt) {
+    constexpr int kPer = (int)(MAXM / THREADS);
+    static_assert(MAXM % THREADS == 0 && MAXM <= 2048, "slots per thread; lengths below 2^12");
+    // subgroups to append, (start, length | depth << 12): the small
+    // instantiation gathers those of several groups, the large one flushes
+    // after every group and keeps them where the windows were
+    constexpr bool kGather = MAXM <= kMedSmall;
+    constexpr uint32_t kQueue = kGather ? MAXM / 2 + MAXM : MAXM / 2;
+    __shared__ uint64_t sw[MAXM];    // the step's window
+    __shared__ uint32_t spos[MAXM];  // member in slot i
+    __shared__ uint32_t slim[MAXM];  // its limit
+    __shared__ uint16_t shead[MAXM]; // first slot of i's subgroup
+    __shared__ uint16_t send[MAXM];  // at a subgroup's first slot: one past its last
+    __shared__ uint8_t st[MAXM];     // symbols left in the window, as an ordering key
+    __shared__ uint8_t sact[MAXM];   // slot i's subgroup is still tied
+    __shared__ uint32_t s_wmax[THREADS / 32];
+    __shared__ uint2 s_own[kGather ? kQueue : 1];
+    uint2 *s_q = kGather ? s_own : reinterpret_cast<uint2 *>(sw);
+    __shared__ uint32_t s_qn, s_cnt[kLists], s_base[kLists];
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t spw = (uint32_t)P.spw;
+    const uint32_t full = lf ? 0u : spw;  // st of a member with a whole window
+    // order of two members with equal windows: symbols left, then for ended
+    // ones the limit (in the boundary order), then position
+    auto ends_before = [&](uint32_t ta, uint32_t la, uint32_t pa, uint32_t tb, uint32_t lb,
+                           uint32_t pb) {
+        if (ta != tb) return ta < tb;
+        if (ta != full && la != lb) return lf ? la > lb : la < lb;
+        return pa < pb;
+    };
+    if (tid == 0) s_qn = 0;
+    __syncthreads();
+    // staged subgroups into the next round's lists, one atomic per list
+    auto flush = [&]() {
+        __syncthreads();
+        const uint32_t nq = s_qn;
+        if (tid < kLists) s_cnt[tid] = 0;
+        __syncthreads();
+        constexpr int kQPer = (int)((kQueue + THREADS - 1) / THREADS);
+        uint32_t at[kQPer];
+#pragma unroll
+        for (int j = 0; j < kQPer; j++) {
+            const uint32_t q = j * THREADS + tid;
+            if (q < nq) {
+                const int l = list_of(s_q[q].y & 0xFFFu, s_q[q].y >> 12);
+                if (l < kLists) at[j] = atomicAdd(&s_cnt[l], 1u);
+            }
+        }
+        __syncthreads();
+        if (tid < kLists && s_cnt[tid]) s_base[tid] = atomicAdd(&G.ctr->n[tid][nxt], s_cnt[tid]);
+        if (tid == 0) s_qn = 0;
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < kQPer; j++) {
+            const uint32_t q = j * THREADS + tid;
+            if (q < nq) {
+                const uint32_t start = s_q[q].x, n2 = s_q[q].y & 0xFFFu, dep = s_q[q].y >> 12;
+                const int l = list_of(n2, dep);
+                if (l < kLists)
+                    list_ptr(G, l, nxt)[s_base[l] + at[j]] = group_entry(start, n2, dep);
+                else
+                    append_big(G, nxt, start, n2, dep);
+            }
+        }
+        __syncthreads();
+    };
     for (uint32_t gi = blockIdx.x; gi < count; gi += gridDim.x) {
         const uint4 g = groups[gi];
         const uint32_t len = g.y;
+        if (len <= kLo || len > MAXM) continue;  // the other instantiation's
         const uint64_t h = g.z;
-        const uint64_t cap = h > kDirectCap ? h : kDirectCap;
-        uint32_t p2 = 1;
-        while (p2 < len) p2 <<= 1;
-        for (uint32_t t = tid; t < p2; t += kMedThreads) {
-            if (t < len) {
-                uint32_t p = sa[g.x + t];
-                spos[t] = p;
-                slim[t] = dev_lim_at(L, p);
-            } else {
-                spos[t] = 0xFFFFFFFFu;  // padding sorts last
-                slim[t] = 0;
+        const uint64_t target = 2 * (h > round_h ? h : round_h);
+        uint64_t d = h;
+#pragma unroll
+        for (int j = 0; j < kPer; j++) {
+            const uint32_t i = j * THREADS + tid;
+            if (i < len) {
+                const uint32_t p = sa[g.x + i];
+                spos[i] = p;
+                slim[i] = (uint32_t)dev_lim_at(L, p);
+                shead[i] = 0;
+                sact[i] = 1;
             }
         }
+        if (tid == 0) send[0] = (uint16_t)len;
         __syncthreads();
-        for (uint32_t kk = 2; kk <= p2; kk <<= 1) {
-            for (uint32_t j = kk >> 1; j > 0; j >>= 1) {
-                for (uint32_t i = tid; i < p2; i += kMedThreads) {
-                    uint32_t ixj = i ^ j;
-                    if (ixj <= i) continue;
-                    uint32_t pa = spos[i], pb = spos[ixj];
-                    bool a_after;
-                    if (pa == 0xFFFFFFFFu || pb == 0xFFFFFFFFu) {
-                        a_after = pa == 0xFFFFFFFFu && pb != 0xFFFFFFFFu;
-                    } else {
-                        int r = direct_cmp(P, pa, slim[i], pb, slim[ixj], h, cap, lf);
-                        a_after = r == 1 || ((r == 0 || r == 2) && pa > pb);
+        for (;;) {
+            // the next window of every tied member
+            bool differ = false;
+#pragma unroll
+            for (int j = 0; j < kPer; j++) {
+                const uint32_t i = j * THREADS + tid;
+                if (i < len) {
+                    uint64_t w = 0;
+                    uint32_t t = 0;
+                    if (sact[i]) {
+                        // a limit below d: equal ranks past the shared prefix can
+                        // join suffixes that end together before the group's depth
+                        const uint64_t rest = slim[i] > d ? slim[i] - d : 0;
+                        if (rest) w = window_at(P, (uint64_t)spos[i] + d);
+                        t = rest < spw ? (uint32_t)rest : spw;
+                        if (t < spw) {
+                            const uint64_t low = P.mask & (~0ull >> (t * (uint32_t)P.b));
+                            w = lf ? (w | low) : (w & ~low);
+                        }
+                        if (lf) t = spw - t;
                     }
-                    bool up = (i & kk) == 0;
-                    if (up == a_after) {
-                        spos[i] = pb;
-                        spos[ixj] = pa;
-                        uint64_t tl = slim[i];
-                        slim[i] = slim[ixj];
-                        slim[ixj] = tl;
+                    sw[i] = w;
+                    st[i] = (uint8_t)t;
+                }
+            }
+            __syncthreads();
+#pragma unroll
+            for (int j = 0; j < kPer; j++) {
+                const uint32_t i = j * THREADS + tid;
+                if (i < len && sact[i]) {
+                    const uint32_t hs = shead[i];
+                    differ |= sw[i] != sw[hs] || st[i] != full;
+                }
+            }
+            const int any = __syncthreads_or(differ ? 1 : 0);
+            d += spw;
+            if (any) {
+                // every subgroup ordered in place: by counting inside blocks of 32
+                // slots, then by merges of doubling runs (a member's new slot is
+                // its old one shifted by a binary search in the sibling run);
+                // `run` 0 is the counting step
+                for (uint32_t run = 0; run < len; run = run ? run * 2 : 32) {
+                    uint32_t to[kPer], mp[kPer], ml[kPer];
+                    uint64_t mw[kPer];
+                    uint8_t mt[kPer];
+                    bool moved = false;
+#pragma unroll
+                    for (int j = 0; j < kPer; j++) {
+                        const uint32_t i = j * THREADS + tid;
+                        to[j] = i;
+                        if (i < len && sact[i]) {
+                            const uint32_t hs = shead[i], he = send[hs];
+                            mw[j] = sw[i];
+                            mt[j] = st[i];
+                            mp[j] = spos[i];
+                            ml[j] = slim[i];
+                            auto before = [&](uint32_t u) {  // slot u's member goes first
+                                const uint64_t wu = sw[u];
+                                return wu < mw[j] ||
+                                       (wu == mw[j] && ends_before(st[u], slim[u], spos[u], mt[j],
+                                                                   ml[j], mp[j]));
+                            };
+                            if (run == 0) {
+                                const uint32_t lo = max(hs, i & ~31u), hi = min(he, (i | 31u) + 1);
+                                uint32_t r = lo;
+                                for (uint32_t u = lo; u < hi; u++) r += before(u) ? 1u : 0u;
+                                to[j] = r;
+                            } else {
+                                const uint32_t p0 = i & ~(2 * run - 1), mid = p0 + run;
+                                if (hs < mid && mid < he) {  // the subgroup spans both runs
+                                    const bool left = i < mid;
+                                    const uint32_t first = left ? mid : max(hs, p0);
+                                    uint32_t lo = first, hi = left ? min(he, mid + run) : mid;
+                                    const uint32_t end = hi;
+                                    while (lo < hi) {
+                                        const uint32_t m = (lo + hi) >> 1;
+                                        if (before(m))
+                                            lo = m + 1;
+                                        else
+                                            hi = m;
+                                    }
+                                    to[j] = left ? i + (lo - first) : i - (end - lo);
+                                }
+                            }
+                            moved |= to[j] != i;
+                        }
                     }
+                    if (!__syncthreads_or(moved ? 1 : 0)) continue;
+#pragma unroll
+                    for (int j = 0; j < kPer; j++) {
+                        if (to[j] != (uint32_t)j * THREADS + tid) {
+                            sw[to[j]] = mw[j];
+                            st[to[j]] = mt[j];
+                            spos[to[j]] = mp[j];
+                            slim[to[j]] = ml[j];
+                        }
+                    }
+                    __syncthreads();
+                }
+                // subgroup heads: a slot starts one when it did before, when its
+                // (window, symbols left) differ from the slot before, or when it
+                // ended there under LongerFirst (equal ends order by position)
+                uint32_t loc[kPer], run = 0;
+                const uint32_t base = tid * kPer;
+#pragma unroll
+                for (int q = 0; q < kPer; q++) {
+                    const uint32_t i = base + q;
+                    if (i < len) {
+                        bool start = shead[i] == i;
+                        if (!start && sact[i])
+                            start = sw[i] != sw[i - 1] || st[i] != st[i - 1] ||
+                                    (st[i] != full && (lf || slim[i] != slim[i - 1]));
+                        if (start) run = i;
+                    }
+                    loc[q] = run;
+                }
+                uint32_t x = run;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+                    if ((int)lane >= o) x = max(x, y);
+                }
+                if (lane == 31) s_wmax[warp] = x;
+                uint32_t carry = __shfl_up_sync(0xffffffffu, x, 1);
+                if (lane == 0) carry = 0;
+                __syncthreads();
+                for (uint32_t w = 0; w < warp; w++) carry = max(carry, s_wmax[w]);
+#pragma unroll
+                for (int q = 0; q < kPer; q++) {
+                    const uint32_t i = base + q;
+                    if (i < len) shead[i] = (uint16_t)max(carry, loc[q]);
                 }
                 __syncthreads();
+#pragma unroll
+                for (int j = 0; j < kPer; j++) {
+                    const uint32_t i = j * THREADS + tid;
+                    if (i < len && (i + 1 == len || shead[i + 1] == i + 1))
+                        send[shead[i]] = (uint16_t)(i + 1);
+                }
+                __syncthreads();
+                // settled: alone in its subgroup, or ended with all of it
+#pragma unroll
+                for (int j = 0; j < kPer; j++) {
+                    const uint32_t i = j * THREADS + tid;
+                    if (i < len && sact[i])
+                        sact[i] = send[shead[i]] - shead[i] > 1 && st[i] == full;
+                }
+            }
+            bool open = false;
+#pragma unroll
+            for (int j = 0; j < kPer; j++) {
+                const uint32_t i = j * THREADS + tid;
+                if (i < len) open |= sact[i] != 0;
+            }
+            if (!__syncthreads_or(open ? 1 : 0) || d >= target) break;
+        }
+        const uint32_t depth = d > 0xFFFFFull ? 0xFFFFFu : (uint32_t)d;  // <= 2 * kDirectMaxH + 64
+#pragma unroll
+        for (int j = 0; j < kPer; j++) {
+            const uint32_t i = j * THREADS + tid;
+            if (i < len) {
+                const uint32_t head = shead[i], p = spos[i];
+                sa[g.x + i] = p;
+                hd[g.x + i] = g.x + head;
+                if (rank) rank[p] = g.x + head;
+                if (sact[i] && head == i) {
+                    const uint32_t q = atomicAdd(&s_qn, 1u);
+                    s_q[q] = make_uint2(g.x + i, (uint32_t)(send[i] - i) | depth << 12);
+                }
             }
         }
-        // relation of each member to its predecessor: -1 starts a subgroup
-        for (uint32_t t = tid; t < len; t += kMedThreads) {
-            int r = -1;
-            if (t > 0) {
-                r = direct_cmp(P, spos[t - 1], slim[t - 1], spos[t], slim[t], h, cap, lf);
-                if (r != 0 && r != 2) r = -1;
-            }
-            rel[t] = (int8_t)r;
-        }
         __syncthreads();
-        // subgroup head of every member: block max-scan of (start ? t : 0)
-        constexpr uint32_t kPer = kMediumMax / kMedThreads;
-        uint32_t base = tid * kPer, run = 0;
-        uint32_t loc[kPer];
-#pragma unroll
-        for (uint32_t q = 0; q < kPer; q++) {
-            uint32_t t = base + q;
-            if (t < len && rel[t] == -1) run = t;
-            loc[q] = run;
-        }
-        uint32_t x = run;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-            if ((int)lane >= o) x = max(x, y);
-        }
-        if (lane == 31) wmax[warp] = x;
-        __syncthreads();
-        uint32_t carry = 0;
-        for (uint32_t w = 0; w < warp; w++) carry = max(carry, wmax[w]);
-        uint32_t prev = __shfl_up_sync(0xffffffffu, x, 1);
-        if (lane == 0) prev = 0;
-        carry = max(carry, prev);
-#pragma unroll
-        for (uint32_t q = 0; q < kPer; q++) {
-            uint32_t t = base + q;
-            if (t < len) shead[t] = max(carry, loc[q]);
-        }
-        __syncthreads();
-        for (uint32_t t = tid; t < len; t += kMedThreads) {
-            uint32_t head = shead[t];
-            sa[g.x + t] = spos[t];
-            hd[g.x + t] = g.x + head;
-            if (rank) rank[spos[t]] = g.x + head;
-            bool last = t + 1 == len || rel[t + 1] == -1;
-            if (last && t > head && rel[t] == 2)
-                append_group(G, nxt, g.x + head, t - head + 1, h + cap);
-        }
-        __syncthreads();
+        if (s_qn + MAXM / 2 > kQueue) flush();
     }
+    flush();
 }
 
 // After the big groups' (ordinal, key) pairs are sorted: scatter back into
@@ -3143,8 +3321,8 @@ capssa_status core_sort(Ctx &c, const EngineArgs &a, uint32_t **sa_out, eng::Pac
             CAPSSA_CUDA(c, cudaMemsetAsync(&G.ctr->n[l][nxt], 0, 4, c.stream));
         CAPSSA_CUDA(c, cudaMemsetAsync(&G.ctr->big_packed[nxt], 0, 8, c.stream));
         // the direct kernels work on disjoint groups and only append to the
-        // next round's lists: the four small-group kinds run on side streams
-        // next to the medium kernel on the main one (each alone is latency-
+        // next round's lists: the small-group kinds run on side streams
+        // next to the large medium kernel on the main one (each alone is latency-
         // bound and leaves the SMs half idle), joined before rank doubling
         CAPSSA_CUDA(c, cudaEventRecord(c.fork_ev, c.stream));
         int forked = 0;
@@ -3176,9 +3354,14 @@ capssa_status core_sort(Ctx &c, const EngineArgs &a, uint32_t **sa_out, eng::Pac
             CAPSSA_LAUNCHED(c);
         }
         if (cnt[L_MEDIUM]) {
-            direct_medium_kernel<<<std::min<unsigned>(cnt[L_MEDIUM], c.sm_count * 8), kMedThreads,
-                                   0, c.stream>>>(G.list[L_MEDIUM][cur], cnt[L_MEDIUM], sa, hd,
-                                                  rk, a.lim, P, lf, G, nxt);
+            // one list, two kernels: each takes the groups of its sizes
+            const unsigned mg = std::min<unsigned>(cnt[L_MEDIUM], c.sm_count * 16);
+            direct_medium_kernel<kSmallMax, kMedSmall, 128><<<mg, 128, 0, side()>>>(
+                G.list[L_MEDIUM][cur], cnt[L_MEDIUM], sa, hd, rk, a.lim, P, lf, h, G, nxt);
+            CAPSSA_LAUNCHED(c);
+            direct_medium_kernel<kMedSmall, kMediumMax, 512>
+                <<<std::min<unsigned>(mg, c.sm_count * 4), 512, 0, c.stream>>>(
+                    G.list[L_MEDIUM][cur], cnt[L_MEDIUM], sa, hd, rk, a.lim, P, lf, h, G, nxt);
             CAPSSA_LAUNCHED(c);
         }
         for (int i = 0; i < forked; i++) {

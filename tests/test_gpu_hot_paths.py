@@ -76,3 +76,40 @@ def test_lcp_array_short_long_and_bounded(ctx, dtype, sigma, max_ctx):
         sa, lcp = ctx.build_in_memory_lcp(t, pos, lp, opts, index=np.uint64)
         wsa, wlcp = orc.build_in_memory(t, pos, lo, max_ctx, index=np.uint64, with_lcp=True)
         assert np.array_equal(sa, wsa) and np.array_equal(lcp, wlcp)
+
+
+# ---------------------------------------------------------------- tied groups of 33 .. 2,048 members
+
+def _copies(rng, sigma, unit, copies, tail):
+    """`copies` copies of one random unit, each followed by `tail` random
+    symbols: tied groups of about `copies` members at every offset."""
+    u = rng.integers(0, sigma, unit)
+    parts = []
+    for _ in range(copies):
+        parts += [u, rng.integers(0, sigma, tail)]
+    return np.concatenate(parts)
+
+
+@pytest.mark.parametrize("sigma,dtype", [(2, np.uint8), (4, np.uint8), (6, np.uint8),
+                                         (100, np.uint8), (40000, np.uint32)])
+@pytest.mark.parametrize("copies", [33, 64, 256, 257, 700, 2048, 2049])
+def test_medium_groups_by_windows(ctx, sigma, dtype, copies):
+    """Groups at the edges of the two block kernels (33, 256, 257, 2,048) and
+    just past them, subgroups above and below the counting limit, members
+    that end inside a window (segment ends cut a third of the copies), under
+    both boundary orders."""
+    rng = np.random.default_rng(copies * 7 + sigma)
+    unit = 90 if copies < 1000 else 40
+    t = _copies(rng, sigma, unit, copies, 3).astype(dtype)
+    t = np.concatenate([t, _copies(rng, 2, 30, 40, 1).astype(dtype)])
+    n = len(t)
+    cut = rng.integers(0, copies, copies // 3) * (unit + 3) + rng.integers(1, unit, copies // 3)
+    ends = np.unique(np.concatenate([cut, [n]]))
+    assert np.array_equal(ctx.build_in_memory(t), orc.build_in_memory(t))
+    lp = capssa.SegmentedText(n, ends, capssa.BoundaryRank.LONGER_FIRST)
+    assert np.array_equal(ctx.build_in_memory(t, lp),
+                          orc.build_in_memory(t, None, orc.Limits(n, ends, True)))
+    # ShorterFirst: the reference's tie order pins the order inside tie classes
+    lp = capssa.SegmentedText(n, ends)
+    got = ctx.build_in_memory(t, lp, capssa.Opts(tie_order=capssa.TieOrder.REFERENCE))
+    assert np.array_equal(got, orc.build_in_memory(t, None, orc.Limits(n, ends)))
