@@ -113,3 +113,45 @@ def test_medium_groups_by_windows(ctx, sigma, dtype, copies):
     lp = capssa.SegmentedText(n, ends)
     got = ctx.build_in_memory(t, lp, capssa.Opts(tie_order=capssa.TieOrder.REFERENCE))
     assert np.array_equal(got, orc.build_in_memory(t, None, orc.Limits(n, ends)))
+
+
+# ---------------------------------------------------------------- alphabet and entropy
+
+@pytest.mark.parametrize("n", [(1 << 20) - 1, 1 << 20, (1 << 20) + 4097])
+def test_alphabet_and_entropy_on_the_device(ctx, n):
+    """The same skewed symbols as u8, u16 and u32, on both sides of the size
+    from which the key length follows the sampled entropy: one geometry for
+    all three (their codes are the same), and the oracle's order."""
+    rng = np.random.default_rng(n & 0xFFFF)
+    t = np.minimum(rng.geometric(0.08, n) - 1, 255)
+    t[:256] = np.arange(256)
+    want = orc.build_in_memory(t.astype(np.uint8))
+    seen = set()
+    for dtype in (np.uint8, np.uint16, np.uint32):
+        got = ctx.build_in_memory(t.astype(dtype))
+        st = ctx.stats()
+        seen.add((st["key_symbols"], st["key_bits_per_symbol"]))
+        assert np.array_equal(got, want)
+    assert len(seen) == 1
+
+
+@pytest.mark.parametrize("values", [[0], [0xFFFFFFFF], [0, 0xFFFFFFFF], [7, 8, 70000, 1 << 31]])
+def test_alphabet_of_extreme_u32_symbols(ctx, values):
+    rng = np.random.default_rng(len(values))
+    n = (1 << 20) + 3
+    t = np.array(values, dtype=np.uint32)[rng.integers(0, len(values), n)]
+    if len(values) == 1:  # all suffixes of one run: shorter first
+        assert np.array_equal(ctx.build_in_memory(t), np.arange(n - 1, -1, -1))
+    else:
+        assert np.array_equal(ctx.build_in_memory(t), orc.build_in_memory(t))
+
+
+@pytest.mark.parametrize("values", [[0], [65535], [0, 65535], list(range(0, 65536, 3))])
+def test_alphabet_of_extreme_u16_symbols(ctx, values):
+    rng = np.random.default_rng(len(values))
+    n = (1 << 20) + 3
+    t = np.array(values, dtype=np.uint16)[rng.integers(0, len(values), n)]
+    if len(values) == 1:
+        assert np.array_equal(ctx.build_in_memory(t), np.arange(n - 1, -1, -1))
+    else:
+        assert np.array_equal(ctx.build_in_memory(t), orc.build_in_memory(t))
