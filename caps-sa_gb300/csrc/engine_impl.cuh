@@ -14,6 +14,7 @@
 #include "engine.cuh"
 #include "cdf.cuh"
 #include "lcp.cuh"
+#include "msd.cuh"
 #include "radix.cuh"
 #include "scan.cuh"
 #include "ties.cuh"
@@ -62,9 +63,9 @@ constexpr unsigned long long kBigTotMask = kBigOrdUnit - 1;
 // What the host needs to pick the key geometry.
 struct AlphabetInfo {
     uint32_t lo, hi;    // u8 / u16: sigma in `hi`; u32: smallest and largest symbol
-    uint64_t entropy;   // order-0 entropy of the sample, bits * kEntropyNs * kEntropyUnit
+    uint64_t entropy;   // order-0 entropy of the sample, bits * sample size * kEntropyUnit
 };
-constexpr uint32_t kEntropyNs = 65536;     // evenly strided sample
+constexpr uint32_t kEntropyNs = 65536;     // evenly strided sample, at most
 constexpr float kEntropyUnit = 1048576.0f;  // fixed-point unit of the sum
 constexpr uint32_t kEntropySlots = 131072; // u32 symbols: hash slots of the sample's counts
 
@@ -79,7 +80,7 @@ constexpr uint32_t kEntropySlots = 131072; // u32 symbols: hash slots of the sam
 // went from 3.44 to 1.52 ms, a 16 M-symbol u8 one from 1.20 to 1.14 ms.
 template <typename S>
 __global__ void __launch_bounds__(256)
-    alphabet_kernel(const S *__restrict__ text, uint64_t n, uint64_t stride,
+    alphabet_kernel(const S *__restrict__ text, uint64_t n, uint32_t ns, uint64_t stride,
                     AlphabetInfo *__restrict__ info, uint32_t *__restrict__ present,
                     uint32_t *__restrict__ cnt, unsigned long long *__restrict__ slots) {
     const uint64_t t0 = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
@@ -100,7 +101,7 @@ __global__ void __launch_bounds__(256)
         }
         for (uint64_t i = nv * 16 + t0; i < n; i += step) f[(uint32_t)text[i]] = 1;
         if (stride)
-            for (uint64_t i = t0; i < kEntropyNs; i += step)
+            for (uint64_t i = t0; i < ns; i += step)
                 atomicAdd(&h[(uint32_t)text[i * stride]], 1u);
         __syncthreads();
         for (int i = threadIdx.x; i < 256; i += blockDim.x) {
@@ -116,7 +117,7 @@ __global__ void __launch_bounds__(256)
             if (__ldcg(present + s) == 0) present[s] = 1;
         }
         if (stride)
-            for (uint64_t i = t0; i < kEntropyNs; i += step)
+            for (uint64_t i = t0; i < ns; i += step)
                 atomicAdd(&cnt[(uint32_t)text[i * stride]], 1u);
         return;
     }
@@ -133,7 +134,7 @@ __global__ void __launch_bounds__(256)
         atomicMax(&info->hi, hi);
     }
     if (stride)
-        for (uint64_t i = t0; i < kEntropyNs; i += step) {
+        for (uint64_t i = t0; i < ns; i += step) {
             const uint64_t s = (uint64_t)text[i * stride];
             const unsigned long long key = (s + 1) << 20;
             uint32_t at = (uint32_t)s * 2654435761u >> 15;  // 17 bits
@@ -161,7 +162,7 @@ template <typename S>
 __global__ void __launch_bounds__(1024)
     alphabet_finish_kernel(AlphabetInfo *__restrict__ info, const uint32_t *__restrict__ present,
                            const uint32_t *__restrict__ cnt,
-                           const unsigned long long *__restrict__ slots, int sampled,
+                           const unsigned long long *__restrict__ slots, uint32_t ns,
                            uint16_t *__restrict__ code) {
     __shared__ uint32_t s_w[32];
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -169,9 +170,20 @@ __global__ void __launch_bounds__(1024)
         constexpr uint32_t kVals = sizeof(S) == 1 ? 256 : 65536;
         constexpr uint32_t kPer = kVals < 1024 ? 1 : kVals / 1024;
         const uint32_t v0 = tid * kPer;
-        uint32_t mine = 0;
-        if (v0 < kVals)
-            for (uint32_t q = 0; q < kPer; q++) mine += present[v0 + q] ? 1u : 0u;
+        // this thread's values as a bit mask (u16: 64 of them, in 16-byte loads)
+        uint64_t bits = 0;
+        if (kPer == 1) {
+            bits = v0 < kVals && present[v0] ? 1u : 0u;
+        } else {
+            const uint4 *p4 = reinterpret_cast<const uint4 *>(present + v0);
+#pragma unroll
+            for (uint32_t q = 0; q < kPer / 4; q++) {
+                const uint4 x = p4[q];
+                const uint32_t b4 = (x.x ? 1u : 0u) | (x.y ? 2u : 0u) | (x.z ? 4u : 0u) | (x.w ? 8u : 0u);
+                bits |= (uint64_t)b4 << (4 * q);
+            }
+        }
+        const uint32_t mine = (uint32_t)__popcll(bits);
         uint32_t x = mine;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -182,19 +194,30 @@ __global__ void __launch_bounds__(1024)
         __syncthreads();
         uint32_t c = x - mine;
         for (uint32_t w = 0; w < warp; w++) c += s_w[w];
-        if (v0 < kVals)
-            for (uint32_t q = 0; q < kPer; q++) {
-                code[v0 + q] = (uint16_t)c;
-                c += present[v0 + q] ? 1u : 0u;
+        if (kPer == 1) {
+            if (v0 < kVals) code[v0] = (uint16_t)c;
+        } else {
+            uint4 *c4 = reinterpret_cast<uint4 *>(code + v0);
+            for (uint32_t q = 0; q < kPer; q += 8) {
+                uint32_t w[4];
+#pragma unroll
+                for (uint32_t e = 0; e < 4; e++) {
+                    const uint32_t at = q + 2 * e;
+                    const uint32_t a = c + (uint32_t)__popcll(bits & ((1ull << at) - 1));
+                    w[e] = (a & 0xFFFFu) | (a + ((bits >> at) & 1 ? 1u : 0u)) << 16;
+                }
+                c4[q / 8] = make_uint4(w[0], w[1], w[2], w[3]);
             }
-        if (tid == 1023) info->hi = c;
+        }
+        if (tid == 1023) info->hi = c + mine;
     }
-    if (!sampled) return;
+    if (!ns) return;
     constexpr uint32_t kCnts = sizeof(S) == 1 ? 256 : sizeof(S) == 2 ? 65536 : kEntropySlots;
     unsigned long long sum = 0;
+#pragma unroll 16
     for (uint32_t i = tid; i < kCnts; i += 1024) {
         const uint32_t q = sizeof(S) <= 2 ? cnt[i] : (uint32_t)(slots[i] & 0xFFFFFu);
-        if (q) sum += (unsigned long long)((float)q * log2f((float)kEntropyNs / q) * kEntropyUnit);
+        if (q) sum += (unsigned long long)((float)q * log2f((float)ns / q) * kEntropyUnit);
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
@@ -231,9 +254,29 @@ __device__ __forceinline__ uint64_t window_at(const Packed &P, uint64_t p) {
     return v & P.mask;
 }
 
-// Composite key of every text position (engine.cuh step 2), with the digit
-// histograms of every radix pass accumulated on the way (so the sort needs
-// no separate histogram read of the keys).  The k-symbol content of each
+// Digits of the key counted while the records are made: the first one the
+// MSD sort distributes by (n = 1), or every 8-bit digit of the LSD passes.
+struct KeyDigits {
+    int n, shift, bits;
+    __device__ __forceinline__ int words() const { return n << bits; }
+    __device__ __forceinline__ void count(uint32_t *hist, uint64_t key) const {
+        if (n == 1) {
+            atomicAdd(&hist[(uint32_t)(key >> shift) & ((1u << bits) - 1u)], 1u);
+            return;
+        }
+        const uint32_t lo = (uint32_t)key, hi = (uint32_t)(key >> 32);
+#pragma unroll
+        for (int ps = 0; ps < 8; ps++)
+            if (ps < n)
+                atomicAdd(&hist[ps * 256 + (((ps < 4 ? lo : hi) >> (8 * (ps & 3))) & 255u)], 1u);
+    }
+};
+constexpr int kDigitWords = 1 << msd::kMaxDigit;  // shared counters of either form
+static_assert(kDigitWords >= radix::kMaxPasses * 256, "the LSD digits fit too");
+
+// Composite key of every text position (engine.cuh step 2), with the counts
+// of the digits the sort needs accumulated on the way (so that it needs no
+// separate read of the keys).  The k-symbol content of each
 // suffix is read straight from the packed text (two 64-bit loads, shared by
 // the neighbouring threads' positions); only suffixes that end inside the
 // window (lim < k) are masked and padded.  Each thread owns kKeyPer
@@ -245,10 +288,10 @@ __device__ __forceinline__ uint64_t window_at(const Packed &P, uint64_t p) {
 template <bool kPlain>
 __global__ void __launch_bounds__(kKeyThreads)
     key_kernel(Packed P, uint64_t n, uint64_t n_rec, DevLimits L, int k, int lbits, int flag_len,
-               int vbits, int lf, int n_passes, int seg_shift, int local_pos,
+               int vbits, int lf, KeyDigits td, int seg_shift, int local_pos,
                uint64_t *__restrict__ keys, uint32_t *__restrict__ counts) {
-    __shared__ uint32_t hist[8 * 256];
-    for (int i = threadIdx.x; i < n_passes * 256; i += kKeyThreads) hist[i] = 0;
+    __shared__ uint32_t hist[kDigitWords];
+    for (int i = threadIdx.x; i < td.words(); i += kKeyThreads) hist[i] = 0;
     __syncthreads();
     const int b = P.b;
     const int kbits = k * b;  // 1..63
@@ -292,12 +335,7 @@ __global__ void __launch_bounds__(kKeyThreads)
                                                 : (uint64_t)(lf ? k - take : take);
                 key = lbits ? (content << lbits) | field : content;
                 if (!kPlain && seg_shift) key |= seg << seg_shift;
-                const uint32_t lo = (uint32_t)key, hi = (uint32_t)(key >> 32);
-#pragma unroll
-                for (int ps = 0; ps < 8; ps++)
-                    if (ps < n_passes)
-                        atomicAdd(&hist[ps * 256 + (((ps < 4 ? lo : hi) >> (8 * (ps & 3))) & 255u)],
-                                  1u);
+                td.count(hist, key);
                 if (vbits) key = (key << vbits) | (p - start);
             }
             out[e] = key;
@@ -314,23 +352,21 @@ __global__ void __launch_bounds__(kKeyThreads)
         }
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < n_passes * 256; i += kKeyThreads)
+    for (int i = threadIdx.x; i < td.words(); i += kKeyThreads)
         if (hist[i]) atomicAdd(&counts[i], hist[i]);
 }
 
-// key_kernel for a plain text in the flagless geometry when a radix digit
-// holds whole symbols (b divides 8) and the key whole digits.  Every record
-// is a full window (p <= n - k), so there is no limit, flag or segment
-// logic; a thread's kKeyPer windows lie in the two packed words at its
+// key_kernel for a plain text in the flagless geometry when b divides 8.
+// Every record is a full window (p <= n - k), so there is no limit, flag or
+// segment logic; a thread's kKeyPer windows lie in the two packed words at its
 // first position (its bit offset is a multiple of 8b, so offset + 7b < 64).
-// Only pass 0's digit histogram is counted: key_hist_shift_kernel derives
-// the other passes' from it.
 __global__ void __launch_bounds__(kKeyThreads)
-    key_flagless_kernel(Packed P, uint64_t n_rec, int kbits, int vbits,
+    key_flagless_kernel(Packed P, uint64_t n_rec, int kbits, int vbits, KeyDigits td,
                         uint64_t *__restrict__ keys, uint32_t *__restrict__ counts) {
-    static_assert(kKeyThreads == 256 && kKeyPer == 8, "one thread per digit; 8 windows per word pair");
-    __shared__ uint32_t hist[256];
-    hist[threadIdx.x] = 0;
+    // one digit only: the top one, or the lowest (see key_hist_shift_kernel)
+    static_assert(kKeyPer == 8, "8 windows per word pair");
+    __shared__ uint32_t hist[kDigitWords];
+    for (int i = threadIdx.x; i < td.words(); i += kKeyThreads) hist[i] = 0;
     __syncthreads();
     const int b = P.b;
     for (uint64_t t0 = (uint64_t)blockIdx.x * kKeyTile; t0 < n_rec;
@@ -345,7 +381,8 @@ __global__ void __launch_bounds__(kKeyThreads)
         for (int e = 0; e < kKeyPer; e++) {
             const uint32_t sh = sh0 + (uint32_t)(e * b);
             const uint64_t content = ((w0 << sh) | ((w1 >> 1) >> (63 - sh))) >> (64 - kbits);
-            if (p0 + e < n_rec) atomicAdd(&hist[(uint32_t)content & 255u], 1u);
+            if (p0 + e < n_rec)
+                atomicAdd(&hist[(uint32_t)(content >> td.shift) & ((1u << td.bits) - 1u)], 1u);
             out[e] = (content << vbits) | (p0 + e);
         }
         if (p0 + kKeyPer <= n_rec) {
@@ -360,7 +397,8 @@ __global__ void __launch_bounds__(kKeyThreads)
         }
     }
     __syncthreads();
-    if (hist[threadIdx.x]) atomicAdd(&counts[threadIdx.x], hist[threadIdx.x]);
+    for (int i = threadIdx.x; i < td.words(); i += kKeyThreads)
+        if (hist[i]) atomicAdd(&counts[i], hist[i]);
 }
 
 // Digit histograms of radix passes 1.. from pass 0's (key_flagless_kernel).
@@ -392,9 +430,9 @@ template <bool kPlain>
 __global__ void __launch_bounds__(kKeyThreads)
     sparse_key_kernel(Packed P, uint64_t n, const uint32_t *__restrict__ pos, uint64_t m,
                       DevLimits L, int k, int lbits, int flag_len, int vbits, int lf,
-                      int n_passes, uint64_t *__restrict__ keys, uint32_t *__restrict__ counts) {
-    __shared__ uint32_t hist[8 * 256];
-    for (int i = threadIdx.x; i < n_passes * 256; i += kKeyThreads) hist[i] = 0;
+                      KeyDigits td, uint64_t *__restrict__ keys, uint32_t *__restrict__ counts) {
+    __shared__ uint32_t hist[kDigitWords];
+    for (int i = threadIdx.x; i < td.words(); i += kKeyThreads) hist[i] = 0;
     __syncthreads();
     const int b = P.b;
     const int kbits = k * b;
@@ -416,16 +454,12 @@ __global__ void __launch_bounds__(kKeyThreads)
         const uint64_t field = flag_len ? (uint64_t)((take == k) != (lf != 0))
                                         : (uint64_t)(lf ? k - take : take);
         uint64_t key = lbits ? (content << lbits) | field : content;
-        const uint32_t lo = (uint32_t)key, hi = (uint32_t)(key >> 32);
-#pragma unroll
-        for (int ps = 0; ps < 8; ps++)
-            if (ps < n_passes)
-                atomicAdd(&hist[ps * 256 + (((ps < 4 ? lo : hi) >> (8 * (ps & 3))) & 255u)], 1u);
+        td.count(hist, key);
         if (vbits) key = (key << vbits) | p;
         keys[i] = key;
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < n_passes * 256; i += kKeyThreads)
+    for (int i = threadIdx.x; i < td.words(); i += kKeyThreads)
         if (hist[i]) atomicAdd(&counts[i], hist[i]);
 }
 
@@ -2620,7 +2654,7 @@ __global__ void pf_table_kernel(const uint64_t *__restrict__ pkey, uint32_t n_pi
 template <bool kPlain, bool LEARNED>
 __global__ void __launch_bounds__(kKeyThreads)
     pf_key_kernel(Packed P, uint64_t n, DevLimits L, int k, int lbits, int flag_len, int vbits,
-                  int lf, int n_passes, int bucket_shift, const uint64_t *__restrict__ pkey,
+                  int lf, KeyDigits td, int bucket_shift, const uint64_t *__restrict__ pkey,
                   const uint32_t *__restrict__ ppos, const uint64_t *__restrict__ plim,
                   const uint16_t *__restrict__ ell, const uint16_t *__restrict__ tbl, uint32_t p,
                   const __nv_bfloat16 *__restrict__ w, int bisect,
@@ -2632,8 +2666,8 @@ __global__ void __launch_bounds__(kKeyThreads)
     constexpr uint32_t kTbl = (1u << kPfTableBits) + 1;
     uint64_t *sk = reinterpret_cast<uint64_t *>(pfs);           // n_piv pivot keys
     uint32_t *bh = reinterpret_cast<uint32_t *>(sk + n_piv);    // p bucket counts
-    uint32_t *hist = bh + p;                                     // 8 * 256 digit counts
-    uint16_t *sell = reinterpret_cast<uint16_t *>(hist + 8 * 256);  // p window offsets
+    uint32_t *hist = bh + p;                                     // top digit counts
+    uint16_t *sell = reinterpret_cast<uint16_t *>(hist + td.words());  // p window offsets
     uint16_t *stbl = sell + p;                                   // kTbl top-bits index
     __nv_bfloat16 *sw = reinterpret_cast<__nv_bfloat16 *>(stbl + kTbl + 1);
     for (uint32_t j = threadIdx.x; j < n_piv; j += kKeyThreads) sk[j] = pkey[j];
@@ -2642,7 +2676,7 @@ __global__ void __launch_bounds__(kKeyThreads)
         bh[j] = 0;
     }
     for (uint32_t j = threadIdx.x; j < kTbl; j += kKeyThreads) stbl[j] = tbl[j];
-    for (int i = threadIdx.x; i < 8 * 256; i += kKeyThreads) hist[i] = 0;
+    for (int i = threadIdx.x; i < td.words(); i += kKeyThreads) hist[i] = 0;
     if (LEARNED)
         for (int j = threadIdx.x; j < cdf::kParams; j += kKeyThreads) sw[j] = w[j];
     __syncthreads();
@@ -2782,12 +2816,7 @@ __global__ void __launch_bounds__(kKeyThreads)
                                                 : (uint64_t)(lf ? k - take : take);
                 rec = (lbits ? (content << lbits) | field : content) |
                       ((uint64_t)bk[e] << bucket_shift);
-                const uint32_t rlo = (uint32_t)rec, rhi = (uint32_t)(rec >> 32);
-#pragma unroll
-                for (int ps = 0; ps < 8; ps++)
-                    if (ps < n_passes)
-                        atomicAdd(&hist[ps * 256 + (((ps < 4 ? rlo : rhi) >> (8 * (ps & 3))) & 255u)],
-                                  1u);
+                td.count(hist, rec);
                 rec = (rec << vbits) | q;
             }
             out[e] = rec;
@@ -2814,7 +2843,7 @@ __global__ void __launch_bounds__(kKeyThreads)
         atomicAdd(&stats[1], mis);
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < n_passes * 256; i += kKeyThreads)
+    for (int i = threadIdx.x; i < td.words(); i += kKeyThreads)
         if (hist[i]) atomicAdd(&counts[i], hist[i]);
     for (uint32_t j = threadIdx.x; j < p; j += kKeyThreads)
         if (bh[j]) atomicAdd(&sizes[j], (unsigned long long)bh[j]);
@@ -2922,8 +2951,7 @@ struct PfRun {
 // pf->fell_back (checked after the sample sort and after the fused kernel).
 template <typename S>
 capssa_status pf_keys(Ctx &c, const EngineArgs &a, const eng::Packed &P, const KeyGeom &geo,
-                      int bucket_bits, int key_passes, uint64_t *keys, uint32_t *counts,
-                      PfRun *pf) {
+                      eng::KeyDigits td, uint64_t *keys, uint32_t *counts, PfRun *pf) {
     using namespace eng;
     const uint64_t n = a.n;
     const int lf = a.lim.longer_first;
@@ -3026,11 +3054,11 @@ capssa_status pf_keys(Ctx &c, const EngineArgs &a, const eng::Packed &P, const K
     pf_table_kernel<<<grid_for((1u << kPfTableBits) + 1, 256), 256, 0, c.stream>>>(pkey, p - 1,
                                                                                     tbl);
     CAPSSA_LAUNCHED(c);
-    // 4. the fused partition + record kernel (the sample's sort used the
-    // histogram buffer: clear it for the records' digit counts)
-    CAPSSA_CUDA(c, cudaMemsetAsync(counts, 0, radix::kMaxPasses * 256 * 4, c.stream));
+    // 4. the fused partition + record kernel (the sample's sort may have used
+    // the digit counts' buffer: clear it again)
+    CAPSSA_CUDA(c, cudaMemsetAsync(counts, 0, (size_t)4 * td.n << td.bits, c.stream));
     CAPSSA_CUDA(c, cudaMemsetAsync(sizes, 0, ((size_t)p + 4) * 8, c.stream));
-    const size_t smem = (size_t)(p - 1) * 8 + (size_t)p * 4 + 8 * 256 * 4 + (size_t)p * 2 +
+    const size_t smem = (size_t)(p - 1) * 8 + (size_t)p * 4 + ((size_t)4 * td.n << td.bits) + (size_t)p * 2 +
                         (((size_t)1 << kPfTableBits) + 2) * 2 + cdf::kParams * 2 + 16;
     const bool plain = !a.lim.segmented;
     const unsigned grid = std::min<unsigned>(grid_for(n, kKeyTile), (unsigned)c.sm_count * 8);
@@ -3042,7 +3070,7 @@ capssa_status pf_keys(Ctx &c, const EngineArgs &a, const eng::Packed &P, const K
         cudaFuncSetAttribute(pf_key_kernel<PL, LE>, cudaFuncAttributeMaxDynamicSharedMemorySize,  \
                              (int)smem);                                                          \
         pf_key_kernel<PL, LE><<<grid, kKeyThreads, smem, c.stream>>>(                             \
-            P, n, a.lim, geo.k, geo.lbits, geo.flag_len, geo.vbits, lf, key_passes, geo.total,    \
+            P, n, a.lim, geo.k, geo.lbits, geo.flag_len, geo.vbits, lf, td, geo.total,            \
             pkey, ppos, plim, ell, tbl, p, wbf, pf->bisect ? 1 : 0, keys, counts, sizes, sizes + p, \
             fb);                                                                                   \
     } while (0)
@@ -3068,7 +3096,6 @@ capssa_status pf_keys(Ctx &c, const EngineArgs &a, const eng::Packed &P, const K
     pf->fell_back = *h_fb != 0;
     pf->d_pivots = ppos;
     pf->d_sizes = sizes;
-    (void)bucket_bits;
     return CAPSSA_OK;
 }
 
@@ -3087,12 +3114,13 @@ capssa_status core_sort(Ctx &c, const EngineArgs &a, uint32_t **sa_out, eng::Pac
     // ---- 1. alphabet -> codes, and the order-0 entropy of the symbols: the
     // key must hold about log2(n) / H + 3 symbols to leave few random ties
     // (the b-bit code width overstates H for skewed alphabets; small texts:
-    // ties are cheap either way)
-    const bool sampled = n >= (1u << 20);
-    const uint64_t stride = sampled ? n / kEntropyNs : 0;
+    // ties are cheap either way, the entropy only picks the kind of sort)
+    const bool sampled = n > msd::kOneBlock;
+    const uint32_t ns = (uint32_t)std::min<uint64_t>(n, kEntropyNs);
+    const uint64_t stride = sampled ? n / ns : 0;
     const size_t nvals = sizeof(S) == 1 ? 256 : sizeof(S) == 2 ? 65536 : 0;
     const size_t cnt_bytes = sizeof(S) <= 2 ? nvals * 4 : (sampled ? kEntropySlots * 8 : 0);
-    const size_t zero_bytes = sizeof(AlphabetInfo) + nvals * 4 + cnt_bytes;
+    const size_t zero_bytes = sizeof(AlphabetInfo) + nvals * 4 + cnt_bytes;  // a multiple of 16
     char *ab = (char *)ws_get(c, WS_CODES, zero_bytes + nvals * 2 + 64);
     if (!ab) return set_err(c, CAPSSA_ENOMEM, "alphabet table");
     AlphabetInfo *d_info = (AlphabetInfo *)ab;
@@ -3101,11 +3129,11 @@ capssa_status core_sort(Ctx &c, const EngineArgs &a, uint32_t **sa_out, eng::Pac
     uint16_t *d_code = (uint16_t *)(ab + zero_bytes);
     CAPSSA_CUDA(c, cudaMemsetAsync(ab, 0, zero_bytes, c.stream));
     alphabet_kernel<S><<<std::min<unsigned>(grid_for(n, 256), c.sm_count * 8), 256, 0, c.stream>>>(
-        text, n, stride, d_info, present, cnts, (unsigned long long *)cnts);
+        text, n, ns, stride, d_info, present, cnts, (unsigned long long *)cnts);
     CAPSSA_LAUNCHED(c);
     alphabet_finish_kernel<S><<<1, 1024, 0, c.stream>>>(d_info, present, cnts,
                                                         (const unsigned long long *)cnts,
-                                                        sampled ? 1 : 0, d_code);
+                                                        sampled ? ns : 0, d_code);
     CAPSSA_LAUNCHED(c);
     AlphabetInfo *h_info = (AlphabetInfo *)c.h_scratch;
     CAPSSA_CUDA(c, cudaMemcpyAsync(h_info, d_info, sizeof(AlphabetInfo), cudaMemcpyDeviceToHost,
@@ -3116,11 +3144,12 @@ capssa_status core_sort(Ctx &c, const EngineArgs &a, uint32_t **sa_out, eng::Pac
     const uint64_t sigma_span =
         sizeof(S) <= 2 ? h_info->hi : (uint64_t)h_info->hi - minv + 1;
     const int b = bits_for(sigma_span > 1 ? sigma_span - 1 : 1);
-    double hbits = (double)b;
-    if (sampled && b > 1) {
-        const double hsum = (double)h_info->entropy / kEntropyUnit / kEntropyNs;
+    double hbits = (double)b, entropy = (double)b;
+    if (sampled) {
+        entropy = (double)h_info->entropy / kEntropyUnit / ns;
         // within 3% of the code width counts as full (sampling noise)
-        hbits = hsum >= 0.97 * b ? (double)b : std::max<double>(hsum, 0.25);
+        if (n >= (1u << 20) && b > 1)
+            hbits = entropy >= 0.97 * b ? (double)b : std::max<double>(entropy, 0.25);
     }
     // segment-major order: the segment index sits above the key bits, and
     // the key only has to tell apart the suffixes of one segment
@@ -3171,10 +3200,25 @@ capssa_status core_sort(Ctx &c, const EngineArgs &a, uint32_t **sa_out, eng::Pac
     // pass instead of 12
     const int vbits = geo.vbits;
     const int local_pos = vbits && seg_bits && geo.local_pos ? 1 : 0;
-    const int key_passes = (sort_bits + 7) / 8;
-    uint32_t *counts = radix::hist_buffer(c);
-    if (!counts) return set_err(c, CAPSSA_ENOMEM, "radix histograms");
-    CAPSSA_CUDA(c, cudaMemsetAsync(counts, 0, radix::kMaxPasses * 256 * 4, c.stream));
+    // Distribution by leading digits (msd.cuh) for spread keys, stable LSD
+    // passes (radix.cuh) for skewed ones, whose leading digits hold little of
+    // their information and leave long pieces level after level: at an
+    // entropy of 0.64 of the code width (a word text, 50 M records of 12
+    // bytes) the MSD levels took 7.7 ms and the LSD passes 3.2 ms, at 0.7 (a
+    // masked genome, 134 M) 7.3 and 7.2 ms, at 1 (DNA, 268 M of 8 bytes) 4.5
+    // and 6.0 ms.
+    const bool use_msd = n_rec <= msd::kOneBlock || entropy >= 0.9 * b;
+    const int lsd_passes = (sort_bits + 7) / 8;
+    const msd::Plan plan =
+        msd::plan(n_rec, sort_bits, seg_bits,
+                  pf ? 2 * n / pf->p : (seg_bits ? a.seg_max_len : n_rec), entropy / geo.b);
+    const int top_bits = std::max(plan.bits[0], 1);
+    const KeyDigits td = use_msd ? KeyDigits{1, sort_bits - top_bits, top_bits}
+                                 : KeyDigits{lsd_passes, 0, 8};
+    uint32_t *counts = use_msd ? msd::count_buffer(c) : radix::hist_buffer(c);
+    if (!counts) return set_err(c, CAPSSA_ENOMEM, "digit counts");
+    if (!use_msd)
+        CAPSSA_CUDA(c, cudaMemsetAsync(counts, 0, radix::kMaxPasses * 256 * 4, c.stream));
     // bit-packed copy of the text: the key windows, and the direct
     // comparisons of small groups
     const uint64_t nwords = (n * (uint64_t)geo.b + 63) / 64 + 4;
@@ -3194,50 +3238,60 @@ capssa_status core_sort(Ctx &c, const EngineArgs &a, uint32_t **sa_out, eng::Pac
     P.mask = P.spw * P.b >= 64 ? ~0ull : (~0ull << (64 - P.spw * P.b));
     const unsigned kgrid = std::min<unsigned>(grid_for(n_rec, kKeyTile), c.sm_count * 8);
     if (pf) {
-        capssa_status s0 = pf_keys<S>(c, a, P, geo, seg_bits, key_passes, keys_a, counts, pf);
+        capssa_status s0 = pf_keys<S>(c, a, P, geo, td, keys_a, counts, pf);
         if (s0 != CAPSSA_OK || pf->fell_back) return s0;
     } else if (sp) {
         const unsigned sg = std::min<unsigned>(grid_for(N, kKeyThreads), c.sm_count * 8);
         if (!a.lim.segmented)
             sparse_key_kernel<true><<<sg, kKeyThreads, 0, c.stream>>>(
-                P, n, sp->pos, N, a.lim, geo.k, geo.lbits, geo.flag_len, vbits, lf, key_passes,
+                P, n, sp->pos, N, a.lim, geo.k, geo.lbits, geo.flag_len, vbits, lf, td,
                 keys_a, counts);
         else
             sparse_key_kernel<false><<<sg, kKeyThreads, 0, c.stream>>>(
-                P, n, sp->pos, N, a.lim, geo.k, geo.lbits, geo.flag_len, vbits, lf, key_passes,
+                P, n, sp->pos, N, a.lim, geo.k, geo.lbits, geo.flag_len, vbits, lf, td,
                 keys_a, counts);
         CAPSSA_LAUNCHED(c);
         if (!vbits)  // the record's value is its position
             CAPSSA_CUDA(c, cudaMemcpyAsync(vals_a, sp->pos, (size_t)N * 4, cudaMemcpyDeviceToDevice,
                                            c.stream));
     } else if (!a.lim.segmented && !seg_bits && geo.flagless && vbits && 8 % geo.b == 0 &&
-               geo.total % 8 == 0 && key_passes == geo.total / 8 && n_rec >= 64) {
+               (use_msd || (geo.total % 8 == 0 && n_rec >= 64))) {
         key_flagless_kernel<<<kgrid, kKeyThreads, 0, c.stream>>>(P, n_rec, geo.total, vbits,
+                                                                 KeyDigits{1, td.shift, td.bits},
                                                                  keys_a, counts);
         CAPSSA_LAUNCHED(c);
-        key_hist_shift_kernel<<<1, 256, 0, c.stream>>>(P, n_rec, geo.total, key_passes, counts);
-        CAPSSA_LAUNCHED(c);
+        if (!use_msd) {
+            key_hist_shift_kernel<<<1, 256, 0, c.stream>>>(P, n_rec, geo.total, lsd_passes, counts);
+            CAPSSA_LAUNCHED(c);
+        }
     } else if (!a.lim.segmented && !seg_bits) {
         key_kernel<true><<<kgrid, kKeyThreads, 0, c.stream>>>(
-            P, n, n_rec, a.lim, geo.k, geo.lbits, geo.flag_len, vbits, lf, key_passes, 0, 0,
+            P, n, n_rec, a.lim, geo.k, geo.lbits, geo.flag_len, vbits, lf, td, 0, 0,
             keys_a, counts);
         CAPSSA_LAUNCHED(c);
     } else {
         key_kernel<false><<<kgrid, kKeyThreads, 0, c.stream>>>(
-            P, n, n_rec, a.lim, geo.k, geo.lbits, geo.flag_len, vbits, lf, key_passes,
+            P, n, n_rec, a.lim, geo.k, geo.lbits, geo.flag_len, vbits, lf, td,
             seg_bits ? geo.total : 0, local_pos, keys_a, counts);
         CAPSSA_LAUNCHED(c);
     }
     cudaEventRecord(c.pev[1], c.stream);
-    bool in_b = false;
     int passes = 0;
-    capssa_status s =
-        vbits ? radix::sort_keys(c, keys_a, keys_b, (uint32_t)n_rec, vbits, vbits + sort_bits,
-                                 &in_b, &passes, /*hist_ready=*/true)
-              : radix::sort_pairs(c, keys_a, vals_a, keys_b, vals_b, nn, 0, sort_bits, !sp, 0,
-                                  &in_b, &passes, /*hist_ready=*/true);
+    bool in_b = false;
+    capssa_status s;
+    if (use_msd) {
+        s = msd::sort(c, plan, keys_a, vbits ? nullptr : vals_a, keys_b, vbits ? nullptr : vals_b,
+                      (uint32_t)n_rec, vbits, sort_bits, bits_for(n - 1), geo.flag_len == 0, !sp,
+                      counts, &passes);
+        c.stats.radix_items = msd::records_per_thread(vbits == 0);
+    } else {
+        s = vbits ? radix::sort_keys(c, keys_a, keys_b, (uint32_t)n_rec, vbits, vbits + sort_bits,
+                                     &in_b, &passes, /*hist_ready=*/true)
+                  : radix::sort_pairs(c, keys_a, vals_a, keys_b, vals_b, nn, 0, sort_bits, !sp, 0,
+                                      &in_b, &passes, /*hist_ready=*/true);
+    }
     if (s != CAPSSA_OK) return s;
-    c.stats.sort_passes = (uint32_t)passes;
+    c.stats.sort_passes = (uint32_t)passes + (use_msd ? 1u : 0u);  // with the local sort
     c.stats.sort_item_bytes = vbits ? 8u : 12u;
     cudaEventRecord(c.pev[2], c.stream);
     const uint64_t *skeys = in_b ? keys_b : keys_a;

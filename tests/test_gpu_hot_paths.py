@@ -155,3 +155,68 @@ def test_alphabet_of_extreme_u16_symbols(ctx, values):
         assert np.array_equal(ctx.build_in_memory(t), np.arange(n - 1, -1, -1))
     else:
         assert np.array_equal(ctx.build_in_memory(t), orc.build_in_memory(t))
+
+
+# ---------------------------------------------------------------- record sort
+
+@pytest.mark.parametrize("n", [2559, 2560, 2561, 4097, 65536, 300007, (1 << 21) + 5])
+@pytest.mark.parametrize("kind", ["dna", "skewed", "runs", "two_values", "u32_wide"])
+def test_record_sort_sizes_and_skew(ctx, n, kind):
+    """Record sorts at the edges of the one-block size, with one and two
+    planned levels, and with keys so uneven that pieces stay long past the
+    planned levels (further levels of 8 bits, down to the position bits)."""
+    rng = np.random.default_rng(n % 1009)
+    if kind == "dna":
+        t = rng.integers(0, 4, n).astype(np.uint8)
+    elif kind == "skewed":
+        t = np.minimum(rng.geometric(0.35, n) - 1, 90).astype(np.uint8)
+    elif kind == "runs":
+        t = rng.integers(0, 4, n).astype(np.uint8)
+        t[n // 7: n // 7 + n // 3] = 2
+        t[n // 2: n // 2 + n // 5] = 0
+    elif kind == "two_values":
+        t = (rng.random(n) < 0.002).astype(np.uint8)
+    else:
+        t = rng.integers(0, 1 << 31, n).astype(np.uint32)
+    got = ctx.build_in_memory(t)
+    assert np.array_equal(got, orc.build_in_memory(t))
+
+
+@pytest.mark.parametrize("n", [30011, 1 << 18])
+@pytest.mark.parametrize("longer_first", [False, True])
+def test_record_sort_complete_ties_keep_position_order(ctx, n, longer_first):
+    """Tens of thousands of one- and two-symbol segments: complete ties far
+    longer than a piece, whose records are ordered by position through the
+    position bits (key and position in one word, and as pairs)."""
+    rng = np.random.default_rng(n)
+    for sigma, dtype in ((3, np.uint8), (60000, np.uint32)):
+        t = rng.integers(0, sigma, n).astype(dtype)
+        t[: n // 2] = 1
+        ends = np.unique(np.concatenate([np.arange(1, n // 2, rng.integers(1, 3)),
+                                         rng.integers(1, n, 50), [n]]))
+        lp = capssa.SegmentedText(n, ends, capssa.BoundaryRank.LONGER_FIRST if longer_first
+                                  else capssa.BoundaryRank.SHORTER_FIRST)
+        lo = orc.Limits(n, ends, longer_first)
+        if longer_first:
+            assert np.array_equal(ctx.build_in_memory(t, lp), orc.build_in_memory(t, None, lo))
+        else:
+            got = ctx.build_in_memory(t, lp, capssa.Opts(tie_order=capssa.TieOrder.REFERENCE))
+            assert np.array_equal(got, orc.build_in_memory(t, None, lo))
+            got = ctx.build_in_memory(t, lp)
+            want = orc.build_in_memory(t, None, lo)
+            assert np.array_equal(got, orc.canonical_ties(want, orc.adjacent_cmp(t, want, lo)))
+
+
+@pytest.mark.parametrize("lens", [[5000, 70000, 3, 400000, 0, 41], [300] * 900, [2560, 1281, 1]])
+def test_record_sort_segment_major(ctx, lens):
+    """Batches of uneven, equal and tiny texts (the text index leads the
+    records), with a run that makes one text's piece long."""
+    rng = np.random.default_rng(len(lens))
+    texts = [rng.integers(0, 4, L).astype(np.uint8) for L in lens]
+    big = int(np.argmax(lens))
+    texts[big][10: 10 + lens[big] // 2] = 3
+    cat = np.concatenate(texts)
+    offs = np.concatenate([[0], np.cumsum(lens)]).astype(np.uint64)
+    got = ctx.build_batched(cat, offs)
+    for i, tx in enumerate(texts):
+        assert np.array_equal(got[offs[i]:offs[i + 1]], orc.build_in_memory(tx)), i
