@@ -177,7 +177,7 @@ __global__ void __launch_bounds__(1024)
         } else {
             const uint4 *p4 = reinterpret_cast<const uint4 *>(present + v0);
 #pragma unroll
-            for (uint32_t q = 0; q < kPer / 4; q++) {
+            for (uint32_t q = 0; q < (kPer + 3) / 4; q++) {
                 const uint4 x = p4[q];
                 const uint32_t b4 = (x.x ? 1u : 0u) | (x.y ? 2u : 0u) | (x.z ? 4u : 0u) | (x.w ? 8u : 0u);
                 bits |= (uint64_t)b4 << (4 * q);
@@ -360,8 +360,9 @@ __global__ void __launch_bounds__(kKeyThreads)
 // Every record is a full window (p <= n - k), so there is no limit, flag or
 // segment logic; a thread's kKeyPer windows lie in the two packed words at its
 // first position (its bit offset is a multiple of 8b, so offset + 7b < 64).
+// flag: 1 with a (set) full-window flag below the key.
 __global__ void __launch_bounds__(kKeyThreads)
-    key_flagless_kernel(Packed P, uint64_t n_rec, int kbits, int vbits, KeyDigits td,
+    key_flagless_kernel(Packed P, uint64_t n_rec, int kbits, int vbits, int flag, KeyDigits td,
                         uint64_t *__restrict__ keys, uint32_t *__restrict__ counts) {
     // one digit only: the top one, or the lowest (see key_hist_shift_kernel)
     static_assert(kKeyPer == 8, "8 windows per word pair");
@@ -380,7 +381,8 @@ __global__ void __launch_bounds__(kKeyThreads)
 #pragma unroll
         for (int e = 0; e < kKeyPer; e++) {
             const uint32_t sh = sh0 + (uint32_t)(e * b);
-            const uint64_t content = ((w0 << sh) | ((w1 >> 1) >> (63 - sh))) >> (64 - kbits);
+            uint64_t content = ((w0 << sh) | ((w1 >> 1) >> (63 - sh))) >> (64 - kbits);
+            content = (content << flag) | (uint64_t)flag;
             if (p0 + e < n_rec)
                 atomicAdd(&hist[(uint32_t)(content >> td.shift) & ((1u << td.bits) - 1u)], 1u);
             out[e] = (content << vbits) | (p0 + e);
@@ -967,6 +969,435 @@ __global__ void __launch_bounds__(256)
         }
         list_ptr(G, li, 0)[slot] = entry;
     }
+}
+
+// ---------------------------------------------------------------- sorted chunks to groups
+//
+// The last step of the MSD record sort (msd.cuh) and the group initialisation
+// in one: a block takes a chunk of distributed records, orders it in shared
+// memory, and writes what init_groups_kernel writes (positions, group heads,
+// the first round's groups), so the sorted records never go back to memory.
+// Only for records that carry their position and one early-end flag (plain
+// texts, and many texts in segment-major order): their tied groups need no
+// order inside.  (Ties that end together, which SegmentedText has, keep
+// ascending position: they take the sorted records and init_groups_kernel.)
+//
+// A chunk's keys differ in few bits, so a record's place is its bin's start
+// plus an atomic rank among 2^13 bins with byte counters, packed four a word:
+// some six bins a record, so a bin mostly holds one record or one tied group.
+// A record alone in its bin has its slot at once; the others leave their low
+// bits (all that a bin's records differ in) in shared memory and find slot,
+// head and group by comparing themselves with their bin.  Positions and heads
+// are staged by slot and written out in order.  A bin of more than kFinBin
+// records (kFinBinOpen when the bins do not resolve every key bit) sends its
+// chunk to finish_crowd_kernel.  Bound by issue and by the round trips of a
+// chunk's phases (1,024 threads an SM): of 11 warp instructions a record the
+// comparisons take 3, placing records 2.6, queueing groups 2.  2^28 DNA records
+// with repeats take 3.5 ms, where the local sort took 2.1 ms and init_groups
+// 1.55 ms; small texts gain more (1 M symbols, the whole call: 0.321 ms with
+// the separate kernels, 0.291 ms).  Bins of 2^14 with three blocks an SM: 0.4
+// ms more at 2^28; listing the shared bins' records first to compare them in
+// full warps: 0.9 ms more.
+constexpr int kFinThreads = 256, kFinIt = msd::kOneBlock / kFinThreads;
+constexpr int kFinBlocks = 4;  // resident per SM
+constexpr int kFinLogBins = 13;
+constexpr uint32_t kFinWords = (1u << kFinLogBins) / 4;
+constexpr uint32_t kFinBin = 250, kFinBinOpen = 63;
+constexpr uint32_t kFinQueue = msd::kOneBlock / 2 + 640;  // a chunk's groups, and some chunks'
+static_assert(kFinThreads * kFinIt == (int)msd::kOneBlock && msd::kOneBlock <= 4096,
+              "a chunk per block, slots of 12 bits");
+
+struct FinArgs {
+    const uint64_t *ka, *kb;  // records
+    int k, lf, vbits;
+    int seg_at;               // segment-local positions: the segment index's bit
+    const uint64_t *seg_ends;
+    uint32_t *hd, *sa;
+};
+
+// Position of a packed record.
+template <bool SEG>
+__device__ __forceinline__ uint32_t rec_pos(const FinArgs &A, uint64_t rec) {
+    uint64_t pos = rec & ((1ull << A.vbits) - 1);
+    if (SEG) {
+        const uint64_t sg = rec >> A.seg_at;
+        pos += sg ? __ldg(A.seg_ends + sg - 1) : 0ull;
+    }
+    return (uint32_t)pos;
+}
+
+// Symbols the members of a group with this key agree on (0: they ended early).
+__device__ __forceinline__ uint32_t rec_depth(const FinArgs &A, uint64_t rec) {
+    return ((uint32_t)(rec >> A.vbits) & 1u) == (A.lf ? 0u : 1u) ? (uint32_t)A.k : 0u;
+}
+
+// Queue of groups in shared memory: (start, length | early end << 31).
+struct FinQueue {
+    uint2 q[kFinQueue];
+    uint32_t n, cnt[kLists], base[kLists];
+};
+
+// The group that ends in this lane (len members from `start`), if len > 0; the
+// whole warp calls (one atomic for all of its groups).
+__device__ __forceinline__ void fin_push(FinQueue &Q, uint32_t start, uint32_t len, bool early) {
+    const unsigned p = __ballot_sync(0xffffffffu, len > 1);
+    if (!p) return;
+    const uint32_t lane = threadIdx.x & 31;
+    uint32_t at = 0;
+    if (lane == 0) at = atomicAdd(&Q.n, (uint32_t)__popc(p));
+    at = __shfl_sync(0xffffffffu, at, 0);
+    if (len > 1)
+        Q.q[at + __popc(p & ((1u << lane) - 1u))] =
+            make_uint2(start, len | (early ? 0x80000000u : 0u));
+}
+
+// Empties the queue into the first round's lists, one atomic per list; the
+// whole block, between barriers of its own.
+__device__ __forceinline__ void fin_flush(const FinArgs &A, FinQueue &Q, const GroupLists &G) {
+    const uint32_t tid = threadIdx.x, lane = tid & 31;
+    __syncthreads();
+    const uint32_t nq = Q.n;
+    if (tid < kLists) Q.cnt[tid] = 0;
+    __syncthreads();
+    constexpr int kPer = (int)((kFinQueue + kFinThreads - 1) / kFinThreads);
+    uint32_t at[kPer];
+#pragma unroll
+    for (int j = 0; j < kPer; j++) {
+        if (j * kFinThreads >= nq) break;
+        const uint32_t i = j * kFinThreads + tid;
+        const int l = i < nq ? list_of(Q.q[i].y & 0x7FFFFFFFu, (uint64_t)A.k) : kLists;
+        const unsigned p = __ballot_sync(0xffffffffu, l == L_PAIR);  // most groups are pairs
+        uint32_t a0 = 0;
+        if (p) {
+            if (lane == 0) a0 = atomicAdd(&Q.cnt[L_PAIR], (uint32_t)__popc(p));
+            a0 = __shfl_sync(0xffffffffu, a0, 0);
+        }
+        at[j] = a0 + __popc(p & ((1u << lane) - 1u));
+        if (l != L_PAIR && l < kLists) at[j] = atomicAdd(&Q.cnt[l], 1u);
+    }
+    __syncthreads();
+    if (tid < kLists && Q.cnt[tid]) Q.base[tid] = atomicAdd(&G.ctr->n[tid][0], Q.cnt[tid]);
+    if (tid == 0) Q.n = 0;
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < kPer; j++) {
+        const uint32_t i = j * kFinThreads + tid;
+        if (j * kFinThreads >= nq) break;
+        if (i < nq) {
+            const uint2 e = Q.q[i];
+            const uint32_t len = e.y & 0x7FFFFFFFu, depth = e.y >> 31 ? 0u : (uint32_t)A.k;
+            const int l = list_of(len, (uint64_t)A.k);
+            // a pair's positions ride along (see kPairPos): this block wrote them
+            if (l == L_PAIR)
+                G.list[L_PAIR][0][Q.base[L_PAIR] + at[j]] =
+                    make_uint4(e.x, A.sa[e.x], depth | kPairPos, A.sa[e.x + 1]);
+            else if (l < kLists)
+                list_ptr(G, l, 0)[Q.base[l] + at[j]] = make_uint4(e.x, len, depth, 0u);
+            else
+                append_big(G, 0, e.x, len, depth);
+        }
+    }
+    __syncthreads();
+}
+
+// Flushes when the queue might not hold another chunk's groups (whole block;
+// one thread's reading decides for all).
+__device__ __forceinline__ void fin_flush_full(const FinArgs &A, FinQueue &Q,
+                                               const GroupLists &G) {
+    __syncthreads();
+    const int full =
+        threadIdx.x == 0 && Q.n + msd::kOneBlock / 2 > kFinQueue;
+    if (__syncthreads_or(full)) fin_flush(A, Q, G);
+}
+
+template <bool SEG>
+__global__ void __launch_bounds__(kFinThreads, kFinBlocks)
+    finish_chunks_kernel(FinArgs A, msd::Chunks C, GroupLists G) {
+    extern __shared__ __align__(16) unsigned char fin_smem[];
+    uint32_t *s_cnt = reinterpret_cast<uint32_t *>(fin_smem);           // four bins a word
+    uint16_t *s_base = reinterpret_cast<uint16_t *>(s_cnt + kFinWords);  // a word's first slot
+    uint32_t *s_pos = reinterpret_cast<uint32_t *>(s_base + kFinWords);  // by slot
+    uint32_t *s_lo = s_pos + msd::kOneBlock;                             // shared bins: low bits
+    // by slot: the group's first slot
+    uint16_t *s_head = reinterpret_cast<uint16_t *>(s_lo + msd::kOneBlock);
+    FinQueue &Q = *reinterpret_cast<FinQueue *>(s_head + msd::kOneBlock);
+    __shared__ uint32_t s_w[kFinThreads / 32];
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (tid == 0) Q.n = 0;
+    const uint32_t nc = C.single.y ? 1u : *C.count;
+    uint4 next = C.single;
+    if (!C.single.y && blockIdx.x < nc) next = C.list[blockIdx.x];
+    for (uint32_t ci = blockIdx.x; ci < nc; ci += gridDim.x) {
+        const uint4 ch = next;
+        if (ci + gridDim.x < nc) next = C.list[ci + gridDim.x];  // a round trip ahead
+        const uint32_t m = ch.y & ~msd::kInB, at = ch.x;
+        const uint64_t *ks = (ch.y & msd::kInB) ? A.kb : A.ka;
+        if (ch.w >= msd::kRunPiece) {  // a run of one key longer than a chunk
+            if (ch.w == msd::kRunWhole) {
+                if (tid == 0) append_group(G, 0, at, ch.z, rec_depth(A, ks[at]));
+            } else {
+                for (uint32_t i = tid; i < m; i += kFinThreads) {
+                    A.sa[at + i] = rec_pos<SEG>(A, ks[at + i]);
+                    A.hd[at + i] = ch.z;
+                }
+            }
+            continue;
+        }
+        const msd::ChunkBins B(ch, kFinLogBins, A.vbits);
+        // key bits left below the bins; a bin's records differ in their low B.sh
+        // bits, compared as a word: past 32 bits it drops position bits (records
+        // of one key stay together), but no key bits (wide keys of few records
+        // are left to the crowd kernel when any bin is shared)
+        const bool open = B.sh > A.vbits;
+        const int drop = B.sh > 32 ? B.sh - 32 : 0;
+        const bool wide = open && drop > A.vbits;
+        const uint32_t klow = A.vbits > drop ? (uint32_t)(A.vbits - drop) : 0u;
+        uint64_t k[kFinIt];
+#pragma unroll
+        for (int j = 0; j < kFinIt; j++) {
+            if (j * kFinThreads >= m) break;
+            const uint32_t i = j * kFinThreads + tid;
+            if (i < m) k[j] = ks[at + i];
+        }
+#pragma unroll
+        for (uint32_t q = 0; q < kFinWords / 4 / kFinThreads; q++)
+            reinterpret_cast<uint4 *>(s_cnt)[q * kFinThreads + tid] = make_uint4(0, 0, 0, 0);
+        __syncthreads();
+        const uint32_t limit = wide ? 1u : (open ? kFinBinOpen : kFinBin);
+        uint32_t rk[(kFinIt + 3) / 4] = {};  // ranks, a byte each
+        bool crowd = false;
+#pragma unroll
+        for (int j = 0; j < kFinIt; j++) {
+            if (j * kFinThreads >= m) break;
+            if (j * kFinThreads + tid < m) {
+                const uint32_t b = B.of(k[j]), by = (b & 3u) * 8u;
+                const uint32_t r = (atomicAdd(&s_cnt[b >> 2], 1u << by) >> by) & 255u;
+                // (counts carry into the next bin past 255, but not unseen: the
+                // limit is passed first)
+                crowd |= r >= limit;
+                rk[j / 4] |= r << (8 * (j % 4));
+            }
+        }
+        if (__syncthreads_or(crowd ? 1 : 0)) {
+            if (tid == 0) C.spare[atomicAdd(C.n_spare, 1u)] = ch;
+            __syncthreads();
+            continue;
+        }
+        {  // each word's first slot: exclusive prefix, eight words a thread
+            constexpr int kW = (int)kFinWords / kFinThreads;
+            static_assert(kW % 8 == 0, "16-byte loads and stores");
+            const uint4 *c4 = reinterpret_cast<const uint4 *>(s_cnt) + tid * (kW / 4);
+            uint32_t w[kW], sum = 0;
+#pragma unroll
+            for (int q = 0; q < kW / 4; q++) {
+                const uint4 x = c4[q];
+                w[4 * q] = __dp4a(x.x, 0x01010101u, 0u);
+                w[4 * q + 1] = __dp4a(x.y, 0x01010101u, 0u);
+                w[4 * q + 2] = __dp4a(x.z, 0x01010101u, 0u);
+                w[4 * q + 3] = __dp4a(x.w, 0x01010101u, 0u);
+                sum += w[4 * q] + w[4 * q + 1] + w[4 * q + 2] + w[4 * q + 3];
+            }
+            uint32_t z = sum;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t t = __shfl_up_sync(0xffffffffu, z, o);
+                if ((int)lane >= o) z += t;
+            }
+            if (lane == 31) s_w[warp] = z;
+            __syncthreads();
+            uint32_t run = z - sum;
+#pragma unroll
+            for (uint32_t q = 0; q < kFinThreads / 32; q++) run += q < warp ? s_w[q] : 0u;
+#pragma unroll
+            for (int q = 0; q < kW / 8; q++) {
+                uint32_t o4[4];
+#pragma unroll
+                for (int e = 0; e < 4; e++) {
+                    const int at2 = 8 * q + 2 * e;
+                    o4[e] = run | (run + w[at2]) << 16;
+                    run += w[at2] + w[at2 + 1];
+                }
+                reinterpret_cast<uint4 *>(s_base)[tid * (kW / 8) + q] =
+                    make_uint4(o4[0], o4[1], o4[2], o4[3]);
+            }
+        }
+        __syncthreads();
+        // first slot of a bin, from its word and the counts before it there
+        auto start_of = [&](uint32_t b, uint32_t word) {
+            const uint32_t below = word & ((1u << ((b & 3u) * 8u)) - 1u);
+            return __dp4a(below, 0x01010101u, (uint32_t)s_base[b >> 2]);
+        };
+        // records that share their bin: slot | rank << 12 | count << 20
+        uint32_t company[kFinIt];
+#pragma unroll
+        for (int j = 0; j < kFinIt; j++) {
+            if (j * kFinThreads >= m) break;
+            if (j * kFinThreads + tid < m) {
+                const uint32_t b = B.of(k[j]), word = s_cnt[b >> 2];
+                const uint32_t s = start_of(b, word), c = (word >> ((b & 3u) * 8u)) & 255u;
+                const uint32_t r = (rk[j / 4] >> (8 * (j % 4))) & 255u;
+                company[j] = c > 1 ? (s + r) | r << 12 | c << 20 : 0u;
+                if (c == 1) {
+                    s_pos[s] = rec_pos<SEG>(A, k[j]);
+                    s_head[s] = (uint16_t)s;
+                } else {
+                    s_lo[s + r] = (uint32_t)(k[j] >> drop);
+                }
+            } else {
+                company[j] = 0;
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < kFinIt; j++) {
+            if (j * kFinThreads >= m) break;
+            uint32_t len = 0, head = 0;  // the group that this record ends
+            bool early = false;
+            if (company[j]) {
+                const uint32_t mine = company[j] & 0xFFFu, s = mine - ((company[j] >> 12) & 255u);
+                const uint32_t e = s + (company[j] >> 20);
+                uint32_t slot = mine, end = e;
+                head = s;
+                if (open) {
+                    // records before this key, before this record, and up to the
+                    // end of this key (equal words: by rank)
+                    const uint32_t me = (uint32_t)(k[j] >> drop);
+                    const uint32_t k0 = (me >> klow) << klow, k1 = me | ((1u << klow) - 1u);
+                    slot = end = s;
+#pragma unroll 1
+                    for (uint32_t u = s; u < e; u++) {
+                        const uint32_t x = s_lo[u];
+                        head += x < k0 ? 1u : 0u;
+                        end += x <= k1 ? 1u : 0u;
+                        slot += x < me || (x == me && u < mine) ? 1u : 0u;
+                    }
+                }
+                s_pos[slot] = rec_pos<SEG>(A, k[j]);
+                s_head[slot] = (uint16_t)head;
+                if (slot + 1 == end) len = end - head;
+                early = rec_depth(A, k[j]) == 0;
+            }
+            fin_push(Q, at + head, len, early);
+        }
+        __syncthreads();
+        for (uint32_t i = tid; i < m; i += kFinThreads) {
+            A.sa[at + i] = s_pos[i];
+            A.hd[at + i] = at + s_head[i];
+        }
+        fin_flush_full(A, Q, G);
+    }
+    fin_flush(A, Q, G);
+}
+
+// The chunks finish_chunks_kernel left (many equal keys): a merge sort in
+// shared memory, by counting inside 32 slots, then runs of doubling length by
+// binary search; heads by a block-wide max-scan.
+template <bool SEG>
+__global__ void __launch_bounds__(kFinThreads)
+    finish_crowd_kernel(FinArgs A, const uint4 *__restrict__ list,
+                        const uint32_t *__restrict__ count, GroupLists G) {
+    extern __shared__ __align__(16) unsigned char fin_smem[];
+    uint64_t *s_key = reinterpret_cast<uint64_t *>(fin_smem);
+    FinQueue &Q = *reinterpret_cast<FinQueue *>(s_key + msd::kOneBlock);
+    __shared__ uint32_t s_w[kFinThreads / 32];
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (tid == 0) Q.n = 0;
+    const uint32_t nc = *count;
+    for (uint32_t ci = blockIdx.x; ci < nc; ci += gridDim.x) {
+        const uint4 ch = list[ci];
+        const uint32_t m = ch.y & ~msd::kInB, at = ch.x;
+        const uint64_t *ks = (ch.y & msd::kInB) ? A.kb : A.ka;
+        for (uint32_t i = tid; i < m; i += kFinThreads) s_key[i] = ks[at + i];
+        __syncthreads();
+        for (uint32_t run = 0; run < m; run = run ? run * 2 : 32) {
+            uint64_t k[kFinIt];
+            uint32_t to[kFinIt];
+#pragma unroll
+            for (int j = 0; j < kFinIt; j++) {
+                const uint32_t i = j * kFinThreads + tid;
+                if (i < m) {
+                    k[j] = s_key[i];
+                    if (run == 0) {
+                        const uint32_t b0 = i & ~31u, b1 = min(m, b0 + 32);
+                        uint32_t p = b0;
+                        for (uint32_t u = b0; u < b1; u++) p += s_key[u] < k[j] ? 1u : 0u;
+                        to[j] = p;
+                    } else {  // records are distinct
+                        const uint32_t p0 = i & ~(2 * run - 1), mid = p0 + run;
+                        const bool left = i < mid;
+                        const uint32_t a0 = left ? min(mid, m) : p0;
+                        const uint32_t a1 = left ? min(mid + run, m) : mid;
+                        uint32_t l = a0, h = a1;
+                        while (l < h) {
+                            const uint32_t mm = (l + h) >> 1;
+                            if (s_key[mm] < k[j])
+                                l = mm + 1;
+                            else
+                                h = mm;
+                        }
+                        to[j] = left ? i + (l - a0) : i - (a1 - l);
+                    }
+                }
+            }
+            __syncthreads();
+#pragma unroll
+            for (int j = 0; j < kFinIt; j++)
+                if (j * kFinThreads + tid < m) s_key[to[j]] = k[j];
+            __syncthreads();
+        }
+        // head of every slot: consecutive slots a thread, max-scan of the heads
+        uint32_t hv[kFinIt], run = 0;
+#pragma unroll
+        for (int j = 0; j < kFinIt; j++) {
+            const uint32_t i = tid * kFinIt + j;
+            if (i < m && (i == 0 || s_key[i - 1] >> A.vbits != s_key[i] >> A.vbits)) run = i;
+            hv[j] = run;
+        }
+        uint32_t x = run;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+            if ((int)lane >= o) x = max(x, y);
+        }
+        if (lane == 31) s_w[warp] = x;
+        uint32_t carry = __shfl_up_sync(0xffffffffu, x, 1);
+        if (lane == 0) carry = 0;
+        __syncthreads();
+        for (uint32_t w = 0; w < warp; w++) carry = max(carry, s_w[w]);
+#pragma unroll
+        for (int j = 0; j < kFinIt; j++) {
+            const uint32_t i = tid * kFinIt + j;
+            uint32_t len = 0, head = 0;
+            bool early = false;
+            if (i < m) {
+                const uint64_t rec = s_key[i];
+                head = max(carry, hv[j]);
+                A.sa[at + i] = rec_pos<SEG>(A, rec);
+                A.hd[at + i] = at + head;
+                early = rec_depth(A, rec) == 0;
+                if (head != i && (i + 1 == m || s_key[i + 1] >> A.vbits != rec >> A.vbits))
+                    len = i - head + 1;
+            }
+            fin_push(Q, at + head, len, early);
+        }
+        fin_flush_full(A, Q, G);
+    }
+    fin_flush(A, Q, G);
+}
+
+// Records of the short suffixes (positions n_full .. n - 1) of a text whose
+// other records key_flagless_kernel made: the symbols they have, zero padded,
+// and a clear flag; counted with the others' first digit.
+__global__ void short_records_kernel(Packed P, uint64_t n, uint64_t n_full, int k, int vbits,
+                                     KeyDigits td, uint64_t *__restrict__ keys,
+                                     uint32_t *__restrict__ counts) {
+    const uint64_t p = n_full + threadIdx.x;
+    if (p >= n) return;
+    const int take = (int)(n - p);  // < k
+    uint64_t key = window_at(P, p) >> (64 - k * P.b);
+    key = (key & ~((1ull << ((k - take) * P.b)) - 1)) << 1;
+    keys[p] = (key << vbits) | p;
+    atomicAdd(&counts[(uint32_t)(key >> td.shift) & ((1u << td.bits) - 1u)], 1u);
 }
 
 // Sort key of suffix p for a round at depth h: the rank of p + h, or the
@@ -3099,6 +3530,26 @@ capssa_status pf_keys(Ctx &c, const EngineArgs &a, const eng::Packed &P, const K
     return CAPSSA_OK;
 }
 
+// A batch of distributed chunks to positions, heads and groups.
+template <bool SEG>
+capssa_status finish_chunks(Ctx &c, const eng::FinArgs &A, const msd::Chunks &C,
+                            const eng::GroupLists &G) {
+    using namespace eng;
+    const size_t crowd_smem = (size_t)msd::kOneBlock * 8 + sizeof(FinQueue);
+    const size_t smem = kFinWords * 6 + (size_t)msd::kOneBlock * 10 + sizeof(FinQueue);
+    cudaFuncSetAttribute(finish_chunks_kernel<SEG>,
+                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    finish_chunks_kernel<SEG>
+        <<<C.single.y ? 1u : (unsigned)c.sm_count * kFinBlocks, kFinThreads, smem,
+           c.stream>>>(A, C, G);
+    CAPSSA_LAUNCHED(c);
+    finish_crowd_kernel<SEG>
+        <<<C.single.y ? 1u : (unsigned)c.sm_count * 2, kFinThreads, crowd_smem, c.stream>>>(
+            A, C.spare, C.n_spare, G);
+    CAPSSA_LAUNCHED(c);
+    return CAPSSA_OK;
+}
+
 // Steps 1-4 of engine.cuh over every text position under the unbounded
 // comparator; *sa_out receives the device SA (n entries).  With `pf`, the
 // records lead with the sample sort's bucket (partition first).
@@ -3174,11 +3625,27 @@ capssa_status core_sort(Ctx &c, const EngineArgs &a, uint32_t **sa_out, eng::Pac
                        seg_bits ? a.seg_max_len : (sp ? sp->m : 0), allow_flagless,
                        a.seg_major && !lf);
     }
-    // records the radix sort orders: every suffix, or the full ones only
-    const uint64_t n_short = geo.flagless ? (uint64_t)geo.k - 1 : 0;
     // suffixes in the output: every position, or the chosen subset's
     const uint64_t N = sp ? sp->m : n;
-    const uint64_t n_rec = N - n_short;
+    // Distribution by leading digits (msd.cuh) for spread keys, stable LSD
+    // passes (radix.cuh) for skewed ones, whose leading digits hold little of
+    // their information and leave long pieces level after level: at an
+    // entropy of 0.64 of the code width (a word text, 50 M records of 12
+    // bytes) the MSD levels took 7.7 ms and the LSD passes 3.2 ms, at 0.7 (a
+    // masked genome, 134 M) 7.3 and 7.2 ms, at 1 (DNA, 268 M of 8 bytes) 4.5
+    // and 6.0 ms.
+    const bool use_msd = N <= msd::kOneBlock || entropy >= 0.9 * b;
+    // short suffixes of the flagless geometry; the MSD sort, whose levels do
+    // not depend on the key's width, takes them along with a flag bit
+    const uint64_t n_short = geo.flagless ? (uint64_t)geo.k - 1 : 0;
+    const bool flag_short = geo.flagless && use_msd && geo.total + 1 + geo.vbits <= 64;
+    if (flag_short) {
+        geo.lbits = geo.flag_len = 1;
+        geo.total++;
+        geo.flagless = 0;
+    }
+    // records the sort orders: every suffix, or the full ones only
+    const uint64_t n_rec = N - (geo.flagless ? n_short : 0);
     const int sort_bits = geo.total + seg_bits;
     c.stats.key_symbols = geo.k;
     c.stats.key_bits_per_symbol = geo.b;
@@ -3200,15 +3667,10 @@ capssa_status core_sort(Ctx &c, const EngineArgs &a, uint32_t **sa_out, eng::Pac
     // pass instead of 12
     const int vbits = geo.vbits;
     const int local_pos = vbits && seg_bits && geo.local_pos ? 1 : 0;
-    // Distribution by leading digits (msd.cuh) for spread keys, stable LSD
-    // passes (radix.cuh) for skewed ones, whose leading digits hold little of
-    // their information and leave long pieces level after level: at an
-    // entropy of 0.64 of the code width (a word text, 50 M records of 12
-    // bytes) the MSD levels took 7.7 ms and the LSD passes 3.2 ms, at 0.7 (a
-    // masked genome, 134 M) 7.3 and 7.2 ms, at 1 (DNA, 268 M of 8 bytes) 4.5
-    // and 6.0 ms.
-    const bool use_msd = n_rec <= msd::kOneBlock || entropy >= 0.9 * b;
     const int lsd_passes = (sort_bits + 7) / 8;
+    // packed records with a flag below the key go from the distributed chunks
+    // straight to groups
+    const bool fused = use_msd && vbits && geo.flag_len == 1;
     const msd::Plan plan =
         msd::plan(n_rec, sort_bits, seg_bits,
                   pf ? 2 * n / pf->p : (seg_bits ? a.seg_max_len : n_rec), entropy / geo.b);
@@ -3254,13 +3716,19 @@ capssa_status core_sort(Ctx &c, const EngineArgs &a, uint32_t **sa_out, eng::Pac
         if (!vbits)  // the record's value is its position
             CAPSSA_CUDA(c, cudaMemcpyAsync(vals_a, sp->pos, (size_t)N * 4, cudaMemcpyDeviceToDevice,
                                            c.stream));
-    } else if (!a.lim.segmented && !seg_bits && geo.flagless && vbits && 8 % geo.b == 0 &&
+    } else if (!a.lim.segmented && !seg_bits && (geo.flagless || flag_short) && 8 % geo.b == 0 &&
                (use_msd || (geo.total % 8 == 0 && n_rec >= 64))) {
-        key_flagless_kernel<<<kgrid, kKeyThreads, 0, c.stream>>>(P, n_rec, geo.total, vbits,
-                                                                 KeyDigits{1, td.shift, td.bits},
-                                                                 keys_a, counts);
+        const uint64_t n_full = n - n_short;
+        key_flagless_kernel<<<std::min<unsigned>(grid_for(n_full, kKeyTile), c.sm_count * 8),
+                              kKeyThreads, 0, c.stream>>>(
+            P, n_full, geo.k * geo.b, vbits, flag_short ? 1 : 0, KeyDigits{1, td.shift, td.bits},
+            keys_a, counts);
         CAPSSA_LAUNCHED(c);
-        if (!use_msd) {
+        if (flag_short) {
+            short_records_kernel<<<1, 64, 0, c.stream>>>(P, n, n_full, geo.k, vbits, td, keys_a,
+                                                         counts);
+            CAPSSA_LAUNCHED(c);
+        } else if (!use_msd) {
             key_hist_shift_kernel<<<1, 256, 0, c.stream>>>(P, n_rec, geo.total, lsd_passes, counts);
             CAPSSA_LAUNCHED(c);
         }
@@ -3276,35 +3744,7 @@ capssa_status core_sort(Ctx &c, const EngineArgs &a, uint32_t **sa_out, eng::Pac
         CAPSSA_LAUNCHED(c);
     }
     cudaEventRecord(c.pev[1], c.stream);
-    int passes = 0;
-    bool in_b = false;
-    capssa_status s;
-    if (use_msd) {
-        s = msd::sort(c, plan, keys_a, vbits ? nullptr : vals_a, keys_b, vbits ? nullptr : vals_b,
-                      (uint32_t)n_rec, vbits, sort_bits, bits_for(n - 1), geo.flag_len == 0, !sp,
-                      counts, &passes);
-        c.stats.radix_items = msd::records_per_thread(vbits == 0);
-    } else {
-        s = vbits ? radix::sort_keys(c, keys_a, keys_b, (uint32_t)n_rec, vbits, vbits + sort_bits,
-                                     &in_b, &passes, /*hist_ready=*/true)
-                  : radix::sort_pairs(c, keys_a, vals_a, keys_b, vals_b, nn, 0, sort_bits, !sp, 0,
-                                      &in_b, &passes, /*hist_ready=*/true);
-    }
-    if (s != CAPSSA_OK) return s;
-    c.stats.sort_passes = (uint32_t)passes + (use_msd ? 1u : 0u);  // with the local sort
-    c.stats.sort_item_bytes = vbits ? 8u : 12u;
-    cudaEventRecord(c.pev[2], c.stream);
-    const uint64_t *skeys = in_b ? keys_b : keys_a;
-    // packed positions are unpacked into vals_a by init_groups
-    uint32_t *sa = (in_b && !vbits) ? vals_b : vals_a;
-    // packed records are unpacked straight into a u32 output of a full build,
-    // which then needs no final copy
-    if (vbits && !a.positions && !a.keep_bits && a.out_bytes == 4 && a.out_sa)
-        sa = (uint32_t *)a.out_sa;
-    uint32_t *spare_vals = sa == vals_a ? vals_b : vals_a;
-
-    // ---- 4. tied groups: direct comparison while shallow, rank doubling when deep
-    // list capacities from the smallest group each list can hold
+    // the groups the sort leaves tied: list capacities from the smallest group each list can hold
     const size_t cap_of[kLists] = {(size_t)N / 2 + 2,  (size_t)N / 3 + 2, (size_t)N / 9 + 2,
                                    (size_t)N / 33 + 2, (size_t)N / 2 + 2, (size_t)N / 5 + 2};
     const size_t big_cap = (size_t)N / (kSmallMax + 1) + 2;
@@ -3323,23 +3763,59 @@ capssa_status core_sort(Ctx &c, const EngineArgs &a, uint32_t **sa_out, eng::Pac
         }
     G.big[0] = (BigGroup *)cursor;
     G.big[1] = G.big[0] + big_cap;
+    CAPSSA_CUDA(c, cudaMemsetAsync(G.ctr, 0, sizeof(Counters), c.stream));
+    // packed positions are unpacked into vals_a, or straight into a u32 output
+    // of a full build, which then needs no final copy
+    uint32_t *sa = vals_a;
+    if (vbits && !a.positions && !a.keep_bits && a.out_bytes == 4 && a.out_sa)
+        sa = (uint32_t *)a.out_sa;
+    const int seg_at = local_pos ? vbits + geo.total : 0;
+    int passes = 0;
+    bool in_b = false;
+    capssa_status s;
+    if (fused) {
+        const FinArgs fa{keys_a, keys_b, geo.k, lf, vbits, seg_at, a.lim.ends, hd, sa};
+        s = msd::distribute(c, plan, keys_a, keys_b, (uint32_t)n_rec, vbits, sort_bits, counts,
+                            &passes, [&](const msd::Chunks &ch) {
+                                return seg_at ? finish_chunks<true>(c, fa, ch, G)
+                                              : finish_chunks<false>(c, fa, ch, G);
+                            });
+        c.stats.radix_items = msd::records_per_thread(false);
+    } else if (use_msd) {
+        s = msd::sort(c, plan, keys_a, vbits ? nullptr : vals_a, keys_b, vbits ? nullptr : vals_b,
+                      (uint32_t)n_rec, vbits, sort_bits, bits_for(n - 1), geo.flag_len == 0, !sp,
+                      counts, &passes);
+        c.stats.radix_items = msd::records_per_thread(vbits == 0);
+    } else {
+        s = vbits ? radix::sort_keys(c, keys_a, keys_b, (uint32_t)n_rec, vbits, vbits + sort_bits,
+                                     &in_b, &passes, /*hist_ready=*/true)
+                  : radix::sort_pairs(c, keys_a, vals_a, keys_b, vals_b, nn, 0, sort_bits, !sp, 0,
+                                      &in_b, &passes, /*hist_ready=*/true);
+    }
+    if (s != CAPSSA_OK) return s;
+    c.stats.sort_passes = (uint32_t)passes + (use_msd ? 1u : 0u);  // with the local sort
+    c.stats.sort_item_bytes = vbits ? 8u : 12u;
+    cudaEventRecord(c.pev[2], c.stream);
+    const uint64_t *skeys = in_b ? keys_b : keys_a;
+    if (in_b && !vbits) sa = vals_b;
+    uint32_t *spare_vals = sa == vals_a ? vals_b : vals_a;
+
+    // ---- 4. tied groups: direct comparison while shallow, rank doubling when deep
     uint64_t h = (uint64_t)geo.k;
     KernelTimes kt(profile_on());
     kt.start(c.stream);
     // flagless: where the short suffixes go among the sorted full ones
     ShortList *d_short = nullptr;
-    if (n_short) {
+    if (geo.flagless) {
         d_short = (ShortList *)ws_get(c, WS_SAMPLE, sizeof(ShortList) + 64);
         if (!d_short) return set_err(c, CAPSSA_ENOMEM, "short suffixes");
         short_place_kernel<<<1, 64, 0, c.stream>>>(P, n, (uint32_t)n_rec, geo.k, skeys, vbits,
                                                    d_short);
         CAPSSA_LAUNCHED(c);
     }
-    CAPSSA_CUDA(c, cudaMemsetAsync(G.ctr, 0, sizeof(Counters), c.stream));
-    {
+    if (!fused) {
         const unsigned ig = grid_for(n_rec, kInitTile);
         const uint64_t lm = (1ull << geo.lbits) - 1;
-        const int seg_at = local_pos ? vbits + geo.total : 0;
 #define CAPSSA_IG(FL, UN, SG)                                                                  \
     init_groups_kernel<FL, UN, SG><<<ig, 256, 0, c.stream>>>(skeys, (uint32_t)n_rec, geo.k, lm, \
                                                              lf, vbits, hd, sa, G, d_short,      \
@@ -3358,9 +3834,9 @@ capssa_status core_sort(Ctx &c, const EngineArgs &a, uint32_t **sa_out, eng::Pac
             else CAPSSA_IG(2, true, false);
         }
 #undef CAPSSA_IG
+        CAPSSA_LAUNCHED(c);
     }
-    CAPSSA_LAUNCHED(c);
-    if (n_short) {
+    if (geo.flagless) {
         short_write_kernel<<<1, 64, 0, c.stream>>>(d_short, sa, hd);
         CAPSSA_LAUNCHED(c);
     }

@@ -42,7 +42,8 @@ constexpr int kLocalBlocks = 3;            // resident blocks per SM
 constexpr uint32_t kChunk = kLocalThreads * kLocalIt;  // records a local sort holds
 static_assert(kChunk == kOneBlock, "one block's worth");
 constexpr uint32_t kPiece = kChunk / 2;    // longest piece joined into a chunk
-constexpr uint32_t kLocalBins = 2048;
+constexpr int kLogLocalBins = 11;
+constexpr uint32_t kLocalBins = 1u << kLogLocalBins;
 constexpr uint32_t kBinMax = 48;           // records of one bin ordered by counting
 constexpr int kExtraBits = 8;              // digit of the levels past the planned ones
 
@@ -55,22 +56,10 @@ struct Tile {
 struct Counters {
     uint32_t ranges, tiles, chunks, unused;
 };
-constexpr uint32_t kInB = 0x80000000u;  // chunk length flag: the records are in the b buffers
-
-// A digit: `bits` bits at `shift` of the key, or of the position.
-struct Digit {
-    int shift, bits, from_val;
-};
-
 template <bool PAIRS>
 __device__ __forceinline__ uint32_t digit_of(uint64_t key, uint32_t val, const Digit &d) {
     if (PAIRS && d.from_val) return (val >> d.shift) & ((1u << d.bits) - 1u);
     return (uint32_t)(key >> d.shift) & ((1u << d.bits) - 1u);
-}
-
-// A chunk's keys: the digit values first .. first + span - 1 of digit dg.
-__device__ __host__ __forceinline__ uint32_t chunk_key(uint32_t span, const Digit &d) {
-    return span | (uint32_t)d.shift << 16 | (uint32_t)d.bits << 24 | (uint32_t)d.from_val << 31;
 }
 
 // Digit counts of every range (bins[range << bits | digit]), a tile at a time.
@@ -260,7 +249,7 @@ __global__ void __launch_bounds__(kThreads, 2)
 // chunk, written by the bin that starts it.
 __global__ void __launch_bounds__(256)
     pieces_kernel(const Range *__restrict__ ranges, const Counters *__restrict__ ctr, Digit dg,
-                  const uint32_t *__restrict__ bins, uint32_t tile_recs, int last,
+                  const uint32_t *__restrict__ bins, uint32_t tile_recs, int last, int runs,
                   uint32_t in_b, Range *__restrict__ next_ranges, Tile *__restrict__ next_tiles,
                   Counters *__restrict__ next, uint4 *__restrict__ chunks,
                   uint32_t *__restrict__ n_chunks) {
@@ -277,11 +266,14 @@ __global__ void __launch_bounds__(256)
         if (end - start > kPiece) {
             const uint32_t len = end - start;
             if (last) {
+                // one key: a run entry and its pieces, or pieces to sort alone
                 const uint32_t nc = (len + kChunk - 1) / kChunk;
-                const uint32_t at = atomicAdd(n_chunks, nc);
+                uint32_t at = atomicAdd(n_chunks, nc + (runs ? 1 : 0));
+                if (runs) chunks[at++] = make_uint4(start, in_b, len, kRunWhole);
                 for (uint32_t q = 0; q < nc; q++)
-                    chunks[at + q] = make_uint4(start + q * kChunk,
-                                                min(kChunk, len - q * kChunk) | in_b, d, chunk_key(1, dg));
+                    chunks[at + q] =
+                        make_uint4(start + q * kChunk, min(kChunk, len - q * kChunk) | in_b,
+                                   runs ? start : d, runs ? kRunPiece : chunk_key(1, dg));
             } else {
                 const uint32_t nt = (len + tile_recs - 1) / tile_recs;
                 const uint32_t id = atomicAdd(&next->ranges, 1u);
@@ -360,19 +352,9 @@ __global__ void __launch_bounds__(kLocalThreads, kLocalBlocks)
                 if (PAIRS) v[j] = gen_vals ? at + i : vs[at + i];
             }
         }
-        // bin of a record: its digit less the chunk's first, and the g bits below
-        const uint32_t span = ch.w & 0xFFFFu;
-        const int shift = (int)(ch.w >> 16) & 63, bits = (int)(ch.w >> 24) & 15;
+        const ChunkBins bins(ch, kLogLocalBins, 0);
         const bool fv = PAIRS && (ch.w >> 31);
-        int g = __clz((int)span) - __clz((int)kLocalBins);  // span << g <= kLocalBins
-        if (span << g > kLocalBins) g--;
-        if (g < 0) g = 0;
-        if (g > shift) g = shift;
-        const int sh = shift - g;
-        const uint32_t mask = (1u << (bits + g)) - 1u, base = ch.z << g;
-        auto bin_of = [&](uint64_t key, uint32_t val) -> uint32_t {
-            return ((fv ? val >> sh : (uint32_t)(key >> sh)) & mask) - base;
-        };
+        auto bin_of = [&](uint64_t key, uint32_t val) { return bins.of(fv ? (uint64_t)val : key); };
         for (uint32_t i = tid; i <= kLocalBins / 4; i += kLocalThreads)
             reinterpret_cast<uint4 *>(s_bin)[i] = make_uint4(0, 0, 0, 0);
         __syncthreads();
@@ -541,7 +523,8 @@ size_t scatter_smem(int bits) {
 template <bool PAIRS>
 capssa_status run(Ctx &c, const Plan &pl, uint64_t *ka, uint32_t *va, uint64_t *kb, uint32_t *vb,
                   uint32_t n, int low, int nbits, int pos_bits, bool pos_order, bool gen_vals,
-                  uint32_t *counts, int *levels_out) {
+                  uint32_t *counts, int *levels_out,
+                  const std::function<capssa_status(const Chunks &)> &finish) {
     constexpr uint32_t T = (uint32_t)kThreads * (PAIRS ? kItPairs : kItKeys);
     const size_t local_smem =
         (size_t)kChunk * (PAIRS ? 12 : 8) + ((size_t)kLocalBins + 4) * 4 + 16;
@@ -556,7 +539,7 @@ capssa_status run(Ctx &c, const Plan &pl, uint64_t *ka, uint32_t *va, uint64_t *
     // last level), two range and tile lists, the counters
     const uint64_t max_ranges = (uint64_t)n / kPiece + 2;
     const uint64_t max_tiles = (uint64_t)n / T + max_ranges + 2;
-    const uint64_t max_chunks = 5 * ((uint64_t)n / kPiece + 4) + 64;
+    const uint64_t max_chunks = 6 * ((uint64_t)n / kPiece + 4) + 64;
     auto up = [](size_t x) { return (x + 255) & ~(size_t)255; };
     const size_t bytes = 2 * up(max_chunks * 16) + 2 * up(max_ranges * sizeof(Range)) +
                          2 * up(max_tiles * sizeof(Tile)) + 4096;
@@ -582,6 +565,7 @@ capssa_status run(Ctx &c, const Plan &pl, uint64_t *ka, uint32_t *va, uint64_t *
     }
     // sorts the listed chunks (or the one given)
     auto local = [&](uint4 single) -> capssa_status {
+        if (finish) return finish(Chunks{chunks, n_chunks, single, crowded, n_crowded});
         local_kernel<PAIRS><<<single.y ? 1u : blocks * kLocalBlocks, kLocalThreads, local_smem, c.stream>>>(
             ka, va, kb, vb, single, single.y && gen_vals ? 1 : 0, chunks, n_chunks, crowded,
             n_crowded);
@@ -653,6 +637,7 @@ capssa_status run(Ctx &c, const Plan &pl, uint64_t *ka, uint32_t *va, uint64_t *
         CAPSSA_CUDA(c, cudaMemsetAsync(ctr[nxt], 0, sizeof(Counters), c.stream));
         pieces_kernel<<<(unsigned)std::min<uint64_t>((n_bins + 255) / 256, (uint64_t)blocks * 16),
                         256, 0, c.stream>>>(ranges[cur], ctr[cur], dg, bins, T, last ? 1 : 0,
+                                            finish ? 1 : 0,
                                             in_b ? 0u : kInB, ranges[nxt], tiles[nxt], ctr[nxt],
                                             chunks, n_chunks);
         CAPSSA_LAUNCHED(c);
@@ -720,9 +705,16 @@ capssa_status sort(Ctx &c, const Plan &pl, uint64_t *ka, uint32_t *va, uint64_t 
         return CAPSSA_OK;
     }
     return va ? run<true>(c, pl, ka, va, kb, vb, n, low, nbits, pos_bits, pos_order, gen_vals,
-                          counts, levels_out)
+                          counts, levels_out, nullptr)
               : run<false>(c, pl, ka, nullptr, kb, nullptr, n, low, nbits, pos_bits, pos_order,
-                           false, counts, levels_out);
+                           false, counts, levels_out, nullptr);
+}
+
+capssa_status distribute(Ctx &c, const Plan &pl, uint64_t *ka, uint64_t *kb, uint32_t n, int low,
+                         int nbits, uint32_t *counts, int *levels_out,
+                         const std::function<capssa_status(const Chunks &)> &finish) {
+    return run<false>(c, pl, ka, nullptr, kb, nullptr, n, low, nbits, 0, false, false, counts,
+                      levels_out, finish);
 }
 
 }  // namespace msd

@@ -1,6 +1,8 @@
 // msd.cuh — interface of the MSD record sort (msd.cu).
 #pragma once
 
+#include <functional>
+
 #include "common.cuh"
 
 namespace capssa {
@@ -21,6 +23,60 @@ constexpr int kMaxDigit = 12;  // bits of a planned digit
 // sized or `longest`-bounded pieces (a segment or bucket index; longest = n
 // without one); eff: bits of entropy per key bit.
 Plan plan(uint64_t n, int nbits, int top_bits, uint64_t longest, double eff);
+
+// A chunk of the distributed records, at most kOneBlock of them, holding whole
+// runs of equal keys: (start, length | kInB, first digit value, key), the key
+// packing the digit's values span, shift and width (chunk_key).  Every record
+// of a chunk agrees above that digit.
+constexpr uint32_t kInB = 0x80000000u;  // the records are in the b buffers
+struct Chunks {
+    const uint4 *list;       // device
+    const uint32_t *count;   // device
+    uint4 single;            // length > 0: this chunk alone
+    uint4 *spare;            // device, room for as many entries again
+    uint32_t *n_spare;       // device, zero
+};
+// Entries of a run of equal keys longer than a chunk, when the order of equal
+// keys is left open (see distribute): pieces (start, length | kInB, the run's
+// first index, kRunPiece) and one (start, kInB or 0, run length, kRunWhole).
+constexpr uint32_t kRunPiece = 0x80000000u, kRunWhole = 0xC0000000u;
+
+struct Digit {  // `bits` bits at `shift` of the key, or of the position
+    int shift, bits, from_val;
+};
+// span digit values: a chunk's keys are first .. first + span - 1 of digit d
+__host__ __device__ __forceinline__ uint32_t chunk_key(uint32_t span, const Digit &d) {
+    return span | (uint32_t)d.shift << 16 | (uint32_t)d.bits << 24 | (uint32_t)d.from_val << 31;
+}
+// Bin of a chunk's record among at most 2^log2_bins: its digit less the first,
+// and the bits below down to bit `low`.  Bins grow with the key.
+struct ChunkBins {
+    int sh;
+    uint32_t mask, base;
+    __device__ __forceinline__ ChunkBins(const uint4 &ch, int log2_bins, int low) {
+        const uint32_t span = ch.w & 0xFFFFu;
+        const int shift = (int)(ch.w >> 16) & 63, bits = (int)(ch.w >> 24) & 15;
+        int g = log2_bins - (31 - __clz((int)span));  // span << g <= 2^log2_bins
+        if ((span & (span - 1)) != 0) g--;
+        if (g > shift - low) g = shift - low;
+        if (g < 0) g = 0;
+        sh = shift - g;
+        mask = (1u << (bits + g)) - 1u;
+        base = ch.z << g;
+    }
+    __device__ __forceinline__ uint32_t of(uint64_t key) const {
+        return ((uint32_t)(key >> sh) & mask) - base;
+    }
+};
+
+// Distributes packed records (u64, position in the low bits, distinct) by key
+// bits [low, low + nbits) until every chunk fits one block, and calls finish
+// for each batch of chunks (it must leave the records it is given where they
+// are until it has read them; the b buffer is scratch).  Equal keys stay
+// together; a run of more than a chunk comes as kRunPiece / kRunWhole entries.
+capssa_status distribute(Ctx &c, const Plan &pl, uint64_t *ka, uint64_t *kb, uint32_t n, int low,
+                         int nbits, uint32_t *counts, int *levels_out,
+                         const std::function<capssa_status(const Chunks &)> &finish);
 
 // Sorts n records by key bits [low, low + nbits), records with equal keys by
 // position.  vals null: each u64 record carries its position in the low bits
