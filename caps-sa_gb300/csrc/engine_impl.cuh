@@ -25,7 +25,17 @@ namespace eng {
 
 constexpr uint32_t kSmallMax = 32;    // tied groups up to this size: one warp each (pairs: one thread)
 constexpr uint32_t kMediumMax = 2048; // up to this size: one block, direct comparisons
-constexpr uint64_t kDirectCap = 256;   // symbols compared past the shared prefix (at least it)
+// Symbols compared past the shared prefix in one round (at least it).  Most
+// ties of a repeat-rich text end within a few hundred symbols; the few longer
+// ones would hold their warps, and the next round takes them together.  Once a
+// round leaves less than one group in kFewLeft, the rest is few and thins out
+// (substituted copies), and another round's launches and read-back cost more
+// than the wait: it compares kDirectCapFew symbols (16 M symbols of DNA:
+// refinement 0.36 -> 0.31 ms, two rounds for three; 4 M: 0.23 -> 0.18 ms).  Not
+// from the first round on: 0.27 ms there, but exact copies of long passages,
+// which stay tied round after round, took 27 ms for 13 (50 M word text).
+constexpr uint64_t kDirectCap = 256, kDirectCapFew = 2048;
+constexpr uint64_t kFewLeft = 8;
 constexpr uint64_t kDirectMaxH = 4096; // deeper groups fall back to rank doubling
 constexpr int kKeyThreads = 256;
 constexpr int kKeyPer = 8;          // positions per thread in the key kernel
@@ -1777,12 +1787,12 @@ __global__ void __launch_bounds__(256)
 // Two-member tied groups (the bulk of the work on repeat-rich text): one
 // thread compares the pair directly past their shared depth g.z, writes
 // the SA slice and heads (and ranks once they exist), and passes a pair
-// still undecided after max(g.z, kDirectCap) more symbols to the next
+// still undecided after max(g.z, dcap) more symbols to the next
 // round with that larger depth.
 __global__ void __launch_bounds__(256, 5)
     direct_pair_kernel(const uint4 *__restrict__ groups, uint32_t count, uint32_t *__restrict__ sa,
                        uint32_t *__restrict__ hd, uint32_t *__restrict__ rank, DevLimits L,
-                       Packed P, int lf, GroupLists G, int nxt) {
+                       Packed P, int lf, uint64_t dcap, GroupLists G, int nxt) {
     const uint32_t gi = blockIdx.x * blockDim.x + threadIdx.x;
     bool again = false;
     uint4 g = make_uint4(0, 0, 0, 0);
@@ -1792,7 +1802,7 @@ __global__ void __launch_bounds__(256, 5)
         g = groups[gi];
         const bool carried = (g.z & kPairPos) != 0;  // positions in the entry
         o = g.z & ~kPairPos;
-        cap = o > kDirectCap ? o : kDirectCap;
+        cap = o > dcap ? o : dcap;
         uint32_t p0 = carried ? g.y : sa[g.x], p1 = carried ? g.w : sa[g.x + 1];
         uint64_t l0 = dev_lim_at(L, p0), l1 = dev_lim_at(L, p1);
         int r = direct_cmp<kPairBurst>(P, p0, l0, p1, l1, o, cap, lf);
@@ -1938,14 +1948,14 @@ template <int M>
 __global__ void __launch_bounds__(128)
     direct_tiny_kernel(const uint4 *__restrict__ groups, uint32_t count,
                        uint32_t *__restrict__ sa, uint32_t *__restrict__ hd,
-                       uint32_t *__restrict__ rank, DevLimits L, Packed P, int lf, GroupLists G,
-                       int nxt) {
+                       uint32_t *__restrict__ rank, DevLimits L, Packed P, int lf,
+                       uint64_t dcap, GroupLists G, int nxt) {
     for (uint32_t gi = blockIdx.x * blockDim.x + threadIdx.x; gi < count;
          gi += gridDim.x * blockDim.x) {
         const uint4 g = groups[gi];
         const int len = (int)g.y;
         const uint64_t o = g.z;
-        const uint64_t cap = o > kDirectCap ? o : kDirectCap;
+        const uint64_t cap = o > dcap ? o : dcap;
         uint32_t pp[M], lm[M];
         uint64_t minend = o + cap;  // no comparison of the group looks past this
 #pragma unroll
@@ -2062,7 +2072,7 @@ template <int S>
 __global__ void __launch_bounds__(128)
     direct_tiny_seg_kernel(const uint4 *__restrict__ groups, uint32_t count,
                            uint32_t *__restrict__ sa, uint32_t *__restrict__ hd,
-                           uint32_t *__restrict__ rank, DevLimits L, Packed P, int lf,
+                           uint32_t *__restrict__ rank, DevLimits L, Packed P, int lf, uint64_t dcap,
                            GroupLists G, int nxt) {
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t sl = lane & (S - 1), sb = lane & ~(uint32_t)(S - 1);
@@ -2071,7 +2081,7 @@ __global__ void __launch_bounds__(128)
     const int len = (int)g.y;
     const bool mine = (int)sl < len;
     const uint64_t o = g.z;
-    const uint64_t cap = o > kDirectCap ? o : kDirectCap;
+    const uint64_t cap = o > dcap ? o : dcap;
     const uint64_t horizon = o + cap;
     const uint32_t my_p = mine ? sa[g.x + sl] : 0u;
     const uint32_t my_lim = mine ? (uint32_t)dev_lim_at(L, my_p) : 0xFFFFFFFFu;
@@ -2162,7 +2172,7 @@ __global__ void __launch_bounds__(128)
 // Groups deeper than kDirectMaxH are left to rank doubling.
 __global__ void direct_warp_kernel(const uint4 *__restrict__ groups, uint32_t count,
                                    uint32_t *__restrict__ sa, uint32_t *__restrict__ hd,
-                                   uint32_t *__restrict__ rank, DevLimits L, Packed P, int lf,
+                                   uint32_t *__restrict__ rank, DevLimits L, Packed P, int lf, uint64_t dcap,
                                    GroupLists G, int nxt) {
     const uint32_t lane = threadIdx.x & 31;
     const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
@@ -2172,7 +2182,7 @@ __global__ void direct_warp_kernel(const uint4 *__restrict__ groups, uint32_t co
         const uint4 g = groups[gi];
         const uint32_t len = g.y;
         const uint64_t o = g.z;
-        const uint64_t cap = o > kDirectCap ? o : kDirectCap;
+        const uint64_t cap = o > dcap ? o : dcap;
         const uint64_t horizon = o + cap;
         const bool mine = lane < len;
         const uint32_t my_p = mine ? sa[g.x + lane] : 0u;
@@ -3847,6 +3857,7 @@ capssa_status core_sort(Ctx &c, const EngineArgs &a, uint32_t **sa_out, eng::Pac
     const uint64_t empty_lf = (1ull << k2bits) - 1;  // above every rank
     const uint64_t empty = lf ? empty_lf : 0ull;
     bool ranks_ready = false;
+    uint64_t last_groups = 0;    // small groups of the round before
     uint32_t *runs_s = nullptr;  // run ends, for the run keys of deep rounds
     int cur = 0;
     Counters *hc = (Counters *)c.h_scratch;
@@ -3895,6 +3906,10 @@ capssa_status core_sort(Ctx &c, const EngineArgs &a, uint32_t **sa_out, eng::Pac
         // next to the large medium kernel on the main one (each alone is latency-
         // bound and leaves the SMs half idle), joined before rank doubling
         CAPSSA_CUDA(c, cudaEventRecord(c.fork_ev, c.stream));
+        const uint64_t n_groups =
+            (uint64_t)cnt[L_PAIR] + cnt[L_TINY] + cnt[L_TINY8] + cnt[L_SMALL];
+        const uint64_t dcap = n_groups < last_groups / kFewLeft ? kDirectCapFew : kDirectCap;
+        last_groups = n_groups;
         int forked = 0;
         auto side = [&]() -> cudaStream_t {
             cudaStream_t st = c.side[forked];
@@ -3904,23 +3919,23 @@ capssa_status core_sort(Ctx &c, const EngineArgs &a, uint32_t **sa_out, eng::Pac
         };
         if (cnt[L_PAIR]) {
             direct_pair_kernel<<<grid_for(cnt[L_PAIR], 256), 256, 0, side()>>>(
-                G.list[L_PAIR][cur], cnt[L_PAIR], sa, hd, rk, a.lim, P, lf, G, nxt);
+                G.list[L_PAIR][cur], cnt[L_PAIR], sa, hd, rk, a.lim, P, lf, dcap, G, nxt);
             CAPSSA_LAUNCHED(c);
         }
         if (cnt[L_TINY]) {
             direct_tiny_kernel<kTiny4><<<grid_for(cnt[L_TINY], 128), 128, 0, side()>>>(
-                G.list[L_TINY][cur], cnt[L_TINY], sa, hd, rk, a.lim, P, lf, G, nxt);
+                G.list[L_TINY][cur], cnt[L_TINY], sa, hd, rk, a.lim, P, lf, dcap, G, nxt);
             CAPSSA_LAUNCHED(c);
         }
         if (cnt[L_TINY8]) {
             direct_tiny_seg_kernel<kTinyMax>
                 <<<grid_for((uint64_t)cnt[L_TINY8] * kTinyMax, 128), 128, 0, side()>>>(
-                    G.list[L_TINY8][cur], cnt[L_TINY8], sa, hd, rk, a.lim, P, lf, G, nxt);
+                    G.list[L_TINY8][cur], cnt[L_TINY8], sa, hd, rk, a.lim, P, lf, dcap, G, nxt);
             CAPSSA_LAUNCHED(c);
         }
         if (cnt[L_SMALL]) {
             direct_warp_kernel<<<grid_for((uint64_t)cnt[L_SMALL] * 32, 128), 128, 0, side()>>>(
-                G.list[L_SMALL][cur], cnt[L_SMALL], sa, hd, rk, a.lim, P, lf, G, nxt);
+                G.list[L_SMALL][cur], cnt[L_SMALL], sa, hd, rk, a.lim, P, lf, dcap, G, nxt);
             CAPSSA_LAUNCHED(c);
         }
         if (cnt[L_MEDIUM]) {

@@ -220,3 +220,29 @@ def test_record_sort_segment_major(ctx, lens):
     got = ctx.build_batched(cat, offs)
     for i, tx in enumerate(texts):
         assert np.array_equal(got[offs[i]:offs[i + 1]], orc.build_in_memory(tx)), i
+
+
+# ---------------------------------------------------------------- horizons of the direct rounds
+
+@pytest.mark.parametrize("lcp", [255, 256, 257, 600, 2303, 2304, 2305, 5000])
+def test_long_ties_across_round_horizons(ctx, lcp):
+    """Pairs and groups of 3, 7 and 20 whose common prefix ends just before,
+    at and after a round's horizon, among thousands of short ties (so that the
+    later rounds are few and look further); every seventh member is cut by a
+    segment end."""
+    rng = np.random.default_rng(lcp)
+    parts = [rng.integers(0, 4, 60000)]
+    for members in (2, 2, 3, 7, 20):
+        unit = rng.integers(0, 4, lcp)
+        for i in range(members):
+            parts += [unit, rng.integers(0, 4, 37)]
+    short = rng.integers(0, 4, 400 * 40).reshape(400, 40)
+    parts += [np.concatenate([np.concatenate([s, rng.integers(0, 4, 9)]) for s in
+                              np.repeat(short, 3, axis=0)])]
+    t = np.concatenate(parts).astype(np.uint8)
+    n = len(t)
+    assert np.array_equal(ctx.build_in_memory(t), orc.build_in_memory(t))
+    ends = np.unique(np.concatenate([rng.integers(1, n, 30), [n]]))
+    lp = capssa.SegmentedText(n, ends, capssa.BoundaryRank.LONGER_FIRST)
+    assert np.array_equal(ctx.build_in_memory(t, lp),
+                          orc.build_in_memory(t, None, orc.Limits(n, ends, True)))
