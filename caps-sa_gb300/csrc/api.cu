@@ -57,14 +57,25 @@ capssa_status cuda_err(Ctx &c, cudaError_t e, const char *where) {
     return set_err(c, CAPSSA_ECUDA, m);
 }
 
-capssa_status check_dev_flags(Ctx &c) {
-    int h[2] = {0, 0};
-    CAPSSA_CUDA(c, cudaMemcpyAsync(h, c.d_flags, 4, cudaMemcpyDeviceToHost, c.stream));
-    CAPSSA_CUDA(c, cudaStreamSynchronize(c.stream));
-    if (h[0] == DEV_LOOKBACK_TIMEOUT)
+namespace {
+
+int *flags_readback(Ctx &c) { return (int *)((char *)c.h_scratch + kScratchBytes - 64); }
+
+capssa_status flags_status(Ctx &c) {
+    const int f = *flags_readback(c);
+    if (f == DEV_LOOKBACK_TIMEOUT)
         return set_err(c, CAPSSA_ETIMEOUT, "a device-side wait exceeded its limit");
-    if (h[0] != DEV_OK) return set_err(c, CAPSSA_ECUDA, "device error flag set");
+    if (f != DEV_OK) return set_err(c, CAPSSA_ECUDA, "device error flag set");
     return CAPSSA_OK;
+}
+
+}  // namespace
+
+capssa_status check_dev_flags(Ctx &c) {
+    CAPSSA_CUDA(c, cudaMemcpyAsync(flags_readback(c), c.d_flags, 4, cudaMemcpyDeviceToHost,
+                                   c.stream));
+    CAPSSA_CUDA(c, cudaStreamSynchronize(c.stream));
+    return flags_status(c);
 }
 
 // Key geometry for b bits per symbol on a text of n symbols.  Symbols past
@@ -320,17 +331,39 @@ struct CallScope {
         c.err.clear();
         c.stats = capssa_stats{};
         c.launches = 0;
+        c.timed_passes = -1;
+        c.timed_finish = false;
         cudaSetDevice(c.device);
         cudaMemsetAsync(c.d_flags, 0, 16, c.stream);
         cudaEventRecord(c.ev0, c.stream);
     }
+    // One synchronisation for the device flags, the call's time and the
+    // phases' (each used to wait for its own: five waits a call).
     capssa_status finish(capssa_status s) {
-        if (s == CAPSSA_OK) s = check_dev_flags(c);
         cudaEventRecord(c.ev1, c.stream);
-        cudaEventSynchronize(c.ev1);
-        float ms = 0;
-        cudaEventElapsedTime(&ms, c.ev0, c.ev1);
-        c.stats.device_ms = ms;
+        const cudaError_t fe = cudaMemcpyAsync(flags_readback(c), c.d_flags, 4,
+                                               cudaMemcpyDeviceToHost, c.stream);
+        const cudaError_t se = cudaStreamSynchronize(c.stream);
+        if (s == CAPSSA_OK) {
+            if (fe != cudaSuccess) s = cuda_err(c, fe, "device flags");
+            else if (se != cudaSuccess) s = cuda_err(c, se, "call");
+            else s = flags_status(c);
+        }
+        auto ms = [](cudaEvent_t a, cudaEvent_t b) {
+            float t = 0;
+            cudaEventElapsedTime(&t, a, b);
+            return (double)t;
+        };
+        c.stats.device_ms = ms(c.ev0, c.ev1);
+        if (c.timed_passes >= 0) {
+            c.stats.keys_ms = ms(c.pev[0], c.pev[1]);
+            c.stats.sort_ms = ms(c.pev[1], c.pev[2]);
+            c.stats.refine_ms = ms(c.pev[2], c.pev[3]);
+            c.stats.sort_pass_ms = 0;
+            for (int i = 0; i < c.timed_passes && i < 16; i++)
+                c.stats.sort_pass_ms += ms(c.kev[2 * i], c.kev[2 * i + 1]);
+        }
+        if (c.timed_finish) c.stats.finish_ms = ms(c.pev[4], c.pev[5]);
         c.stats.kernel_launches = c.launches;
         cudaError_t e = cudaGetLastError();
         if (s == CAPSSA_OK && e != cudaSuccess) s = cuda_err(c, e, "call");
@@ -368,13 +401,15 @@ struct PartRequest {
     uint64_t *sizes;   // host, p
 };
 
-// Every builder funnels through here.
+// Every builder funnels through here.  deliver: the caller passes the device
+// output on to the host itself.
 template <typename ST>
 capssa_status build_common(Ctx &c, const ST *text, uint64_t n, const void *positions,
                            int pos_bytes, uint64_t m, const capssa_limits *lp,
                            const capssa_opts *opts, void *out_sa, int out_bytes, void *out_lcp,
                            const PartRequest *part = nullptr, uint64_t seg_major_len = 0,
-                           const uint32_t *keep_bits = nullptr, bool in_memory = false) {
+                           const uint32_t *keep_bits = nullptr, bool in_memory = false,
+                           bool deliver = false) {
     if (!text && n) return set_err(c, CAPSSA_EINVAL, "null text");
     if (opts && (opts->tie_order < CAPSSA_TIES_POSITION || opts->tie_order > CAPSSA_TIES_REFERENCE))
         return set_err(c, CAPSSA_EINVAL, "unknown tie order");
@@ -387,8 +422,24 @@ capssa_status build_common(Ctx &c, const ST *text, uint64_t n, const void *posit
     capssa_status s = stage_limits(c, lp, n, &L);
     if (s != CAPSSA_OK) return s;
     void *d_text = nullptr;
-    s = stage_text(c, text, n, &d_text);
-    if (s != CAPSSA_OK) return s;
+    // A device text is read in place when every kernel that will touch it stays
+    // inside it: only the alphabet, packing and run kernels do (16-byte loads
+    // of a u8 text); those of a finite context, a partition plan or the
+    // reference's tie order read past the end and need the padded copy, as does
+    // a text that the outputs overlap.  (268 M symbols: 0.08 ms.)
+    auto overlaps = [&](const void *p, uint64_t bytes) {
+        return p && (uintptr_t)p < (uintptr_t)text + n * sizeof(ST) &&
+               (uintptr_t)text < (uintptr_t)p + bytes;
+    };
+    const uint64_t out_total = (chosen ? m : n) * (uint64_t)out_bytes;
+    if (n && ((uintptr_t)text & 15) == 0 && max_ctx >= n && !part &&
+        !(opts && opts->tie_order == CAPSSA_TIES_REFERENCE) && !overlaps(out_sa, out_total) &&
+        !overlaps(out_lcp, out_total) && is_device_ptr(text)) {
+        d_text = const_cast<ST *>(text);
+    } else {
+        s = stage_text(c, text, n, &d_text);
+        if (s != CAPSSA_OK) return s;
+    }
     const uint64_t count = chosen ? m : n;
     void *d_pos = nullptr;
     if (positions && m) {
@@ -434,8 +485,11 @@ capssa_status build_common(Ctx &c, const ST *text, uint64_t n, const void *posit
     if (positions && m == 0) return CAPSSA_OK;
     s = engine_build(c, a);
     if (s != CAPSSA_OK) return s;
-    s = check_dev_flags(c);
-    if (s != CAPSSA_OK) return s;
+    if (!out_dev || (out_lcp && !lcp_dev) || deliver) {
+        // nothing reaches the host from a build whose device waits failed
+        s = check_dev_flags(c);
+        if (s != CAPSSA_OK) return s;
+    }
     if (!out_dev) {
         s = stage_out(c, out_sa, d_out, count * (size_t)out_bytes);
         if (s != CAPSSA_OK) return s;
@@ -521,7 +575,8 @@ capssa_status sample_sort_common(Ctx &c, const ST *text, uint64_t n, const uint6
                    part_mode(opts),
                    nullptr, nullptr};
     capssa_status s =
-        build_common<ST>(c, text, n, positions, 8, m, lp, opts, d_sa, 8, nullptr, &pr);
+        build_common<ST>(c, text, n, positions, 8, m, lp, opts, d_sa, 8, nullptr, &pr, 0, nullptr,
+                         false, /*deliver=*/true);
     if (s != CAPSSA_OK) return s;
     return emit_stream(c, d_sa, count, emit, user);
 }
@@ -543,7 +598,7 @@ capssa_status ext_mem_common(Ctx &c, const ST *text, uint64_t n, const void *pos
     uint64_t *d_sa = (uint64_t *)ws_get(c, WS_OUT, count * 8 + 64);
     if (!d_sa) return set_err(c, CAPSSA_ENOMEM, "output buffer");
     capssa_status s = build_common<ST>(c, text, n, positions, pos_bytes, m, lp, opts, d_sa, 8,
-                                       nullptr, nullptr, 0, keep_bits);
+                                       nullptr, nullptr, 0, keep_bits, false, /*deliver=*/true);
     if (s != CAPSSA_OK) return s;
     return emit_stream(c, d_sa, count, emit, user);
 }
@@ -835,7 +890,7 @@ capssa_status capssa_ctx_create(capssa_ctx **out, int device) {
     if (cudaSetDevice(device) != cudaSuccess ||
         cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaMalloc(&c->d_flags, 64) != cudaSuccess ||
-        cudaMallocHost(&c->h_scratch, 1 << 16) != cudaSuccess ||
+        cudaMallocHost(&c->h_scratch, kScratchBytes) != cudaSuccess ||
         cudaEventCreate(&c->ev0) != cudaSuccess || cudaEventCreate(&c->ev1) != cudaSuccess ||
         [&] {
             for (auto &e : c->pev)

@@ -145,6 +145,11 @@ struct Ctx {
     // (0 = not tuned yet), and its timing events
     int radix_shape[2][33] = {};
     cudaEvent_t tune_ev[2] = {};
+    // device times of the call's last sort and output step, taken from the
+    // events above once the call has synchronised: radix passes timed (-1: no
+    // sort ran), and whether an output step was
+    int timed_passes = -1;
+    bool timed_finish = false;
     // the last sort produced segment-major order (every segment contiguous)
     bool seg_major_done = false;
     uint64_t *h_emit = nullptr;     // pinned double buffer of the emit stream
@@ -176,6 +181,9 @@ capssa_status cuda_err(Ctx &c, cudaError_t e, const char *where);
         cudaError_t _e = cudaGetLastError();                        \
         if (_e != cudaSuccess) return ::capssa::cuda_err((c), _e, "kernel launch"); \
     } while (0)
+
+// Bytes of the pinned scratch; its last 64 are the device flags' read-back.
+constexpr size_t kScratchBytes = 1 << 16;
 
 // Device flag check: returns CAPSSA_ETIMEOUT / CAPSSA_ENOMEM after a sync.
 capssa_status check_dev_flags(Ctx &c);

@@ -36,6 +36,7 @@ constexpr uint32_t kMediumMax = 2048; // up to this size: one block, direct comp
 // which stay tied round after round, took 27 ms for 13 (50 M word text).
 constexpr uint64_t kDirectCap = 256, kDirectCapFew = 2048;
 constexpr uint64_t kFewLeft = 8;
+constexpr uint64_t kForkGroups = 1ull << 16;  // rounds of fewer groups stay on one stream
 constexpr uint64_t kDirectMaxH = 4096; // deeper groups fall back to rank doubling
 constexpr int kKeyThreads = 256;
 constexpr int kKeyPer = 8;          // positions per thread in the key kernel
@@ -62,9 +63,12 @@ constexpr int kPairBurst = 4;  // windows the pair kernel loads in its first rou
 
 // Device counters of the refinement rounds, double-buffered by round parity.
 struct Counters {
-    uint32_t n[kLists][2];
-    unsigned long long big_packed[2];  // (ordinal << 40) | element total
+    struct Half {  // cleared by one memset
+        uint32_t n[8];
+        unsigned long long big_packed;  // (ordinal << 40) | element total
+    } half[2];
 };
+static_assert(kLists <= 8, "a counter per list");
 constexpr unsigned long long kBigOrdUnit = 1ull << 40;
 constexpr unsigned long long kBigTotMask = kBigOrdUnit - 1;
 
@@ -561,7 +565,7 @@ __device__ __forceinline__ uint4 group_entry(uint32_t start, uint32_t len, uint6
 
 __device__ __forceinline__ void append_big(const GroupLists &G, int nxt, uint32_t start,
                                            uint32_t len, uint64_t depth) {
-    unsigned long long old = atomicAdd(&G.ctr->big_packed[nxt], kBigOrdUnit | len);
+    unsigned long long old = atomicAdd(&G.ctr->half[nxt].big_packed, kBigOrdUnit | len);
     uint32_t ord = (uint32_t)(old >> 40);
     BigGroup g;
     g.start = start;
@@ -594,7 +598,7 @@ __device__ __forceinline__ void append_group(const GroupLists &G, int nxt, uint3
         append_big(G, nxt, start, len, depth);
         return;
     }
-    uint32_t idx = warp_append(&G.ctr->n[l][nxt]);
+    uint32_t idx = warp_append(&G.ctr->half[nxt].n[l]);
     list_ptr(G, l, nxt)[idx] = group_entry(start, len, depth);
 }
 
@@ -611,7 +615,7 @@ __device__ __forceinline__ void block_append(const GroupLists &G, int nxt, bool 
     if (l >= 0 && l < kLists) local = atomicAdd(&s_cnt[l], 1u);
     __syncthreads();
     if (threadIdx.x < kLists && s_cnt[threadIdx.x])
-        s_base[threadIdx.x] = atomicAdd(&G.ctr->n[threadIdx.x][nxt], s_cnt[threadIdx.x]);
+        s_base[threadIdx.x] = atomicAdd(&G.ctr->half[nxt].n[threadIdx.x], s_cnt[threadIdx.x]);
     __syncthreads();
     if (l >= 0 && l < kLists) list_ptr(G, l, nxt)[s_base[l] + local] = group_entry(start, len, depth);
     if (l == kLists) append_big(G, nxt, start, len, depth);
@@ -940,7 +944,7 @@ __global__ void __launch_bounds__(256)
         const int li = (int)threadIdx.x;
         const uint32_t total =
             (uint32_t)(((li < 4 ? tot_lo : tot_hi) >> (16 * (li & 3))) & 0xFFFFu);
-        if (total) s_base[li] = atomicAdd(&G.ctr->n[li][0], total);
+        if (total) s_base[li] = atomicAdd(&G.ctr->half[0].n[li], total);
     }
     __syncthreads();
     // pass 3: write the entries of the groups found in pass 2
@@ -1086,7 +1090,7 @@ __device__ __forceinline__ void fin_flush(const FinArgs &A, FinQueue &Q, const G
         if (l != L_PAIR && l < kLists) at[j] = atomicAdd(&Q.cnt[l], 1u);
     }
     __syncthreads();
-    if (tid < kLists && Q.cnt[tid]) Q.base[tid] = atomicAdd(&G.ctr->n[tid][0], Q.cnt[tid]);
+    if (tid < kLists && Q.cnt[tid]) Q.base[tid] = atomicAdd(&G.ctr->half[0].n[tid], Q.cnt[tid]);
     if (tid == 0) Q.n = 0;
     __syncthreads();
 #pragma unroll
@@ -2327,7 +2331,7 @@ __global__ void __launch_bounds__(THREADS)
             }
         }
         __syncthreads();
-        if (tid < kLists && s_cnt[tid]) s_base[tid] = atomicAdd(&G.ctr->n[tid][nxt], s_cnt[tid]);
+        if (tid < kLists && s_cnt[tid]) s_base[tid] = atomicAdd(&G.ctr->half[nxt].n[tid], s_cnt[tid]);
         if (tid == 0) s_qn = 0;
         __syncthreads();
 #pragma unroll
@@ -3782,14 +3786,21 @@ capssa_status core_sort(Ctx &c, const EngineArgs &a, uint32_t **sa_out, eng::Pac
     const int seg_at = local_pos ? vbits + geo.total : 0;
     int passes = 0;
     bool in_b = false;
+    Counters *group_counts = (Counters *)((char *)c.h_scratch + 128);  // pinned
+    bool counts_read = false;  // ... and current: read back with the sort's own counters
     capssa_status s;
     if (fused) {
         const FinArgs fa{keys_a, keys_b, geo.k, lf, vbits, seg_at, a.lim.ends, hd, sa};
         s = msd::distribute(c, plan, keys_a, keys_b, (uint32_t)n_rec, vbits, sort_bits, counts,
                             &passes, [&](const msd::Chunks &ch) {
-                                return seg_at ? finish_chunks<true>(c, fa, ch, G)
-                                              : finish_chunks<false>(c, fa, ch, G);
-                            });
+                                const capssa_status fs = seg_at
+                                                             ? finish_chunks<true>(c, fa, ch, G)
+                                                             : finish_chunks<false>(c, fa, ch, G);
+                                if (fs != CAPSSA_OK) return fs;
+                                CAPSSA_CUDA(c, cudaMemcpyAsync(group_counts, G.ctr, sizeof(Counters),
+                                                               cudaMemcpyDeviceToHost, c.stream));
+                                return CAPSSA_OK;
+                            }, &counts_read);
         c.stats.radix_items = msd::records_per_thread(false);
     } else if (use_msd) {
         s = msd::sort(c, plan, keys_a, vbits ? nullptr : vals_a, keys_b, vbits ? nullptr : vals_b,
@@ -3860,16 +3871,19 @@ capssa_status core_sort(Ctx &c, const EngineArgs &a, uint32_t **sa_out, eng::Pac
     uint64_t last_groups = 0;    // small groups of the round before
     uint32_t *runs_s = nullptr;  // run ends, for the run keys of deep rounds
     int cur = 0;
-    Counters *hc = (Counters *)c.h_scratch;
+    Counters *hc = group_counts;
     for (;;) {
-        CAPSSA_CUDA(c, cudaMemcpyAsync(hc, G.ctr, sizeof(Counters), cudaMemcpyDeviceToHost,
-                                       c.stream));
-        CAPSSA_CUDA(c, cudaStreamSynchronize(c.stream));
+        if (!counts_read) {
+            CAPSSA_CUDA(c, cudaMemcpyAsync(hc, G.ctr, sizeof(Counters), cudaMemcpyDeviceToHost,
+                                           c.stream));
+            CAPSSA_CUDA(c, cudaStreamSynchronize(c.stream));
+        }
+        counts_read = false;
         uint32_t cnt[kLists];
         uint32_t any = 0;
-        for (int l = 0; l < kLists; l++) any |= (cnt[l] = hc->n[l][cur]);
-        const uint32_t nb = (uint32_t)(hc->big_packed[cur] >> 40);
-        const uint32_t big_total = (uint32_t)(hc->big_packed[cur] & kBigTotMask);
+        for (int l = 0; l < kLists; l++) any |= (cnt[l] = hc->half[cur].n[l]);
+        const uint32_t nb = (uint32_t)(hc->half[cur].big_packed >> 40);
+        const uint32_t big_total = (uint32_t)(hc->half[cur].big_packed & kBigTotMask);
         if (profile_on())
             std::fprintf(stderr,
                          "capssa profile  round %u depth %llu: pairs %u tiny %u+%u small %u "
@@ -3898,20 +3912,22 @@ capssa_status core_sort(Ctx &c, const EngineArgs &a, uint32_t **sa_out, eng::Pac
             kt.mark(c.stream, "ranks");
         }
         uint32_t *rk = ranks_ready ? rank : nullptr;
-        for (int l = 0; l < kLists; l++)
-            CAPSSA_CUDA(c, cudaMemsetAsync(&G.ctr->n[l][nxt], 0, 4, c.stream));
-        CAPSSA_CUDA(c, cudaMemsetAsync(&G.ctr->big_packed[nxt], 0, 8, c.stream));
+        CAPSSA_CUDA(c, cudaMemsetAsync(&G.ctr->half[nxt], 0, sizeof(G.ctr->half[0]), c.stream));
         // the direct kernels work on disjoint groups and only append to the
         // next round's lists: the small-group kinds run on side streams
         // next to the large medium kernel on the main one (each alone is latency-
         // bound and leaves the SMs half idle), joined before rank doubling
-        CAPSSA_CUDA(c, cudaEventRecord(c.fork_ev, c.stream));
         const uint64_t n_groups =
             (uint64_t)cnt[L_PAIR] + cnt[L_TINY] + cnt[L_TINY8] + cnt[L_SMALL];
         const uint64_t dcap = n_groups < last_groups / kFewLeft ? kDirectCapFew : kDirectCap;
         last_groups = n_groups;
+        // ... unless the round is small: then the forks and joins cost more than
+        // they overlap
+        const bool wide = n_groups + cnt[L_MEDIUM] >= kForkGroups;
+        if (wide) CAPSSA_CUDA(c, cudaEventRecord(c.fork_ev, c.stream));
         int forked = 0;
         auto side = [&]() -> cudaStream_t {
+            if (!wide) return c.stream;
             cudaStream_t st = c.side[forked];
             cudaStreamWaitEvent(st, c.fork_ev, 0);
             forked++;
@@ -4010,27 +4026,24 @@ capssa_status core_sort(Ctx &c, const EngineArgs &a, uint32_t **sa_out, eng::Pac
         cur = nxt;
     }
     cudaEventRecord(c.pev[3], c.stream);
-    CAPSSA_CUDA(c, cudaEventSynchronize(c.pev[3]));
-    float t01 = 0, t12 = 0, t23 = 0;
-    cudaEventElapsedTime(&t01, c.pev[0], c.pev[1]);
-    cudaEventElapsedTime(&t12, c.pev[1], c.pev[2]);
-    cudaEventElapsedTime(&t23, c.pev[2], c.pev[3]);
-    c.stats.keys_ms = t01;
-    c.stats.sort_ms = t12;
-    c.stats.refine_ms = t23;
-    double pass_ms = 0;
-    for (int i = 0; i < passes && i < 16; i++) {
-        float ms = 0;
-        cudaEventElapsedTime(&ms, c.kev[2 * i], c.kev[2 * i + 1]);
-        pass_ms += ms;
-    }
-    c.stats.sort_pass_ms = pass_ms;
-    if (profile_on())
+    c.timed_passes = passes;  // read at the end of the call
+    if (profile_on()) {
+        CAPSSA_CUDA(c, cudaEventSynchronize(c.pev[3]));
+        float t01 = 0, t12 = 0, t23 = 0, pass_ms = 0;
+        cudaEventElapsedTime(&t01, c.pev[0], c.pev[1]);
+        cudaEventElapsedTime(&t12, c.pev[1], c.pev[2]);
+        cudaEventElapsedTime(&t23, c.pev[2], c.pev[3]);
+        for (int i = 0; i < passes && i < 16; i++) {
+            float ms = 0;
+            cudaEventElapsedTime(&ms, c.kev[2 * i], c.kev[2 * i + 1]);
+            pass_ms += ms;
+        }
         std::fprintf(stderr,
                      "capssa profile  n %llu k %d b %d: keys %.3f ms, sort %.3f ms (%d passes, "
                      "%.3f ms in pass kernels), refine %.3f ms (%u rounds)\n",
                      (unsigned long long)n, geo.k, geo.b, t01, t12, passes, pass_ms, t23,
                      c.stats.refine_rounds);
+    }
     *sa_out = sa;
     *pk_out = P;
     return CAPSSA_OK;
@@ -4102,18 +4115,14 @@ inline capssa_status lcp_array(Ctx &c, const EngineArgs &a, const eng::Packed &P
     return CAPSSA_OK;
 }
 
-// Records the device time from its construction to its destruction as
-// stats.finish_ms (the output ordering and copies of a build).
+// Marks the output ordering and copies of a build, from its construction to
+// its destruction (stats.finish_ms, read at the end of the call).
 struct FinishTimer {
     Ctx &c;
     explicit FinishTimer(Ctx &cc) : c(cc) { cudaEventRecord(c.pev[4], c.stream); }
     ~FinishTimer() {
         cudaEventRecord(c.pev[5], c.stream);
-        if (cudaEventSynchronize(c.pev[5]) == cudaSuccess) {
-            float ms = 0;
-            cudaEventElapsedTime(&ms, c.pev[4], c.pev[5]);
-            c.stats.finish_ms = ms;
-        }
+        c.timed_finish = true;
     }
 };
 

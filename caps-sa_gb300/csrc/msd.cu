@@ -101,16 +101,17 @@ __global__ void __launch_bounds__(kThreads)
     }
 }
 
-// Counts -> the position of each bin's first record (a block per range).
+// Counts -> the position of each bin's first record (a block per range;
+// whole > 0: one range of that many records).
 __global__ void __launch_bounds__(256)
     offsets_kernel(const Range *__restrict__ ranges, const Counters *__restrict__ ctr, int bits,
-                   uint32_t *__restrict__ bins) {
+                   uint32_t whole, uint32_t *__restrict__ bins) {
     __shared__ uint32_t s_w[8];
-    const uint32_t R = 1u << bits, nr = ctr->ranges;
+    const uint32_t R = 1u << bits, nr = whole ? 1u : ctr->ranges;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (uint32_t r = blockIdx.x; r < nr; r += gridDim.x) {
         uint32_t *b = bins + ((uint64_t)r << bits);
-        uint32_t before = ranges[r].start;
+        uint32_t before = whole ? 0u : ranges[r].start;
         for (uint32_t d0 = 0; d0 < R; d0 += 256) {
             const uint32_t d = d0 + threadIdx.x;
             const uint32_t v = d < R ? b[d] : 0u;
@@ -248,19 +249,21 @@ __global__ void __launch_bounds__(kThreads, 2)
 // whose starts lie in the same kPiece-sized stretch of their range form one
 // chunk, written by the bin that starts it.
 __global__ void __launch_bounds__(256)
-    pieces_kernel(const Range *__restrict__ ranges, const Counters *__restrict__ ctr, Digit dg,
+    pieces_kernel(const Range *__restrict__ ranges, const Counters *__restrict__ ctr,
+                  uint32_t whole, Digit dg,
                   const uint32_t *__restrict__ bins, uint32_t tile_recs, int last, int runs,
                   uint32_t in_b, Range *__restrict__ next_ranges, Tile *__restrict__ next_tiles,
                   Counters *__restrict__ next, uint4 *__restrict__ chunks,
                   uint32_t *__restrict__ n_chunks) {
     const int bits = dg.bits;
-    const uint64_t total = (uint64_t)ctr->ranges << bits;
+    const uint64_t total = (uint64_t)(whole ? 1u : ctr->ranges) << bits;
     const uint32_t R = 1u << bits;
     for (uint64_t idx = blockIdx.x * 256ull + threadIdx.x; idx < total;
          idx += (uint64_t)gridDim.x * 256) {
         const uint32_t r = (uint32_t)(idx >> bits), d = (uint32_t)idx & (R - 1);
         const uint32_t *e = bins + ((uint64_t)r << bits);  // ends of the range's bins
-        const uint32_t s0 = ranges[r].start;
+        const Range rg = whole ? Range{0u, whole} : ranges[r];
+        const uint32_t s0 = rg.start;
         const uint32_t start = d ? e[d - 1] : s0, end = e[d];
         if (end == start) continue;
         if (end - start > kPiece) {
@@ -301,7 +304,7 @@ __global__ void __launch_bounds__(256)
         if (start != (q ? e[first_end(s0 + q * kPiece)] : s0)) continue;  // not the chunk's first bin
         // the chunk's last bin holds the stretch's end; a long one is left out
         const uint64_t stop = (uint64_t)s0 + (uint64_t)(q + 1) * kPiece;
-        const uint32_t z = stop >= (uint64_t)s0 + ranges[r].len ? R - 1 : first_end((uint32_t)stop);
+        const uint32_t z = stop >= (uint64_t)s0 + rg.len ? R - 1 : first_end((uint32_t)stop);
         uint32_t last_start = z ? e[z - 1] : s0;
         uint32_t stop_at = e[z];
         if (stop_at - last_start > kPiece) stop_at = last_start;
@@ -509,11 +512,6 @@ __global__ void __launch_bounds__(kLocalThreads)
     }
 }
 
-__global__ void whole_range_kernel(Range *r, Counters *ctr, uint32_t n) {
-    r[0] = Range{0u, n};
-    ctr->ranges = 1;
-}
-
 template <bool PAIRS>
 size_t scatter_smem(int bits) {
     const size_t T = (size_t)kThreads * (PAIRS ? kItPairs : kItKeys);
@@ -524,7 +522,8 @@ template <bool PAIRS>
 capssa_status run(Ctx &c, const Plan &pl, uint64_t *ka, uint32_t *va, uint64_t *kb, uint32_t *vb,
                   uint32_t n, int low, int nbits, int pos_bits, bool pos_order, bool gen_vals,
                   uint32_t *counts, int *levels_out,
-                  const std::function<capssa_status(const Chunks &)> &finish) {
+                  const std::function<capssa_status(const Chunks &)> &finish,
+                  bool *synced = nullptr) {
     constexpr uint32_t T = (uint32_t)kThreads * (PAIRS ? kItPairs : kItKeys);
     const size_t local_smem =
         (size_t)kChunk * (PAIRS ? 12 : 8) + ((size_t)kLocalBins + 4) * 4 + 16;
@@ -581,8 +580,6 @@ capssa_status run(Ctx &c, const Plan &pl, uint64_t *ka, uint32_t *va, uint64_t *
         const Digit all{std::min(top, 63), 1, 0};
         return local(make_uint4(0, n, 0, chunk_key(top > 63 ? 2 : 1, all)));
     }
-    whole_range_kernel<<<1, 1, 0, c.stream>>>(ranges[0], ctr[0], n);
-    CAPSSA_LAUNCHED(c);
     int key_left = nbits;                    // key bits below the digits used so far
     int val_left = PAIRS ? pos_bits : low;   // then position bits
     uint32_t nr_bound = 1;
@@ -603,6 +600,7 @@ capssa_status run(Ctx &c, const Plan &pl, uint64_t *ka, uint32_t *va, uint64_t *
             dg.shift = val_left;
             dg.from_val = PAIRS ? 1 : 0;
         }
+        const uint32_t whole = level == 0 ? n : 0u;  // one range: the whole array
         const bool last = key_left == 0 && (!pos_order || val_left == 0);
         const uint64_t n_bins = (uint64_t)nr_bound << dg.bits;
         uint32_t *bins = counts;
@@ -624,7 +622,7 @@ capssa_status run(Ctx &c, const Plan &pl, uint64_t *ka, uint32_t *va, uint64_t *
             CAPSSA_LAUNCHED(c);
         }
         offsets_kernel<<<std::min<unsigned>(nr_bound, blocks * 8), 256, 0, c.stream>>>(
-            ranges[cur], ctr[cur], dg.bits, bins);
+            ranges[cur], ctr[cur], dg.bits, whole, bins);
         CAPSSA_LAUNCHED(c);
         const size_t sm = scatter_smem<PAIRS>(dg.bits);
         if (level < 16) cudaEventRecord(c.kev[2 * level], c.stream);
@@ -636,7 +634,7 @@ capssa_status run(Ctx &c, const Plan &pl, uint64_t *ka, uint32_t *va, uint64_t *
         const int nxt = cur ^ 1;
         CAPSSA_CUDA(c, cudaMemsetAsync(ctr[nxt], 0, sizeof(Counters), c.stream));
         pieces_kernel<<<(unsigned)std::min<uint64_t>((n_bins + 255) / 256, (uint64_t)blocks * 16),
-                        256, 0, c.stream>>>(ranges[cur], ctr[cur], dg, bins, T, last ? 1 : 0,
+                        256, 0, c.stream>>>(ranges[cur], ctr[cur], whole, dg, bins, T, last ? 1 : 0,
                                             finish ? 1 : 0,
                                             in_b ? 0u : kInB, ranges[nxt], tiles[nxt], ctr[nxt],
                                             chunks, n_chunks);
@@ -654,7 +652,10 @@ capssa_status run(Ctx &c, const Plan &pl, uint64_t *ka, uint32_t *va, uint64_t *
                                        c.stream));
         CAPSSA_CUDA(c, cudaMemsetAsync(n_chunks, 0, 8, c.stream));
         CAPSSA_CUDA(c, cudaStreamSynchronize(c.stream));
-        if (hc->ranges == 0) break;
+        if (hc->ranges == 0) {
+            if (synced) *synced = true;
+            break;
+        }
         nr_bound = hc->ranges;
     }
     return CAPSSA_OK;
@@ -712,9 +713,10 @@ capssa_status sort(Ctx &c, const Plan &pl, uint64_t *ka, uint32_t *va, uint64_t 
 
 capssa_status distribute(Ctx &c, const Plan &pl, uint64_t *ka, uint64_t *kb, uint32_t n, int low,
                          int nbits, uint32_t *counts, int *levels_out,
-                         const std::function<capssa_status(const Chunks &)> &finish) {
+                         const std::function<capssa_status(const Chunks &)> &finish,
+                         bool *synced) {
     return run<false>(c, pl, ka, nullptr, kb, nullptr, n, low, nbits, 0, false, false, counts,
-                      levels_out, finish);
+                      levels_out, finish, synced);
 }
 
 }  // namespace msd

@@ -72,11 +72,13 @@ struct ChunkBins {
 // Distributes packed records (u64, position in the low bits, distinct) by key
 // bits [low, low + nbits) until every chunk fits one block, and calls finish
 // for each batch of chunks (it must leave the records it is given where they
-// are until it has read them; the b buffer is scratch).  Equal keys stay
+// are until it has read them; the b buffer is scratch).  synced: set when the
+// host has waited for the last batch.  Equal keys stay
 // together; a run of more than a chunk comes as kRunPiece / kRunWhole entries.
 capssa_status distribute(Ctx &c, const Plan &pl, uint64_t *ka, uint64_t *kb, uint32_t n, int low,
                          int nbits, uint32_t *counts, int *levels_out,
-                         const std::function<capssa_status(const Chunks &)> &finish);
+                         const std::function<capssa_status(const Chunks &)> &finish,
+                         bool *synced);
 
 // Sorts n records by key bits [low, low + nbits), records with equal keys by
 // position.  vals null: each u64 record carries its position in the low bits
