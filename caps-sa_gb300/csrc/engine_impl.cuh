@@ -1943,8 +1943,10 @@ __device__ __forceinline__ uint32_t pick32(const uint32_t (&A)[N], int q) {
 // windows (128 DNA symbols): a round loads the next four windows of
 // every member with independent loads (one round trip for the group) and
 // settles every still-undecided member pair that differs in them.  Near a
-// member's end (rare: the last symbols of a text or segment) the remaining
-// pairs are settled one by one by direct_cmp.  A member's place is the
+// member's end (the last symbols of a text or segment) the pairs of that span
+// are settled one by one by direct_cmp; the others then go on by rounds.  (To
+// settle all pairs up to the horizon there made one ended member hold its
+// group's thread for thousands of symbols.)  A member's place is the
 // count of members before it, so nothing moves until the final scatter;
 // counts (4 bits per member) and pair relations (2 bits per pair) live in
 // packed registers.
@@ -1961,7 +1963,8 @@ __global__ void __launch_bounds__(128)
         const uint64_t o = g.z;
         const uint64_t cap = o > dcap ? o : dcap;
         uint32_t pp[M], lm[M];
-        uint64_t minend = o + cap;  // no comparison of the group looks past this
+        const uint64_t horizon = o + cap;
+        uint64_t minend = horizon;  // no comparison of the group looks past this
 #pragma unroll
         for (int t = 0; t < M; t++) {
             if (t < len) {
@@ -2004,21 +2007,32 @@ __global__ void __launch_bounds__(128)
                     }
                 base += span;
             } else {
-                // a member's end or the horizon is within reach: the rest
-                // pair by pair (direct_cmp settles a pair at its end too)
+                // a member's end or the horizon is within reach: this span pair
+                // by pair (direct_cmp settles a pair at its end too); members
+                // that are not settled go on without those that are
+                const uint64_t step = horizon - base < span ? horizon - base : span;
+                uint32_t open_m = 0;  // members with an unsettled pair
                 for (uint64_t m = und64; m; m &= m - 1) {
                     const int pi = __ffsll((long long)m) - 1;
                     const int i = pi / M, j = pi % M;
                     const uint32_t a = pick32(pp, i), b = pick32(pp, j);
                     const uint32_t la = pick32(lm, i), lb = pick32(lm, j);
-                    const uint64_t done = base - o;  // symbols known equal past o
-                    const int r = direct_cmp(P, a, la, b, lb, base, cap - done, lf);
+                    const int r = direct_cmp(P, a, la, b, lb, base, step, lf);
+                    if (r == 2 && base + step < horizon) {
+                        open_m |= 1u << i | 1u << j;
+                        continue;
+                    }
+                    und64 &= ~(1ull << pi);
                     const bool i_first = r == -1 || ((r == 0 || r == 2) && a < b);
                     bef += i_first ? (1u << (4 * j)) : (1u << (4 * i));
                     if (r == 0) tie |= 1ull << pi;
                     if (r == 2) undc |= 1ull << pi;
                 }
-                und64 = 0;
+                base += step;
+                minend = horizon;
+#pragma unroll
+                for (int t = 0; t < M; t++)
+                    if (((open_m >> t) & 1u) && lm[t] < minend) minend = lm[t];
             }
         }
         // slot of each member, relation of each slot to the one before it
@@ -2069,8 +2083,9 @@ __global__ void __launch_bounds__(128)
 // the next four windows of its member (one round trip for the group),
 // exchanges them with its group by shuffles and settles its undecided
 // relations that differ in them.  Near a member's end or the horizon the
-// rest is settled by direct_cmp, the other member's position and limit
-// taken by shuffles in a loop every lane runs (no per-member arrays).  A
+// relations of that span are settled by direct_cmp, the other member's
+// position and limit taken by shuffles in a loop every lane runs (no per-member
+// arrays); what is still equal past it goes on by rounds.  A
 // member's place is the count of members before it.
 template <int S>
 __global__ void __launch_bounds__(128)
@@ -2089,17 +2104,18 @@ __global__ void __launch_bounds__(128)
     const uint64_t horizon = o + cap;
     const uint32_t my_p = mine ? sa[g.x + sl] : 0u;
     const uint32_t my_lim = mine ? (uint32_t)dev_lim_at(L, my_p) : 0xFFFFFFFFu;
-    uint32_t lmin = my_lim;
-#pragma unroll
-    for (int x = 1; x < S; x <<= 1) lmin = min(lmin, __shfl_xor_sync(0xffffffffu, lmin, x));
-    const uint64_t minend = lmin < horizon ? lmin : horizon;
     // bit u: relation with member u not settled yet
     uint32_t und = mine ? ((1u << len) - 1u) & ~(1u << sl) : 0u;
     uint32_t before = 0, tie = 0, undc = 0;  // tie / undc: bit u, relation with u
     const uint64_t span = 4 * (uint64_t)P.spw;
     uint64_t base = o;
     while (__any_sync(0xffffffffu, und != 0)) {
-        const bool fast = base + span <= minend;
+        // the nearest end among the members still undecided, or the horizon
+        uint32_t lmin = und ? my_lim : 0xFFFFFFFFu;
+#pragma unroll
+        for (int x = 1; x < S; x <<= 1) lmin = min(lmin, __shfl_xor_sync(0xffffffffu, lmin, x));
+        const bool fast = base + span <= (lmin < horizon ? lmin : horizon);
+        const uint64_t step = horizon - base < span ? horizon - base : span;
         const bool seg_busy = (__ballot_sync(0xffffffffu, und != 0) >> sb) & ((1u << S) - 1u);
         uint64_t w[4] = {0, 0, 0, 0};
         if (mine && fast && seg_busy) windows4_at(P, (uint64_t)my_p + base, w);
@@ -2122,7 +2138,9 @@ __global__ void __launch_bounds__(128)
                 const uint32_t b = __shfl_sync(0xffffffffu, my_p, sb + u);
                 const uint32_t lb = __shfl_sync(0xffffffffu, my_lim, sb + u);
                 if (!fast && ((und >> u) & 1u)) {
-                    const int r = direct_cmp(P, my_p, my_lim, b, lb, base, horizon - base, lf);
+                    const int r = direct_cmp(P, my_p, my_lim, b, lb, base, step, lf);
+                    if (r == 2 && base + step < horizon) continue;  // still equal: goes on
+                    und &= ~(1u << u);
                     const bool me_first = r == -1 || ((r == 0 || r == 2) && my_p < b);
                     before += me_first ? 0u : 1u;
                     if (r == 0) tie |= 1u << u;
@@ -2130,10 +2148,7 @@ __global__ void __launch_bounds__(128)
                 }
             }
         }
-        if (fast)
-            base += span;
-        else
-            und = 0;
+        base += fast ? span : step;
     }
     // sorted slot, relation to the slot before, tie-run heads
     const uint32_t slot = before;
@@ -2170,8 +2185,8 @@ __global__ void __launch_bounds__(128)
 // for the group) and compares them with every other member's through
 // shuffles, settling the relations that differ in them (relations settle
 // in both lanes at once, so a settled member's windows are not needed
-// again).  Near a member's end or the horizon the rest is settled by
-// direct_cmp (ties by position).  A member's place is the count of members
+// again).  Near a member's end or the horizon the relations of that span are
+// settled by direct_cmp (ties by position), the others go on by rounds.  A member's place is the count of members
 // before it, so the relation to its sorted predecessor is already known.
 // Groups deeper than kDirectMaxH are left to rank doubling.
 __global__ void direct_warp_kernel(const uint4 *__restrict__ groups, uint32_t count,
@@ -2191,14 +2206,15 @@ __global__ void direct_warp_kernel(const uint4 *__restrict__ groups, uint32_t co
         const bool mine = lane < len;
         const uint32_t my_p = mine ? sa[g.x + lane] : 0u;
         const uint32_t my_l = mine ? (uint32_t)dev_lim_at(L, my_p) : 0xFFFFFFFFu;
-        const uint32_t lmin = __reduce_min_sync(0xffffffffu, my_l);
-        const uint64_t minend = lmin < horizon ? lmin : horizon;
         const uint32_t members = len >= 32 ? 0xFFFFFFFFu : (1u << len) - 1u;
         uint32_t und = mine ? members & ~(1u << lane) : 0u;  // bit u: not settled with u
         uint32_t before = 0, tie = 0, undc = 0;  // tie / undc: bit u, relation with u
         uint64_t base = o;
         while (__any_sync(0xffffffffu, und != 0)) {
-            if (base + span <= minend) {
+            // the nearest end among the members still undecided, or the horizon
+            const uint32_t lmin = __reduce_min_sync(0xffffffffu, und ? my_l : 0xFFFFFFFFu);
+            const uint64_t step = horizon - base < span ? horizon - base : span;
+            if (base + span <= (lmin < horizon ? lmin : horizon)) {
                 uint64_t w[4] = {0, 0, 0, 0};
                 if (und) windows4_at(P, (uint64_t)my_p + base, w);
                 for (uint32_t u = 0; u < len; u++) {
@@ -2219,14 +2235,16 @@ __global__ void direct_warp_kernel(const uint4 *__restrict__ groups, uint32_t co
                     const uint32_t b = __shfl_sync(0xffffffffu, my_p, u);
                     const uint32_t lb = __shfl_sync(0xffffffffu, my_l, u);
                     if ((und >> u) & 1u) {
-                        const int r = direct_cmp(P, my_p, my_l, b, lb, base, horizon - base, lf);
+                        const int r = direct_cmp(P, my_p, my_l, b, lb, base, step, lf);
+                        if (r == 2 && base + step < horizon) continue;  // still equal: goes on
+                        und &= ~(1u << u);
                         const bool me_first = r == -1 || ((r == 0 || r == 2) && my_p < b);
                         before += me_first ? 0u : 1u;
                         if (r == 0) tie |= 1u << u;
                         if (r == 2) undc |= 1u << u;
                     }
                 }
-                und = 0;
+                base += step;
             }
         }
         // sorted slot, relation to the slot before, tie-run heads

@@ -246,3 +246,32 @@ def test_long_ties_across_round_horizons(ctx, lcp):
     lp = capssa.SegmentedText(n, ends, capssa.BoundaryRank.LONGER_FIRST)
     assert np.array_equal(ctx.build_in_memory(t, lp),
                           orc.build_in_memory(t, None, orc.Limits(n, ends, True)))
+
+
+@pytest.mark.parametrize("members", [3, 4, 5, 8, 9, 20, 32])
+@pytest.mark.parametrize("sigma", [2, 4, 6, 100])
+def test_members_that_end_inside_a_deep_group(ctx, members, sigma):
+    """Groups whose members share thousands of symbols while some of them end
+    on the way (segment ends at growing offsets, two at the same one): the
+    ended ones are settled span by span and the others go on."""
+    rng = np.random.default_rng(members * 101 + sigma)
+    unit = rng.integers(0, sigma, 2600)
+    parts, ends, at = [], [], 0
+    for i in range(members):
+        cut = [2600, 37, 130, 131, 131, 600, 2599, 1300][i % 8]
+        parts.append(unit[:cut])
+        at += cut
+        if cut < 2600 or i % 3 == 0:
+            ends.append(at)
+        tail = rng.integers(0, sigma, 11)
+        parts.append(tail)
+        at += 11
+    parts.append(rng.integers(0, sigma, 5000))
+    t = np.concatenate(parts).astype(np.uint8)
+    n = len(t)
+    ends = np.unique(np.array(ends + [n]))
+    for lf in (True, False):
+        lp = capssa.SegmentedText(n, ends, capssa.BoundaryRank.LONGER_FIRST if lf
+                                  else capssa.BoundaryRank.SHORTER_FIRST)
+        got = ctx.build_in_memory(t, lp, capssa.Opts(tie_order=capssa.TieOrder.REFERENCE))
+        assert np.array_equal(got, orc.build_in_memory(t, None, orc.Limits(n, ends, lf)))
