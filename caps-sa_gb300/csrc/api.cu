@@ -16,6 +16,7 @@
 #include "scan.cuh"
 #include "lcp.cuh"
 #include "radix.cuh"
+#include "small.cuh"
 
 namespace capssa {
 
@@ -333,6 +334,7 @@ struct CallScope {
         c.launches = 0;
         c.timed_passes = -1;
         c.timed_finish = false;
+        c.waited = false;
         cudaSetDevice(c.device);
         cudaMemsetAsync(c.d_flags, 0, 16, c.stream);
         cudaEventRecord(c.ev0, c.stream);
@@ -340,11 +342,13 @@ struct CallScope {
     // One synchronisation for the device flags, the call's time and the
     // phases' (each used to wait for its own: five waits a call).
     capssa_status finish(capssa_status s) {
-        cudaEventRecord(c.ev1, c.stream);
-        const cudaError_t fe = cudaMemcpyAsync(flags_readback(c), c.d_flags, 4,
-                                               cudaMemcpyDeviceToHost, c.stream);
-        const cudaError_t se = cudaStreamSynchronize(c.stream);
-        if (s == CAPSSA_OK) {
+        cudaError_t fe = cudaSuccess, se = cudaSuccess;
+        if (!c.waited) {
+            cudaEventRecord(c.ev1, c.stream);
+            fe = cudaMemcpyAsync(flags_readback(c), c.d_flags, 4, cudaMemcpyDeviceToHost, c.stream);
+            se = cudaStreamSynchronize(c.stream);
+        }
+        if (s == CAPSSA_OK && !c.waited) {
             if (fe != cudaSuccess) s = cuda_err(c, fe, "device flags");
             else if (se != cudaSuccess) s = cuda_err(c, se, "call");
             else s = flags_status(c);
@@ -451,6 +455,20 @@ capssa_status build_common(Ctx &c, const ST *text, uint64_t n, const void *posit
     if (!out_dev && count) {
         d_out = ws_get(c, WS_OUT, count * (size_t)out_bytes + 64);
         if (!d_out) return set_err(c, CAPSSA_ENOMEM, "output buffer");
+    }
+    // a small whole plain text: one launch (the call's last event and wait are
+    // then behind it, unless the output still goes to the host)
+    if (n && n <= kSmallText && !chosen && !part && !seg_major_len && !out_lcp && !L.segmented &&
+        max_ctx >= n) {
+        bool done = false;
+        s = small_build(c, d_text, (int)sizeof(ST), (uint32_t)n, L.longer_first, d_out, out_bytes,
+                        &done);
+        if (s != CAPSSA_OK) return s;
+        if (done) {
+            c.stats.n_suffixes = n;
+            c.waited = true;
+            return out_dev ? CAPSSA_OK : stage_out(c, out_sa, d_out, count * (size_t)out_bytes);
+        }
     }
     void *d_lcp = nullptr;
     bool lcp_dev = out_lcp && is_device_ptr(out_lcp);

@@ -150,6 +150,9 @@ struct Ctx {
     // sort ran), and whether an output step was
     int timed_passes = -1;
     bool timed_finish = false;
+    // the call's last kernel has been waited for, ev1 recorded after it (a small
+    // text, which sets no device flags)
+    bool waited = false;
     // the last sort produced segment-major order (every segment contiguous)
     bool seg_major_done = false;
     uint64_t *h_emit = nullptr;     // pinned double buffer of the emit stream

@@ -275,3 +275,45 @@ def test_members_that_end_inside_a_deep_group(ctx, members, sigma):
                                   else capssa.BoundaryRank.SHORTER_FIRST)
         got = ctx.build_in_memory(t, lp, capssa.Opts(tie_order=capssa.TieOrder.REFERENCE))
         assert np.array_equal(got, orc.build_in_memory(t, None, orc.Limits(n, ends, lf)))
+
+
+# ---------------------------------------------------------------- small texts in one block
+
+@pytest.mark.parametrize("n", [1, 2, 12, 13, 14, 33, 1023, 1024, 1025, 4099, 8191, 8192, 8193])
+@pytest.mark.parametrize("sigma,dtype", [(1, np.uint8), (2, np.uint8), (4, np.uint8),
+                                         (27, np.uint8), (256, np.uint8), (3000, np.uint16),
+                                         (65536, np.uint16), (5, np.uint32), (1 << 32, np.uint32)])
+def test_small_texts_in_one_block(ctx, n, sigma, dtype):
+    """Both sides of the largest one-block text, codes of 1 to 32 bits, both
+    boundary orders and index widths, host and device buffers."""
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(n * 31 + sigma % 1000)
+    t = rng.integers(0, sigma, n, dtype=np.uint64).astype(dtype)
+    if n > 40:
+        t[n // 2: n // 2 + n // 5] = t[: n // 5]  # a repeat, possibly deep
+        t[-7:] = t[0]
+    for lf in (False, True):
+        b = capssa.BoundaryRank.LONGER_FIRST if lf else capssa.BoundaryRank.SHORTER_FIRST
+        for index in (np.uint32, np.uint64):
+            want = orc.build_in_memory(t, None, orc.Limits(n, None, lf), index=index)
+            got = ctx.build_in_memory(t, capssa.PlainText(n, b), index=index)
+            assert np.array_equal(got, want)
+    if dtype == np.uint8:
+        for off in (0, 3):  # a device text at an odd address too
+            dt = torch.from_numpy(np.concatenate([np.zeros(off, np.uint8), t])).cuda()[off:]
+            out = torch.zeros(n + 1, dtype=torch.int32, device="cuda")
+            ctx.build_in_memory(dt, out=out[:n])
+            assert np.array_equal(out.cpu().numpy()[:n].view(np.uint32),
+                                  orc.build_in_memory(dt.cpu().numpy()))
+            assert int(out[n]) == 0
+
+
+@pytest.mark.parametrize("make", ["equal", "period", "copies", "skewed"])
+def test_small_texts_too_deep_for_one_block(ctx, make):
+    """Ties that exceed a thread's comparisons: the general path takes over."""
+    rng = np.random.default_rng(4)
+    n = 8000
+    t = {"equal": np.zeros(n, np.int64), "period": np.arange(n) % 3,
+         "copies": np.tile(rng.integers(0, 4, 500), 16),
+         "skewed": (rng.random(n) < 0.004).astype(np.int64)}[make].astype(np.uint8)
+    assert np.array_equal(ctx.build_in_memory(t), orc.build_in_memory(t))
