@@ -1446,17 +1446,19 @@ __global__ void gather_small_kernel(const uint4 *__restrict__ groups, uint32_t c
 // (a single group can hold millions: runs of one symbol): member t belongs
 // to the group whose flattened offset range holds it (groups' offsets grow
 // with their ordinals).
-// Runs of one symbol (ShorterFirst).  A tied group whose members all start
+// Runs of one symbol.  A tied group whose members all start
 // with c^h (c repeated through the depth h) is a run group: its members are
 // ordered at once by how their runs end instead of by doubling through the
 // run (a run of length L would take log2(L / h) rounds, each re-sorting the
 // whole group).  Member p with run length rr = min(run of c from p, lim):
-//   * ends at rr (the suffix is c^rr): below every continuation of c^rr;
+//   * ends at rr (the suffix is c^rr): below every continuation of c^rr
+//     (ShorterFirst), or above every one (LongerFirst);
 //   * continues with x != c at rr: c^rr x.. < c^rr' .. for rr < rr' when
 //     x < c, and > when x > c;
-// so the order is class A (x < c, or ended), ascending rr; then the members
-// whose run reaches the key's cap; then class B (x > c), descending rr; and
-// inside equal (class, rr) the rank of the suffix p + rr (0: ended).  Equal
+// so the order is class A (x < c, or ended under ShorterFirst), ascending rr;
+// then the members whose run reaches the key's cap; then class B (x > c, or
+// ended under LongerFirst), descending rr; and inside equal (class, rr) the
+// rank of the suffix p + rr (ended: first or last).  Equal
 // keys then agree on rr + h symbols (ranks are exact to the round depth h),
 // the depth their subgroup is queued with; a group deeper than h is sorted
 // by the rank at its own depth d, and its subgroups agree on d + h.
@@ -1510,19 +1512,21 @@ __global__ void gather_big_kernel(const BigGroup *__restrict__ groups, uint32_t 
             const uint64_t rl = run_from(R, p);
             const uint64_t rr = rl < lim ? rl : lim;
             uint64_t cls, rq, k2;
+            const uint64_t one = lf ? 0ull : 1ull;  // rank keys as in doubling_key
+            const uint64_t ended = lf ? empty_lf : 0ull;
             if (rr >= cap) {  // past the cap: between the two classes, by the
                 cls = 0;      // doubling key at offset cap (lim >= rr >= cap)
                 rq = cap;
-                k2 = lim > cap ? (uint64_t)__ldcg(rank + p + cap) + 1 : 0ull;
+                k2 = lim > cap ? (uint64_t)__ldcg(rank + p + cap) + one : ended;
             } else if (rr == lim) {  // ends inside the run
-                cls = 0;
-                rq = rr;
-                k2 = 0;
+                cls = lf ? 1 : 0;
+                rq = lf ? cap - 1 - rr : rr;
+                k2 = ended;
             } else {
                 const uint32_t c = code_at(R.P, p), x = code_at(R.P, p + rr);
                 cls = x < c ? 0 : 1;
                 rq = x < c ? rr : cap - 1 - rr;
-                k2 = (uint64_t)__ldcg(rank + p + rr) + 1;
+                k2 = (uint64_t)__ldcg(rank + p + rr) + one;
             }
             key = ((((((uint64_t)lo << 1) | cls) << R.rbits) | rq) << k2bits) | k2;
         } else {
@@ -4003,11 +4007,13 @@ capssa_status core_sort(Ctx &c, const EngineArgs &a, uint32_t **sa_out, eng::Pac
         }
         const int ord_bits = nb > 1 ? bits_for(nb - 1) : 1;
         if (nb) {
-            // run keys for ShorterFirst whole texts, when a run-length field
-            // of at least 12 bits fits beside the ordinal and the rank
+            // run keys for whole texts, when a run-length field of at least 12
+            // bits fits beside the ordinal and the rank (a masked genome of 40 M
+            // symbols, runs up to 50,000, LongerFirst: 12 rounds of doubling and
+            // 3.5 ms of refinement without them, 2.2 ms with them)
             RunKeys R{nullptr, P, n, 0};
             const int rbits = std::min(24, 64 - ord_bits - 1 - k2bits);
-            if (!lf && !sp && rbits >= 12 && h >= 2 * (uint64_t)geo.k) {
+            if (!sp && rbits >= 12 && h >= 2 * (uint64_t)geo.k) {
                 if (!runs_s) {  // built once, the first deep round that can use it
                     runs_s = (uint32_t *)ws_get(c, WS_RUNS, (size_t)n * 4 + 64);
                     if (!runs_s) return set_err(c, CAPSSA_ENOMEM, "run lengths");

@@ -317,3 +317,28 @@ def test_small_texts_too_deep_for_one_block(ctx, make):
          "copies": np.tile(rng.integers(0, 4, 500), 16),
          "skewed": (rng.random(n) < 0.004).astype(np.int64)}[make].astype(np.uint8)
     assert np.array_equal(ctx.build_in_memory(t), orc.build_in_memory(t))
+
+
+# ---------------------------------------------------------------- run groups, longer first
+
+@pytest.mark.parametrize("n,longest", [(1 << 17, 900), (1 << 20, 3000), (1 << 20, 70000)])
+def test_run_groups_longer_first(ctx, n, longest):
+    """Deep groups of run suffixes under LongerFirst: runs of every symbol that
+    end in a smaller symbol, a larger one, a segment end (several of the same
+    length, ordered by position) or the text's end, plain and segmented."""
+    rng = np.random.default_rng(n + longest)
+    t = rng.integers(0, 6, n).astype(np.uint8)
+    ends = np.unique(np.concatenate([rng.integers(1, n, 200), [n]]))
+    for c in range(6):
+        for _ in range(12):
+            L = int(rng.integers(longest // 10, longest))
+            e = int(ends[rng.integers(0, len(ends))]) if rng.random() < 0.4 else None
+            a = max(0, e - L) if e is not None else int(rng.integers(0, n - L))
+            t[a:a + L] = c
+    t[n - 400:] = 3
+    lp = capssa.PlainText(n, capssa.BoundaryRank.LONGER_FIRST)
+    assert np.array_equal(ctx.build_in_memory(t, lp),
+                          orc.build_in_memory(t, None, orc.Limits(n, None, True)))
+    lp = capssa.SegmentedText(n, ends, capssa.BoundaryRank.LONGER_FIRST)
+    assert np.array_equal(ctx.build_in_memory(t, lp),
+                          orc.build_in_memory(t, None, orc.Limits(n, ends, True)))
