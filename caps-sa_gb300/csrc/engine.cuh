@@ -79,7 +79,10 @@ struct KeyGeom {
     int k;         // symbols per key
     int lbits;     // bits of the length field
     int total;     // k*b + lbits
-    int flag_len;  // 1: the length field is one "ended early" flag (plain texts)
+    // 1: the length field is one "ended early" flag (plain texts); 3: none,
+    // the codes leave the padding (0, or all ones under LongerFirst) free, so a
+    // key that ends in it ended early
+    int flag_len;
     int vbits;     // > 0: the position is packed below the key in vbits bits
     // 1: no length field at all (lbits 0, flag_len 2).  Only for ShorterFirst
     // plain texts, when the flag bit alone would cost a radix pass: the k - 1
@@ -97,8 +100,10 @@ struct KeyGeom {
 // a ShorterFirst plain text may drop the early-end flag (see KeyGeom);
 // seg_flag: a segment-major ShorterFirst sort may mark the suffixes that end
 // inside the key with one flag bit instead of a length field.
+// pad_codes: no symbol's code is 0 or all ones.
 KeyGeom key_geom(int b, uint64_t n, bool plain, double hbits, int top_bits = 0,
-                 uint64_t n_k = 0, bool allow_flagless = false, bool seg_flag = false);
+                 uint64_t n_k = 0, bool allow_flagless = false, bool seg_flag = false,
+                 bool pad_codes = false);
 
 // Key geometry of a partition-first sort: a bucket index of bucket_bits
 // above a window of k symbols taken after the bucket's common prefix, a

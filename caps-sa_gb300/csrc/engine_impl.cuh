@@ -166,8 +166,17 @@ __global__ void __launch_bounds__(256)
         }
 }
 
+// First code of sigma dense codes in their bits_for(sigma - 1) bits: 1 when
+// that leaves both 0 and the largest code free for the padding of suffixes
+// that end inside a key (see KeyGeom::flag_len), else 0.
+__host__ __device__ __forceinline__ uint32_t code_base(uint64_t sigma) {
+    uint64_t room = 2;
+    while (room < sigma) room *= 2;
+    return sigma + 2 <= room ? 1u : 0u;
+}
+
 // One block: the dense order-preserving codes of the present values (u8 /
-// u16; code = present values below, as Packer::new assigns them,
+// u16; code = code_base + present values below, as Packer::new assigns them,
 // src/pack.rs:103-167) with their number, and the sample's entropy.  Each
 // value's share is rounded to 1 / kEntropyUnit before it is added, so the sum does not
 // depend on the order of the threads (float: the chip's few FP64 lanes took
@@ -206,8 +215,13 @@ __global__ void __launch_bounds__(1024)
         }
         if (lane == 31) s_w[warp] = x;
         __syncthreads();
-        uint32_t c = x - mine;
-        for (uint32_t w = 0; w < warp; w++) c += s_w[w];
+        uint32_t c = x - mine, sigma = 0;
+        for (uint32_t w = 0; w < 32; w++) {
+            if (w < warp) c += s_w[w];
+            sigma += s_w[w];
+        }
+        if (tid == 0) info->hi = sigma;
+        c += code_base(sigma);
         if (kPer == 1) {
             if (v0 < kVals) code[v0] = (uint16_t)c;
         } else {
@@ -223,7 +237,6 @@ __global__ void __launch_bounds__(1024)
                 c4[q / 8] = make_uint4(w[0], w[1], w[2], w[3]);
             }
         }
-        if (tid == 1023) info->hi = c + mine;
     }
     if (!ns) return;
     constexpr uint32_t kCnts = sizeof(S) == 1 ? 256 : sizeof(S) == 2 ? 65536 : kEntropySlots;
@@ -882,6 +895,9 @@ __global__ void __launch_bounds__(256)
         if (flag_len == 2) {  // no length field: every record is a full suffix
             complete = false;
             depth = (uint64_t)k;
+        } else if (flag_len == 3) {  // the last symbol is padding, or not
+            complete = lenf == (lf ? (uint32_t)lmask : 0u);
+            depth = (uint64_t)k;
         } else if (flag_len) {
             complete = false;
             depth = lenf == (lf ? 0u : 1u) ? (uint64_t)k : 0ull;
@@ -903,7 +919,7 @@ __global__ void __launch_bounds__(256)
     uint64_t cnt_lo = 0, cnt_hi = 0;  // 16-bit counts: lists 0..3, lists 4..
     uint32_t ends = 0;                 // bit j: key j ends a group that needs refining
     // only LongerFirst with a length field separates complete ties by position
-    const bool lf_field = lf && !flag_len;
+    const bool lf_field = lf && (flag_len == 0 || flag_len == 3);
     // pass 2: the group members' heads, and the groups this thread ends
     auto pass1 = [&](auto fast_c) {
         constexpr bool FAST = decltype(fast_c)::value;
@@ -3627,9 +3643,11 @@ capssa_status core_sort(Ctx &c, const EngineArgs &a, uint32_t **sa_out, eng::Pac
                                    c.stream));
     CAPSSA_CUDA(c, cudaStreamSynchronize(c.stream));
     const uint16_t *table = sizeof(S) <= 2 ? d_code : nullptr;
-    const uint32_t minv = sizeof(S) <= 2 ? 0u : ~h_info->lo;
     const uint64_t sigma_span =
-        sizeof(S) <= 2 ? h_info->hi : (uint64_t)h_info->hi - minv + 1;
+        sizeof(S) <= 2 ? h_info->hi : (uint64_t)h_info->hi - (uint32_t)~h_info->lo + 1;
+    const bool pad_codes = code_base(sigma_span) != 0;
+    // (u32 codes are s - minv; minv wraps below 0 for a smallest symbol of 0)
+    const uint32_t minv = sizeof(S) <= 2 ? 0u : ~h_info->lo - code_base(sigma_span);
     const int b = bits_for(sigma_span > 1 ? sigma_span - 1 : 1);
     double hbits = (double)b, entropy = (double)b;
     if (sampled) {
@@ -3659,7 +3677,7 @@ capssa_status core_sort(Ctx &c, const EngineArgs &a, uint32_t **sa_out, eng::Pac
     } else {
         geo = key_geom(b, n, !a.lim.segmented, hbits, seg_bits,
                        seg_bits ? a.seg_max_len : (sp ? sp->m : 0), allow_flagless,
-                       a.seg_major && !lf);
+                       a.seg_major && !lf, pad_codes);
     }
     // suffixes in the output: every position, or the chosen subset's
     const uint64_t N = sp ? sp->m : n;
@@ -3826,7 +3844,8 @@ capssa_status core_sort(Ctx &c, const EngineArgs &a, uint32_t **sa_out, eng::Pac
         c.stats.radix_items = msd::records_per_thread(false);
     } else if (use_msd) {
         s = msd::sort(c, plan, keys_a, vbits ? nullptr : vals_a, keys_b, vbits ? nullptr : vals_b,
-                      (uint32_t)n_rec, vbits, sort_bits, bits_for(n - 1), geo.flag_len == 0, !sp,
+                      (uint32_t)n_rec, vbits, sort_bits, bits_for(n - 1),
+                      geo.flag_len == 0 || geo.flag_len == 3, !sp,
                       counts, &passes);
         c.stats.radix_items = msd::records_per_thread(vbits == 0);
     } else {
@@ -3858,7 +3877,7 @@ capssa_status core_sort(Ctx &c, const EngineArgs &a, uint32_t **sa_out, eng::Pac
     }
     if (!fused) {
         const unsigned ig = grid_for(n_rec, kInitTile);
-        const uint64_t lm = (1ull << geo.lbits) - 1;
+        const uint64_t lm = (1ull << (geo.flag_len == 3 ? geo.b : geo.lbits)) - 1;
 #define CAPSSA_IG(FL, UN, SG)                                                                  \
     init_groups_kernel<FL, UN, SG><<<ig, 256, 0, c.stream>>>(skeys, (uint32_t)n_rec, geo.k, lm, \
                                                              lf, vbits, hd, sa, G, d_short,      \
@@ -3866,14 +3885,17 @@ capssa_status core_sort(Ctx &c, const EngineArgs &a, uint32_t **sa_out, eng::Pac
         if (!vbits) {
             if (geo.flag_len == 0) CAPSSA_IG(0, false, false);
             else if (geo.flag_len == 1) CAPSSA_IG(1, false, false);
+            else if (geo.flag_len == 3) CAPSSA_IG(3, false, false);
             else CAPSSA_IG(2, false, false);
         } else if (seg_at) {
             if (geo.flag_len == 0) CAPSSA_IG(0, true, true);
             else if (geo.flag_len == 1) CAPSSA_IG(1, true, true);
+            else if (geo.flag_len == 3) CAPSSA_IG(3, true, true);
             else CAPSSA_IG(2, true, true);
         } else {
             if (geo.flag_len == 0) CAPSSA_IG(0, true, false);
             else if (geo.flag_len == 1) CAPSSA_IG(1, true, false);
+            else if (geo.flag_len == 3) CAPSSA_IG(3, true, false);
             else CAPSSA_IG(2, true, false);
         }
 #undef CAPSSA_IG

@@ -342,3 +342,38 @@ def test_run_groups_longer_first(ctx, n, longest):
     lp = capssa.SegmentedText(n, ends, capssa.BoundaryRank.LONGER_FIRST)
     assert np.array_equal(ctx.build_in_memory(t, lp),
                           orc.build_in_memory(t, None, orc.Limits(n, ends, True)))
+
+
+# ---------------------------------------------------------------- keys whose padding shows the end
+
+@pytest.mark.parametrize("sigma,dtype", [(5, np.uint8), (6, np.uint8), (7, np.uint8), (9, np.uint8),
+                                         (14, np.uint8), (15, np.uint8), (126, np.uint8),
+                                         (127, np.uint8), (510, np.uint16), (511, np.uint16),
+                                         (6, np.uint32), (30000, np.uint32)])
+def test_padding_codes_on_both_sides_of_the_rule(ctx, sigma, dtype):
+    """Alphabets that leave the codes 0 and all-ones free (no length field in
+    the key) and the next larger ones that do not; many suffixes end inside
+    the key, in ties of both kinds, under both boundary orders; whole texts,
+    subsets, and texts that hold the smallest and largest u32 symbols."""
+    rng = np.random.default_rng(sigma)
+    n = 30000
+    t = rng.integers(0, sigma, n)
+    t[:sigma] = np.arange(sigma)[:n]
+    t[9000:9400] = t[400:800]
+    if dtype == np.uint32:
+        t = t + (0 if sigma == 6 else (1 << 32) - sigma)
+    t = t.astype(dtype)
+    ends = np.unique(np.concatenate([rng.integers(1, n, 6000), [9200, 600, n]]))
+    t[ends[::3] - 1] = t[0]  # many equal short endings
+    keep = np.sort(rng.choice(n, 20000, replace=False)).astype(np.uint32)
+    few = np.sort(rng.choice(n, 2500, replace=False)).astype(np.uint32)
+    for lf in (False, True):
+        lp = capssa.SegmentedText(n, ends, capssa.BoundaryRank.LONGER_FIRST if lf
+                                  else capssa.BoundaryRank.SHORTER_FIRST)
+        lo = orc.Limits(n, ends, lf)
+        opts = capssa.Opts(tie_order=capssa.TieOrder.REFERENCE)
+        assert np.array_equal(ctx.build_in_memory(t, lp, opts), orc.build_in_memory(t, None, lo))
+        for pos in (keep, few):
+            assert np.array_equal(ctx.build_in_memory_for_positions(t, pos, lp, opts),
+                                  orc.build_in_memory(t, pos, lo))
+    assert np.array_equal(ctx.build_in_memory(t), orc.build_in_memory(t))
