@@ -377,3 +377,24 @@ def test_padding_codes_on_both_sides_of_the_rule(ctx, sigma, dtype):
             assert np.array_equal(ctx.build_in_memory_for_positions(t, pos, lp, opts),
                                   orc.build_in_memory(t, pos, lo))
     assert np.array_equal(ctx.build_in_memory(t), orc.build_in_memory(t))
+
+
+# ---------------------------------------------------------------- packing
+
+@pytest.mark.parametrize("values", [[0, 1], [7, 8], [0, 1, 2, 3], [200, 201, 202], [65, 67, 71, 84],
+                                    list(range(252, 256)), list(range(9)), list(range(5, 21)),
+                                    list(range(0, 28, 2)), list(range(256)), list(range(60, 260 - 60)),
+                                    [255]])
+@pytest.mark.parametrize("n", [16384, 16384 + 31, 40961])
+def test_packing_of_consecutive_and_scattered_values(ctx, values, n):
+    """Codes of 1, 2, 4 and 8 bits from consecutive byte values (coded without a
+    table, from 0, from the middle and up to 255) and from scattered ones;
+    lengths that end inside, at and just past a word."""
+    rng = np.random.default_rng(len(values) + n)
+    t = np.array(values, dtype=np.uint8)[rng.integers(0, len(values), n)]
+    t[: len(values)] = values
+    t[n - 50:] = t[: 50]
+    if len(values) == 1:
+        assert np.array_equal(ctx.build_in_memory(t), np.arange(n - 1, -1, -1))
+    else:
+        assert np.array_equal(ctx.build_in_memory(t), orc.build_in_memory(t))
