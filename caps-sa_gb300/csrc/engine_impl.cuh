@@ -36,6 +36,15 @@ constexpr uint32_t kMediumMax = 2048; // up to this size: one block, direct comp
 // which stay tied round after round, took 27 ms for 13 (50 M word text).
 constexpr uint64_t kDirectCap = 256, kDirectCapFew = 2048;
 constexpr uint64_t kFewLeft = 8;
+// Groups of 9..32 of a text with few symbols a window (codes of 4 bits and
+// more) go through the block kernel's window steps, one warp a group: such keys
+// hold few symbols, so most members part within a window or two, and what
+// stays tied queues by its own size instead of staying with a warp of 32 up to
+// the round's horizon (50 M symbols of words, 308,158 such groups after the
+// key: 0.63 ms for 2.87 in all rounds).  Not for few of them: the rounds this
+// adds cost more (8 M tokens, 153 groups: refinement 0.72 ms for 0.50).
+constexpr int kNarrowSpw = 16;
+constexpr uint32_t kManySmall = 1u << 14;
 constexpr uint64_t kForkGroups = 1ull << 16;  // rounds of fewer groups stay on one stream
 constexpr uint64_t kDirectMaxH = 4096; // deeper groups fall back to rank doubling
 constexpr int kKeyThreads = 256;
@@ -2358,8 +2367,9 @@ __global__ void direct_warp_kernel(const uint4 *__restrict__ groups, uint32_t co
     }
 }
 
-// Tied groups of kLo + 1 .. MAXM members (33 .. kMediumMax over the two
-// instantiations): one block per group, window by window.  Each step reads
+// Tied groups of kLo + 1 .. MAXM members (33 .. kMediumMax over two
+// instantiations, and 9 .. 32 by a third, see kNarrowSpw): one block per group,
+// window by window.  Each step reads
 // the next window of every member still tied (one round trip for the group:
 // bound by those random L2 reads), orders each tied subgroup by it inside
 // shared memory, and splits the subgroups where windows differ; a window that
@@ -4072,7 +4082,12 @@ capssa_status core_sort(Ctx &c, const EngineArgs &a, uint32_t **sa_out, eng::Pac
                     G.list[L_TINY8][cur], cnt[L_TINY8], sa, hd, rk, a.lim, P, lf, dcap, G, nxt);
             CAPSSA_LAUNCHED(c);
         }
-        if (cnt[L_SMALL]) {
+        if (P.spw <= kNarrowSpw && cnt[L_SMALL] >= kManySmall) {
+            direct_medium_kernel<kTinyMax, kSmallMax, 32>
+                <<<std::min<unsigned>(cnt[L_SMALL], c.sm_count * 32), 32, 0, side()>>>(
+                    G.list[L_SMALL][cur], cnt[L_SMALL], sa, hd, rk, a.lim, P, lf, h, G, nxt);
+            CAPSSA_LAUNCHED(c);
+        } else if (cnt[L_SMALL]) {
             direct_warp_kernel<<<grid_for((uint64_t)cnt[L_SMALL] * 32, 128), 128, 0, side()>>>(
                 G.list[L_SMALL][cur], cnt[L_SMALL], sa, hd, rk, a.lim, P, lf, dcap, G, nxt);
             CAPSSA_LAUNCHED(c);

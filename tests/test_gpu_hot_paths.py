@@ -277,6 +277,32 @@ def test_members_that_end_inside_a_deep_group(ctx, members, sigma):
         assert np.array_equal(got, orc.build_in_memory(t, None, orc.Limits(n, ends, lf)))
 
 
+@pytest.mark.parametrize("groups", [2000, 17000])
+@pytest.mark.parametrize("sigma", [9, 16, 20, 200])
+def test_groups_of_9_to_32_in_narrow_windows(ctx, groups, sigma):
+    """Groups of 8, 9, 10, 31, 32 and 33 members that part at, before and well
+    after a window's edge, fewer and more of them than the rule of the block
+    kernel asks for; some members end inside the shared part (both boundary
+    orders) and some never part."""
+    rng = np.random.default_rng(sigma + groups)
+    sizes = np.where(np.arange(groups) % 50 == 0, 32, 9)
+    sizes[1::400], sizes[2::400], sizes[3::400], sizes[4::400] = 8, 10, 31, 33
+    unit = rng.integers(0, sigma, (groups, 30))
+    rows = np.repeat(unit, sizes, axis=0)
+    cut = rng.integers(17, 31, len(rows))
+    other = rng.integers(0, sigma, rows.shape)
+    rows = np.where(np.arange(30)[None, :] < cut[:, None], rows, other)
+    t = np.concatenate([rows.ravel(), np.tile(unit[:7].ravel(), 20)]).astype(np.uint8)
+    n = len(t)
+    assert np.array_equal(ctx.build_in_memory(t), orc.build_in_memory(t))
+    ends = np.unique(np.concatenate([rng.integers(1, n, n // 200), [n]]))
+    for lf in (True, False):
+        lp = capssa.SegmentedText(n, ends, capssa.BoundaryRank.LONGER_FIRST if lf
+                                  else capssa.BoundaryRank.SHORTER_FIRST)
+        got = ctx.build_in_memory(t, lp, capssa.Opts(tie_order=capssa.TieOrder.REFERENCE))
+        assert np.array_equal(got, orc.build_in_memory(t, None, orc.Limits(n, ends, lf)))
+
+
 # ---------------------------------------------------------------- small texts in one block
 
 @pytest.mark.parametrize("n", [1, 2, 12, 13, 14, 33, 1023, 1024, 1025, 4099, 8191, 8192, 8193])
