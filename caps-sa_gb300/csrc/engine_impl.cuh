@@ -186,9 +186,9 @@ __host__ __device__ __forceinline__ uint32_t code_base(uint64_t sigma) {
     return sigma + 2 <= room ? 1u : 0u;
 }
 
-// One block: the dense order-preserving codes of the present values (u8 /
+// The first block: the dense order-preserving codes of the present values (u8 /
 // u16; code = code_base + present values below, as Packer::new assigns them,
-// src/pack.rs:103-167) with their number, and the sample's entropy.  Each
+// src/pack.rs:103-167) with their number; all blocks: the sample's entropy.  Each
 // value's share is rounded to 1 / kEntropyUnit before it is added, so the sum does not
 // depend on the order of the threads (float: the chip's few FP64 lanes took
 // 1.6 ms for the 26,000 logarithms of an 8.0 M-token text).
@@ -200,7 +200,7 @@ __global__ void __launch_bounds__(1024)
                            uint16_t *__restrict__ code) {
     __shared__ uint32_t s_w[32], s_range[2];
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    if (sizeof(S) <= 2) {
+    if (sizeof(S) <= 2 && blockIdx.x == 0) {
         constexpr uint32_t kVals = sizeof(S) == 1 ? 256 : 65536;
         constexpr uint32_t kPer = kVals < 1024 ? 1 : kVals / 1024;
         const uint32_t v0 = tid * kPer;
@@ -262,7 +262,7 @@ __global__ void __launch_bounds__(1024)
     constexpr uint32_t kCnts = sizeof(S) == 1 ? 256 : sizeof(S) == 2 ? 65536 : kEntropySlots;
     unsigned long long sum = 0;
 #pragma unroll 16
-    for (uint32_t i = tid; i < kCnts; i += 1024) {
+    for (uint32_t i = blockIdx.x * 1024 + tid; i < kCnts; i += gridDim.x * 1024) {
         const uint32_t q = sizeof(S) <= 2 ? cnt[i] : (uint32_t)(slots[i] & 0xFFFFFu);
         if (q) sum += (unsigned long long)((float)q * log2f((float)ns / q) * kEntropyUnit);
     }
@@ -3708,7 +3708,9 @@ capssa_status core_sort(Ctx &c, const EngineArgs &a, uint32_t **sa_out, eng::Pac
     alphabet_kernel<S><<<std::min<unsigned>(grid_for(n, 256), c.sm_count * 8), 256, 0, c.stream>>>(
         text, n, ns, stride, d_info, present, cnts, (unsigned long long *)cnts);
     CAPSSA_LAUNCHED(c);
-    alphabet_finish_kernel<S><<<1, 1024, 0, c.stream>>>(d_info, present, cnts,
+    // (one block for the 131,072 slots of u32 symbols: 77 us)
+    const unsigned fold = !sampled || sizeof(S) == 1 ? 1u : sizeof(S) == 2 ? 16u : 64u;
+    alphabet_finish_kernel<S><<<fold, 1024, 0, c.stream>>>(d_info, present, cnts,
                                                         (const unsigned long long *)cnts,
                                                         sampled ? ns : 0, d_code);
     CAPSSA_LAUNCHED(c);
