@@ -141,9 +141,9 @@ struct Ctx {
     cudaEvent_t pev[8] = {};        // phase boundaries of one suffix sort
     cudaEvent_t kev[2 * 16] = {};   // around each radix pass of the initial sort
     int sm_count = 0;
-    // radix autotuner: chosen records per thread by [packed records?][log2 n]
-    // (0 = not tuned yet), and its timing events
-    int radix_shape[2][33] = {};
+    // radix autotuner: chosen records per thread of sorts of keys alone, by
+    // log2 n (0 = not tuned yet), and its timing events
+    int radix_shape[33] = {};
     cudaEvent_t tune_ev[2] = {};
     // device times of the call's last sort and output step, taken from the
     // events above once the call has synchronised: radix passes timed (-1: no

@@ -163,8 +163,8 @@ typedef struct capssa_stats {
     uint64_t partition_probes;  /* suffix-vs-splitter comparisons of the partition */
     uint32_t train_samples;     /* learned partition: samples the model trained on */
     float model_loss;           /* learned partition: final mean squared CDF error */
-    uint32_t radix_items;       /* records per thread of the radix passes (the context's
-                                   autotuner picks it on its first large sort of each kind) */
+    uint32_t radix_items;       /* records per thread of the radix passes (for keys alone the context's
+                                   autotuner picks it on its first large sort) */
     uint32_t sparse_subset;     /* 1: a subset build sorted only its own positions */
     uint32_t tie_classes;       /* tie classes of the output (CAPSSA_TIES_REFERENCE) */
     uint32_t reserved_u32;

@@ -182,6 +182,44 @@ def test_record_sort_sizes_and_skew(ctx, n, kind):
     assert np.array_equal(got, orc.build_in_memory(t))
 
 
+@pytest.mark.parametrize("n", [4095, 4096, 4097, 5119, 5121, 40960, 40961, (1 << 22) + 3])
+@pytest.mark.parametrize("p", [0.05, 0.35, 0.7])
+def test_skewed_record_sort_at_tile_edges(ctx, n, p):
+    """Stable passes over uneven keys: tiles of 4,096 and 5,120 records that are
+    full, one short and one over, and a size whose first pass times every
+    shape; records of key and position in one word and as pairs."""
+    rng = np.random.default_rng(n + int(100 * p))
+    t = np.minimum(rng.geometric(p, n) - 1, 250).astype(np.uint8)
+    assert np.array_equal(ctx.build_in_memory(t), orc.build_in_memory(t))
+    ends = np.unique(np.concatenate([rng.integers(1, n, 20), [n]]))
+    got = ctx.build_in_memory(t, capssa.SegmentedText(n, ends, capssa.BoundaryRank.LONGER_FIRST))
+    assert np.array_equal(got, orc.build_in_memory(t, None, orc.Limits(n, ends, True)))
+
+
+def test_skewed_record_sort_of_over_2p30_records(ctx):
+    """Digit counts above 2^30 need the wide status words: a permutation, and
+    neighbours at two million ranks in order (symbol by symbol)."""
+    torch = pytest.importorskip("torch")
+    n = (1 << 30) + 4097
+    g = torch.Generator(device="cuda").manual_seed(5)
+    t = torch.randint(0, 16, (n,), dtype=torch.uint8, device="cuda", generator=g)
+    t &= torch.randint(0, 16, (n,), dtype=torch.uint8, device="cuda", generator=g)
+    sa = torch.empty(n, dtype=torch.int32, device="cuda")
+    ctx.build_in_memory(t, out=sa)
+    seen = torch.zeros(n, dtype=torch.uint8, device="cuda")
+    for a in range(0, n, 1 << 28):
+        seen[sa[a: a + (1 << 28)].long()] = 1
+    assert bool(seen.all())
+    del seen
+    at = torch.randint(0, n - 1, (2_000_000,), device="cuda", generator=g)
+    p, q = sa[at].long(), sa[at + 1].long()
+    order = torch.zeros(len(at), dtype=torch.int32, device="cuda")
+    for j in range(64):
+        x, y = (torch.where(v + j < n, t[(v + j).clamp(max=n - 1)].int(), -1) for v in (p, q))
+        order = torch.where(order == 0, torch.sign(y - x), order)
+    assert bool((order > 0).all())
+
+
 @pytest.mark.parametrize("n", [30011, 1 << 18])
 @pytest.mark.parametrize("longer_first", [False, True])
 def test_record_sort_complete_ties_keep_position_order(ctx, n, longer_first):
