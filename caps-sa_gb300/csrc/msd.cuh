@@ -49,20 +49,26 @@ __host__ __device__ __forceinline__ uint32_t chunk_key(uint32_t span, const Digi
     return span | (uint32_t)d.shift << 16 | (uint32_t)d.bits << 24 | (uint32_t)d.from_val << 31;
 }
 // Bin of a chunk's record among at most 2^log2_bins: its digit less the first,
-// and the bits below down to bit `low`.  Bins grow with the key.
+// and the bits below down to bit `low`; or the digit without its lowest bits
+// where more digit values than bins lie between the first and the last (few
+// records over a wide digit, such as many empty texts).  Bins grow with the
+// key.
 struct ChunkBins {
     int sh;
     uint32_t mask, base;
     __device__ __forceinline__ ChunkBins(const uint4 &ch, int log2_bins, int low) {
-        const uint32_t span = ch.w & 0xFFFFu;
+        const uint32_t span = ch.w & 0xFFFFu, last = ch.z + span - 1;
         const int shift = (int)(ch.w >> 16) & 63, bits = (int)(ch.w >> 24) & 15;
         int g = log2_bins - (31 - __clz((int)span));  // span << g <= 2^log2_bins
         if ((span & (span - 1)) != 0) g--;
         if (g > shift - low) g = shift - low;
-        if (g < 0) g = 0;
+        if (g < 0) {
+            g = 0;
+            while ((last >> -g) - (ch.z >> -g) >= 1u << log2_bins) g--;
+        }
         sh = shift - g;
         mask = (1u << (bits + g)) - 1u;
-        base = ch.z << g;
+        base = g < 0 ? ch.z >> -g : ch.z << g;
     }
     __device__ __forceinline__ uint32_t of(uint64_t key) const {
         return ((uint32_t)(key >> sh) & mask) - base;

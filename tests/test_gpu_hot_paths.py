@@ -260,6 +260,25 @@ def test_record_sort_segment_major(ctx, lens):
         assert np.array_equal(got[offs[i]:offs[i + 1]], orc.build_in_memory(tx)), i
 
 
+@pytest.mark.parametrize("sigma", [4, 200, 256])
+def test_record_sort_of_few_symbols_in_millions_of_texts(ctx, sigma):
+    """2,700 symbols in 2^24 texts, nearly all of them empty: few records over
+    leading digits of 12 bits, so that one block's records lie further apart
+    than it has bins (key and position in one word, and as pairs)."""
+    rng = np.random.default_rng(sigma)
+    texts = 1 << 24
+    lens = np.zeros(texts, dtype=np.int64)
+    lens[rng.choice(texts * 15 // 16, 100, replace=False)] = 1
+    lens[texts - 5000 + 3 * np.arange(1300)] = 2
+    offs = np.concatenate([[0], np.cumsum(lens)]).astype(np.uint64)
+    n = int(offs[-1])
+    cat = rng.permutation(np.arange(n) % sigma).astype(np.uint8)
+    got = ctx.build_batched(cat, offs)
+    for i in np.flatnonzero(lens):
+        a, b = int(offs[i]), int(offs[i + 1])
+        assert np.array_equal(got[a:b], orc.build_in_memory(cat[a:b])), i
+
+
 # ---------------------------------------------------------------- horizons of the direct rounds
 
 @pytest.mark.parametrize("lcp", [255, 256, 257, 600, 2303, 2304, 2305, 5000])
