@@ -3804,10 +3804,15 @@ capssa_status core_sort(Ctx &c, const EngineArgs &a, uint32_t **sa_out, eng::Pac
     const bool fused = use_msd && vbits && geo.flag_len == 1;
     const msd::Plan plan =
         msd::plan(n_rec, sort_bits, seg_bits,
-                  pf ? 2 * n / pf->p : (seg_bits ? a.seg_max_len : n_rec), entropy / geo.b);
+                  pf ? 2 * n / pf->p : (seg_bits ? a.seg_max_len : n_rec), entropy / geo.b,
+                  /*in_pieces=*/use_msd && !pf && !sp);
+    // (the records of a batch come text by text: with their pieces given, the
+    // keys' digits need no counting)
+    const msd::Pieces given{a.lim.ends, (uint32_t)a.lim.n_ends};
     const int top_bits = std::max(plan.bits[0], 1);
-    const KeyDigits td = use_msd ? KeyDigits{1, sort_bits - top_bits, top_bits}
-                                 : KeyDigits{lsd_passes, 0, 8};
+    const KeyDigits td = !use_msd    ? KeyDigits{lsd_passes, 0, 8}
+                         : plan.given ? KeyDigits{0, 0, 0}
+                                      : KeyDigits{1, sort_bits - top_bits, top_bits};
     uint32_t *counts = use_msd ? msd::count_buffer(c) : radix::hist_buffer(c);
     if (!counts) return set_err(c, CAPSSA_ENOMEM, "digit counts");
     if (!use_msd)
@@ -3923,7 +3928,7 @@ capssa_status core_sort(Ctx &c, const EngineArgs &a, uint32_t **sa_out, eng::Pac
     if (fused) {
         const FinArgs fa{keys_a, keys_b, geo.k, lf, vbits, seg_at, a.lim.ends, hd, sa};
         s = msd::distribute(c, plan, keys_a, keys_b, (uint32_t)n_rec, vbits, sort_bits, counts,
-                            &passes, [&](const msd::Chunks &ch) {
+                            given, &passes, [&](const msd::Chunks &ch) {
                                 const capssa_status fs = seg_at
                                                              ? finish_chunks<true>(c, fa, ch, G)
                                                              : finish_chunks<false>(c, fa, ch, G);
@@ -3937,7 +3942,7 @@ capssa_status core_sort(Ctx &c, const EngineArgs &a, uint32_t **sa_out, eng::Pac
         s = msd::sort(c, plan, keys_a, vbits ? nullptr : vals_a, keys_b, vbits ? nullptr : vals_b,
                       (uint32_t)n_rec, vbits, sort_bits, bits_for(n - 1),
                       geo.flag_len == 0 || geo.flag_len == 3, !sp,
-                      counts, &passes);
+                      counts, given, &passes);
         c.stats.radix_items = msd::records_per_thread(vbits == 0);
     } else {
         s = vbits ? radix::sort_keys(c, keys_a, keys_b, (uint32_t)n_rec, vbits, vbits + sort_bits,

@@ -135,6 +135,18 @@ __global__ void __launch_bounds__(256)
     }
 }
 
+// The bins of given pieces, as a level that distributed by their index would
+// leave them: piece i's end, and n past the last piece.
+__global__ void __launch_bounds__(256)
+    given_kernel(Pieces given, uint32_t n, uint32_t R, uint32_t *__restrict__ bins) {
+    for (uint32_t d = blockIdx.x * 256 + threadIdx.x; d < R; d += gridDim.x * 256)
+        bins[d] = d + 1 < given.n ? (uint32_t)given.ends[d] : n;
+}
+
+__global__ void __launch_bounds__(256) iota_kernel(uint32_t *__restrict__ out, uint32_t n) {
+    for (uint32_t i = blockIdx.x * 256 + threadIdx.x; i < n; i += gridDim.x * 256) out[i] = i;
+}
+
 // One tile of a range at a time: ranks by digit in shared memory, a place in
 // every bin from one global atomic per digit present, records staged in digit
 // order and written as runs.  bins: each bin's next free position (its end,
@@ -145,7 +157,8 @@ template <bool PAIRS>
 __global__ void __launch_bounds__(kThreads, 2)
     scatter_kernel(const uint64_t *__restrict__ keys, const uint32_t *__restrict__ vals,
                    uint64_t *__restrict__ keys_out, uint32_t *__restrict__ vals_out, uint32_t n,
-                   int gen_vals, Digit dg, const Tile *__restrict__ tiles, const Counters *__restrict__ ctr,
+                   int gen_vals, Digit dg, const Tile *__restrict__ tiles,
+                   const Counters *__restrict__ ctr,
                    uint32_t *__restrict__ bins) {
     constexpr int IT = PAIRS ? kItPairs : kItKeys;
     constexpr uint32_t T = kThreads * IT;
@@ -521,7 +534,7 @@ size_t scatter_smem(int bits) {
 template <bool PAIRS>
 capssa_status run(Ctx &c, const Plan &pl, uint64_t *ka, uint32_t *va, uint64_t *kb, uint32_t *vb,
                   uint32_t n, int low, int nbits, int pos_bits, bool pos_order, bool gen_vals,
-                  uint32_t *counts, int *levels_out,
+                  uint32_t *counts, const Pieces &given, int *levels_out,
                   const std::function<capssa_status(const Chunks &)> &finish,
                   bool *synced = nullptr) {
     constexpr uint32_t T = (uint32_t)kThreads * (PAIRS ? kItPairs : kItKeys);
@@ -533,12 +546,12 @@ capssa_status run(Ctx &c, const Plan &pl, uint64_t *ka, uint32_t *va, uint64_t *
     *levels_out = 0;
     cudaFuncSetAttribute(scatter_kernel<PAIRS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)scatter_smem<PAIRS>(kMaxDigit));
-    // workspace: the chunks of two levels (each level: one per stretch of its
+    // workspace: the chunks of three levels (each level: one per stretch of its
     // ranges, which number at most n / kPiece, and the cut-up long pieces of a
     // last level), two range and tile lists, the counters
     const uint64_t max_ranges = (uint64_t)n / kPiece + 2;
     const uint64_t max_tiles = (uint64_t)n / T + max_ranges + 2;
-    const uint64_t max_chunks = 6 * ((uint64_t)n / kPiece + 4) + 64;
+    const uint64_t max_chunks = 8 * ((uint64_t)n / kPiece + 4) + 64;
     auto up = [](size_t x) { return (x + 255) & ~(size_t)255; };
     const size_t bytes = 2 * up(max_chunks * 16) + 2 * up(max_ranges * sizeof(Range)) +
                          2 * up(max_tiles * sizeof(Tile)) + 4096;
@@ -565,7 +578,8 @@ capssa_status run(Ctx &c, const Plan &pl, uint64_t *ka, uint32_t *va, uint64_t *
     // sorts the listed chunks (or the one given)
     auto local = [&](uint4 single) -> capssa_status {
         if (finish) return finish(Chunks{chunks, n_chunks, single, crowded, n_crowded});
-        local_kernel<PAIRS><<<single.y ? 1u : blocks * kLocalBlocks, kLocalThreads, local_smem, c.stream>>>(
+        const unsigned lg = single.y ? 1u : blocks * kLocalBlocks;
+        local_kernel<PAIRS><<<lg, kLocalThreads, local_smem, c.stream>>>(
             ka, va, kb, vb, single, single.y && gen_vals ? 1 : 0, chunks, n_chunks, crowded,
             n_crowded);
         CAPSSA_LAUNCHED(c);
@@ -585,10 +599,17 @@ capssa_status run(Ctx &c, const Plan &pl, uint64_t *ka, uint32_t *va, uint64_t *
     uint32_t nr_bound = 1;
     Counters *hc = (Counters *)c.h_scratch;
     int cur = 0;
-    for (int level = 0;; level++) {
+    const int first = pl.given ? -1 : 0;  // level -1: the given pieces
+    if (pl.given && gen_vals) {  // (their short ones never pass through a scatter)
+        iota_kernel<<<std::min<unsigned>(grid_for(n, 256), blocks * 16), 256, 0, c.stream>>>(va, n);
+        CAPSSA_LAUNCHED(c);
+        gen_vals = false;
+    }
+    int moved = 0;  // scatters so far: the records lie in the b buffers after an odd number
+    for (int level = first;; level++) {
         // this level's digit
         Digit dg;
-        const int want = level < pl.levels ? pl.bits[level] : kExtraBits;
+        const int want = level < 0 ? pl.given : level < pl.levels ? pl.bits[level] : kExtraBits;
         if (key_left > 0) {
             dg.bits = std::min(want, key_left);
             key_left -= dg.bits;
@@ -600,46 +621,53 @@ capssa_status run(Ctx &c, const Plan &pl, uint64_t *ka, uint32_t *va, uint64_t *
             dg.shift = val_left;
             dg.from_val = PAIRS ? 1 : 0;
         }
-        const uint32_t whole = level == 0 ? n : 0u;  // one range: the whole array
+        const uint32_t whole = level == first ? n : 0u;  // one range: the whole array
         const bool last = key_left == 0 && (!pos_order || val_left == 0);
         const uint64_t n_bins = (uint64_t)nr_bound << dg.bits;
         uint32_t *bins = counts;
-        if (level > 0) {
+        if (level != first) {
             bins = (uint32_t *)ws_get(c, WS_MSD_BINS, n_bins * 4);
             if (!bins) return set_err(c, CAPSSA_ENOMEM, "record sort bins");
-            CAPSSA_CUDA(c, cudaMemsetAsync(bins, 0, n_bins * 4, c.stream));
         }
-        const bool in_b = level & 1;  // this level reads the b buffers
-        const uint64_t *ki = in_b ? kb : ka;
-        const uint32_t *vi = in_b ? vb : va;
-        uint64_t *ko = in_b ? ka : kb;
-        uint32_t *vo = in_b ? va : vb;
-        const unsigned tile_grid =
-            (unsigned)std::min<uint64_t>((uint64_t)n / T + nr_bound + 1, (uint64_t)blocks * 4);
-        if (level > 0) {
-            hist_kernel<PAIRS><<<tile_grid, kThreads, (size_t)4 << dg.bits, c.stream>>>(
-                ki, vi, dg, tiles[cur], ctr[cur], bins);
+        if (level < 0) {
+            given_kernel<<<grid_for(n_bins, 256), 256, 0, c.stream>>>(given, n, (uint32_t)n_bins,
+                                                                      bins);
             CAPSSA_LAUNCHED(c);
+        } else {
+            const bool in_b = moved & 1;  // this level reads the b buffers
+            const uint64_t *ki = in_b ? kb : ka;
+            const uint32_t *vi = in_b ? vb : va;
+            uint64_t *ko = in_b ? ka : kb;
+            uint32_t *vo = in_b ? va : vb;
+            const unsigned tile_grid =
+                (unsigned)std::min<uint64_t>((uint64_t)n / T + nr_bound + 1, (uint64_t)blocks * 4);
+            if (!whole) {
+                CAPSSA_CUDA(c, cudaMemsetAsync(bins, 0, n_bins * 4, c.stream));
+                hist_kernel<PAIRS><<<tile_grid, kThreads, (size_t)4 << dg.bits, c.stream>>>(
+                    ki, vi, dg, tiles[cur], ctr[cur], bins);
+                CAPSSA_LAUNCHED(c);
+            }
+            offsets_kernel<<<std::min<unsigned>(nr_bound, blocks * 8), 256, 0, c.stream>>>(
+                ranges[cur], ctr[cur], dg.bits, whole, bins);
+            CAPSSA_LAUNCHED(c);
+            const size_t sm = scatter_smem<PAIRS>(dg.bits);
+            if (level < 16) cudaEventRecord(c.kev[2 * level], c.stream);
+            scatter_kernel<PAIRS>
+                <<<std::min<unsigned>(tile_grid, blocks * 2), kThreads, sm, c.stream>>>(
+                    ki, vi, ko, vo, n, gen_vals && whole ? 1 : 0, dg,
+                    whole ? nullptr : tiles[cur], ctr[cur], bins);
+            CAPSSA_LAUNCHED(c);
+            if (level < 16) cudaEventRecord(c.kev[2 * level + 1], c.stream);
+            moved++;
+            if (level < pl.levels) (*levels_out)++;
         }
-        offsets_kernel<<<std::min<unsigned>(nr_bound, blocks * 8), 256, 0, c.stream>>>(
-            ranges[cur], ctr[cur], dg.bits, whole, bins);
-        CAPSSA_LAUNCHED(c);
-        const size_t sm = scatter_smem<PAIRS>(dg.bits);
-        if (level < 16) cudaEventRecord(c.kev[2 * level], c.stream);
-        scatter_kernel<PAIRS><<<std::min<unsigned>(tile_grid, blocks * 2), kThreads, sm, c.stream>>>(
-            ki, vi, ko, vo, n, gen_vals && level == 0 ? 1 : 0, dg, level > 0 ? tiles[cur] : nullptr,
-            ctr[cur], bins);
-        CAPSSA_LAUNCHED(c);
-        if (level < 16) cudaEventRecord(c.kev[2 * level + 1], c.stream);
         const int nxt = cur ^ 1;
         CAPSSA_CUDA(c, cudaMemsetAsync(ctr[nxt], 0, sizeof(Counters), c.stream));
         pieces_kernel<<<(unsigned)std::min<uint64_t>((n_bins + 255) / 256, (uint64_t)blocks * 16),
                         256, 0, c.stream>>>(ranges[cur], ctr[cur], whole, dg, bins, T, last ? 1 : 0,
-                                            finish ? 1 : 0,
-                                            in_b ? 0u : kInB, ranges[nxt], tiles[nxt], ctr[nxt],
-                                            chunks, n_chunks);
+                                            finish ? 1 : 0, (moved & 1) ? kInB : 0u, ranges[nxt],
+                                            tiles[nxt], ctr[nxt], chunks, n_chunks);
         CAPSSA_LAUNCHED(c);
-        if (level < pl.levels) (*levels_out)++;
         nr_bound = (uint32_t)std::min<uint64_t>(n_bins, max_ranges);
         cur = nxt;
         if (level + 1 < pl.levels && !last) continue;
@@ -663,8 +691,8 @@ capssa_status run(Ctx &c, const Plan &pl, uint64_t *ka, uint32_t *va, uint64_t *
 
 }  // namespace
 
-Plan plan(uint64_t n, int nbits, int top_bits, uint64_t longest, double eff) {
-    Plan p{0, {0, 0}};
+Plan plan(uint64_t n, int nbits, int top_bits, uint64_t longest, double eff, bool in_pieces) {
+    Plan p{0, {0, 0}, 0};
     if (n <= kChunk) return p;
     // pieces of at most 0.8 kPiece records on average, which spread keys stay
     // below kPiece with
@@ -676,8 +704,14 @@ Plan plan(uint64_t n, int nbits, int top_bits, uint64_t longest, double eff) {
         need = std::log2((double)n / half);
     }
     const double e = std::min(1.0, std::max(eff, 0.25));
+    if (in_pieces && top_bits > 0 && top_bits <= kMaxGiven) {
+        p.given = top_bits;
+        nbits -= top_bits;
+        top_bits = 0;
+    }
     int bits = top_bits + (int)std::ceil(need / e);
     bits = std::max(1, std::min(bits, nbits));
+    if (p.given && need == 0) return p;  // every piece fits a block
     // one level keeps runs of 8 records a digit up to 2^10 of them in use
     if (bits <= kMaxDigit && top_bits + need <= 10.0) {
         p.levels = 1;
@@ -692,31 +726,32 @@ Plan plan(uint64_t n, int nbits, int top_bits, uint64_t longest, double eff) {
 }
 
 uint32_t *count_buffer(Ctx &c) {
-    const size_t bytes = ((size_t)1 << kMaxDigit) * 4;
-    uint32_t *b = (uint32_t *)ws_get(c, WS_MSD_COUNTS, bytes);
-    if (b && cudaMemsetAsync(b, 0, bytes, c.stream) != cudaSuccess) return nullptr;
+    static_assert(kMaxGiven >= kMaxDigit, "room for either");
+    uint32_t *b = (uint32_t *)ws_get(c, WS_MSD_COUNTS, ((size_t)1 << kMaxGiven) * 4);
+    if (b && cudaMemsetAsync(b, 0, ((size_t)1 << kMaxDigit) * 4, c.stream) != cudaSuccess)
+        return nullptr;
     return b;
 }
 
 capssa_status sort(Ctx &c, const Plan &pl, uint64_t *ka, uint32_t *va, uint64_t *kb, uint32_t *vb,
                    uint32_t n, int low, int nbits, int pos_bits, bool pos_order, bool gen_vals,
-                   uint32_t *counts, int *levels_out) {
+                   uint32_t *counts, const Pieces &given, int *levels_out) {
     if (n == 0) {
         *levels_out = 0;
         return CAPSSA_OK;
     }
     return va ? run<true>(c, pl, ka, va, kb, vb, n, low, nbits, pos_bits, pos_order, gen_vals,
-                          counts, levels_out, nullptr)
+                          counts, given, levels_out, nullptr)
               : run<false>(c, pl, ka, nullptr, kb, nullptr, n, low, nbits, pos_bits, pos_order,
-                           false, counts, levels_out, nullptr);
+                           false, counts, given, levels_out, nullptr);
 }
 
 capssa_status distribute(Ctx &c, const Plan &pl, uint64_t *ka, uint64_t *kb, uint32_t n, int low,
-                         int nbits, uint32_t *counts, int *levels_out,
+                         int nbits, uint32_t *counts, const Pieces &given, int *levels_out,
                          const std::function<capssa_status(const Chunks &)> &finish,
                          bool *synced) {
     return run<false>(c, pl, ka, nullptr, kb, nullptr, n, low, nbits, 0, false, false, counts,
-                      levels_out, finish, synced);
+                      given, levels_out, finish, synced);
 }
 
 }  // namespace msd

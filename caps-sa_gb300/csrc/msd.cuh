@@ -12,17 +12,29 @@ namespace msd {
 // one block's shared memory; level 0's digit counts are the caller's job (the
 // kernel that makes the records sees each of them anyway).
 struct Plan {
-    int levels;     // planned distribution levels: 0 (one block's worth), 1 or 2
+    int levels;     // planned distribution levels: 0, 1 or 2
     int bits[2];    // bits of each level's digit, from the top of the key
+    int given;      // leading key bits the records already lie in order of (see plan)
 };
 
 constexpr uint32_t kOneBlock = 2560;  // records one block sorts on its own
 constexpr int kMaxDigit = 12;  // bits of a planned digit
+constexpr int kMaxGiven = 14;  // ... of a given one (a chunk holds 15 bits of digit)
 
 // n records with nbits key bits, of which the leading top_bits number equally
 // sized or `longest`-bounded pieces (a segment or bucket index; longest = n
-// without one); eff: bits of entropy per key bit.
-Plan plan(uint64_t n, int nbits, int top_bits, uint64_t longest, double eff);
+// without one); eff: bits of entropy per key bit.  in_pieces: the records are
+// laid out piece by piece, in the order of those bits.  Up to kMaxGiven such
+// bits are then given: no level distributes by them, the pieces' ends are read
+// instead (2,048 genomes of 47,000 symbols: 2.83 ms for 3.40 with two levels
+// over both, whose first moved every tile's records to the same few digits).
+Plan plan(uint64_t n, int nbits, int top_bits, uint64_t longest, double eff, bool in_pieces);
+// The pieces of a plan with given bits: piece i ends at record ends[i]
+// (device), and the last at n.
+struct Pieces {
+    const uint64_t *ends;
+    uint32_t n;
+};
 
 // A chunk of the distributed records, at most kOneBlock of them, holding whole
 // runs of equal keys: (start, length | kInB, first digit value, key), the key
@@ -51,8 +63,8 @@ __host__ __device__ __forceinline__ uint32_t chunk_key(uint32_t span, const Digi
 // Bin of a chunk's record among at most 2^log2_bins: its digit less the first,
 // and the bits below down to bit `low`; or the digit without its lowest bits
 // where more digit values than bins lie between the first and the last (few
-// records over a wide digit, such as many empty texts).  Bins grow with the
-// key.
+// records over a wide digit: a thin range of a sort with two 12-bit levels).
+// Bins grow with the key.
 struct ChunkBins {
     int sh;
     uint32_t mask, base;
@@ -82,7 +94,7 @@ struct ChunkBins {
 // host has waited for the last batch.  Equal keys stay
 // together; a run of more than a chunk comes as kRunPiece / kRunWhole entries.
 capssa_status distribute(Ctx &c, const Plan &pl, uint64_t *ka, uint64_t *kb, uint32_t n, int low,
-                         int nbits, uint32_t *counts, int *levels_out,
+                         int nbits, uint32_t *counts, const Pieces &given, int *levels_out,
                          const std::function<capssa_status(const Chunks &)> &finish,
                          bool *synced);
 
@@ -92,15 +104,17 @@ capssa_status distribute(Ctx &c, const Plan &pl, uint64_t *ka, uint64_t *kb, uin
 // Records in (ka, va), scratch (kb, vb); sorted into (ka, va).  counts: the
 // 2^bits[0] digit counts of level 0 (device; overwritten).  pos_order false:
 // the order of equal keys is left open (it is then whatever is cheapest).
-// gen_vals: the input values are not read, value i is i.  levels_out: levels over the whole array (the planned ones).
+// gen_vals: the input values are not read, value i is i.  levels_out: planned
+// levels run.
 capssa_status sort(Ctx &c, const Plan &pl, uint64_t *ka, uint32_t *va, uint64_t *kb, uint32_t *vb,
                    uint32_t n, int low, int nbits, int pos_bits, bool pos_order,
-                   bool gen_vals, uint32_t *counts, int *levels_out);
+                   bool gen_vals, uint32_t *counts, const Pieces &given, int *levels_out);
 
 // Records a thread handles in a distribution tile (stats.radix_items).
 constexpr uint32_t records_per_thread(bool pairs) { return pairs ? 12u : 16u; }
 
-// Device buffer for level 0's digit counts (2^kMaxDigit words), zeroed.
+// Device buffer for level 0's digit counts (2^kMaxDigit words, zeroed), or the
+// ends of given pieces.
 uint32_t *count_buffer(Ctx &c);
 
 }  // namespace msd

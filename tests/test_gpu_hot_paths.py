@@ -260,23 +260,50 @@ def test_record_sort_segment_major(ctx, lens):
         assert np.array_equal(got[offs[i]:offs[i + 1]], orc.build_in_memory(tx)), i
 
 
-@pytest.mark.parametrize("sigma", [4, 200, 256])
-def test_record_sort_of_few_symbols_in_millions_of_texts(ctx, sigma):
-    """2,700 symbols in 2^24 texts, nearly all of them empty: few records over
-    leading digits of 12 bits, so that one block's records lie further apart
-    than it has bins (key and position in one word, and as pairs)."""
+@pytest.mark.parametrize("texts", [1 << 14, (1 << 14) + 1, (1 << 23) + 77])
+@pytest.mark.parametrize("sigma", [4, 200])
+def test_record_sort_of_many_tiny_texts(ctx, texts, sigma):
+    """Texts of one symbol with some of two to five: the most pieces the sort
+    takes as given, one more, and a text index of two 12-bit levels whose
+    every digit holds a record or two (key and position in one word, and as
+    pairs)."""
     rng = np.random.default_rng(sigma)
-    texts = 1 << 24
-    lens = np.zeros(texts, dtype=np.int64)
-    lens[rng.choice(texts * 15 // 16, 100, replace=False)] = 1
-    lens[texts - 5000 + 3 * np.arange(1300)] = 2
+    lens = np.ones(texts, dtype=np.int64)
+    longer = rng.choice(texts, 500, replace=False)
+    lens[longer] = rng.integers(2, 6, 500)
     offs = np.concatenate([[0], np.cumsum(lens)]).astype(np.uint64)
-    n = int(offs[-1])
-    cat = rng.permutation(np.arange(n) % sigma).astype(np.uint8)
+    cat = (np.arange(int(offs[-1])) * 7 % sigma).astype(np.uint8)
     got = ctx.build_batched(cat, offs)
-    for i in np.flatnonzero(lens):
+    assert not got[offs[:-1][lens == 1].astype(np.int64)].any()
+    for i in longer:
         a, b = int(offs[i]), int(offs[i + 1])
         assert np.array_equal(got[a:b], orc.build_in_memory(cat[a:b])), i
+
+
+@pytest.mark.parametrize("sigma,dtype", [(4, np.uint8), (200, np.uint8), (60000, np.uint32)])
+@pytest.mark.parametrize("lens", [[1279, 1280, 1281, 1282], [2559, 2560, 2561, 1, 1, 2562],
+                                  [1] * 3000 + [200000], [300000, 5, 5, 5, 2_000_000],
+                                  [20000] * 40, [1025] * 700])
+def test_record_sort_of_given_pieces(ctx, sigma, dtype, lens):
+    """Batches whose texts are the sort's pieces: at the edges of a joined and
+    of a single block's piece, so uneven that the short ones never move while
+    the long ones take two levels, and all alike; with runs and equal texts
+    (complete ties only within a text)."""
+    rng = np.random.default_rng(len(lens) + sigma)
+    texts = [rng.integers(0, sigma, L).astype(dtype) for L in lens]
+    big = int(np.argmax(lens))
+    texts[big][10: 10 + lens[big] // 20] = 3
+    for i in range(1, len(lens)):
+        if lens[i] == lens[0] and i % 3 == 0:
+            texts[i] = texts[0]
+    cat = np.concatenate(texts)
+    offs = np.concatenate([[0], np.cumsum(lens)]).astype(np.uint64)
+    got = ctx.build_batched(cat, offs)
+    for i, tx in enumerate(texts):
+        if len(tx) == 1:
+            assert got[offs[i]] == 0
+        else:
+            assert np.array_equal(got[offs[i]:offs[i + 1]], orc.build_in_memory(tx)), i
 
 
 # ---------------------------------------------------------------- horizons of the direct rounds
