@@ -327,8 +327,12 @@ static_assert(kDigitWords >= radix::kMaxPasses * 256, "the LSD digits fit too");
 // suffix is read straight from the packed text (two 64-bit loads, shared by
 // the neighbouring threads' positions); only suffixes that end inside the
 // window (lim < k) are masked and padded.  Each thread owns kKeyPer
-// consecutive positions of a tile (the segment end is tracked across
-// them); blocks stride over the tiles and add their histograms to the
+// consecutive positions of a tile.  Where the segment reaches past all their
+// windows, nearly everywhere, and the codes have at most 8 bits, the windows
+// slide through 128 bits read once; elsewhere the segment end is tracked
+// across the positions, and their words are read one by one, which cost 110
+// instructions a record when all did it (96 M records of a batch: 0.46 ms,
+// 0.27 now).  Blocks stride over the tiles and add their histograms to the
 // global counts once.  With vbits > 0 the position is packed below the key
 // (one 64-bit word per suffix).  kPlain: a PlainText text with no segment
 // index (limits are n - p, nothing to track).
@@ -346,13 +350,43 @@ __global__ void __launch_bounds__(kKeyThreads)
          t0 += (uint64_t)gridDim.x * kKeyTile) {
         const uint64_t p0 = t0 + (uint64_t)threadIdx.x * kKeyPer;
         if (p0 >= n_rec) continue;
-        // one past the last symbol of p0's suffix
-        uint64_t end = kPlain ? n : p0 + dev_lim_at(L, p0);
-        // segment-major keys carry the segment index above the key bits
-        uint64_t seg = !kPlain && seg_shift ? dev_seg_at(L, p0) : 0;
-        // first position of p0's segment (segment-local packed positions)
-        uint64_t start = !kPlain && local_pos && seg ? __ldg(L.ends + seg - 1) : 0;
+        // one past the last symbol of p0's suffix, and its segment: the index
+        // goes above segment-major keys, packed positions may count from the
+        // segment's first
+        uint64_t end = n, seg = 0, start = 0;
+        if (!kPlain) {
+            const uint64_t i = dev_seg_at(L, p0);
+            if (i < L.n_ends) end = __ldg(L.ends + i);
+            if (seg_shift) seg = i;
+            if (local_pos && i) start = __ldg(L.ends + i - 1);
+        }
         uint64_t out[kKeyPer];
+        if (b <= 8 && p0 + kKeyPer <= n_rec && end - p0 >= (uint64_t)(k + kKeyPer - 1)) {
+            static_assert(63 + 8 * (kKeyPer - 1) <= 128, "a thread's windows in 128 bits");
+            const uint64_t bit = p0 * (uint64_t)b;
+            const uint64_t *w = P.w + (bit >> 6);
+            const uint32_t sh = (uint32_t)(bit & 63);
+            const uint64_t w0 = __ldg(w), w1 = __ldg(w + 1), w2 = __ldg(w + 2);
+            uint64_t hi = (w0 << sh) | ((w1 >> 1) >> (63 - sh));
+            uint64_t lo = (w1 << sh) | ((w2 >> 1) >> (63 - sh));
+            const uint64_t top = (!kPlain && seg_shift ? seg << seg_shift : 0) |
+                                 (!lbits ? 0 : flag_len ? (uint64_t)(lf == 0) : (lf ? 0u : k));
+            uint64_t val = p0 - start;
+#pragma unroll
+            for (int e = 0; e < kKeyPer; e++) {
+                const uint64_t key = (hi >> (64 - kbits)) << lbits | top;
+                td.count(hist, key);
+                out[e] = vbits ? (key << vbits) | val++ : key;
+                hi = (hi << b) | (lo >> (64 - b));
+                lo <<= b;
+            }
+            uint4 *dst = reinterpret_cast<uint4 *>(keys + p0);
+#pragma unroll
+            for (int e = 0; e < kKeyPer; e += 2)
+                dst[e / 2] = make_uint4((uint32_t)out[e], (uint32_t)(out[e] >> 32),
+                                        (uint32_t)out[e + 1], (uint32_t)(out[e + 1] >> 32));
+            continue;
+        }
 #pragma unroll
         for (int e = 0; e < kKeyPer; e++) {
             const uint64_t p = p0 + e;
