@@ -1532,12 +1532,17 @@ __global__ void gather_small_kernel(const uint4 *__restrict__ groups, uint32_t c
 // keys then agree on rr + h symbols (ranks are exact to the round depth h),
 // the depth their subgroup is queued with; a group deeper than h is sorted
 // by the rank at its own depth d, and its subgroups agree on d + h.
-// runs_s: the inclusive max-scan of "last index of a run" over the reversed
-// text, from which the run from p ends at n - 1 - runs_s[n - 1 - p].
+// ends: one bit a text position, set where a run of one symbol ends, with a
+// summary bit for every nonzero word of the level below up to a single word:
+// the end of the run from p is the next set bit, a few words up and down the
+// levels.  Only the big groups' members look (2 of every 100 suffixes of a
+// masked genome), so a word for every position, which stood here as a max-scan
+// over the reversed text, cost more than all their keys: 0.88 ms for 134 M
+// positions, 0.21 ms for the bits.
+constexpr int kRunLevels = 6;  // 64^6 > 2^32
 struct RunKeys {
-    const uint32_t *runs_s;  // null: no run keys this round
+    const uint64_t *ends[kRunLevels];  // ends[0] null: no run keys this round
     Packed P;
-    uint64_t n;
     int rbits;               // bits of the run-length field (cap 2^rbits - 1)
 };
 
@@ -1550,8 +1555,24 @@ __device__ __forceinline__ uint32_t code_at(const Packed &P, uint64_t q) {
     return (uint32_t)(v >> (64 - P.b));
 }
 
+// Symbols of the run from p.  The text's last position is an end, so every
+// level has a set bit at or past the index looked from.
 __device__ __forceinline__ uint64_t run_from(const RunKeys &R, uint64_t p) {
-    return R.n - 1 - (uint64_t)__ldg(R.runs_s + (R.n - 1 - p)) - p + 1;
+    uint64_t at = p, w = 0;
+    int l = 0;
+#pragma unroll
+    for (int q = 0; q < kRunLevels; q++) {
+        if (w == 0) {
+            if (q) at = (at >> 6) + 1;
+            l = q;
+            w = __ldg(R.ends[q] + (at >> 6)) >> (at & 63);
+        }
+    }
+    at += (uint64_t)(__ffsll((long long)w) - 1);
+#pragma unroll
+    for (int q = kRunLevels - 2; q >= 0; q--)
+        if (q < l) at = (at << 6) + (uint64_t)(__ffsll((long long)__ldg(R.ends[q] + at)) - 1);
+    return at - p + 1;
 }
 
 __global__ void gather_big_kernel(const BigGroup *__restrict__ groups, uint32_t nb,
@@ -1576,7 +1597,7 @@ __global__ void gather_big_kernel(const BigGroup *__restrict__ groups, uint32_t 
         uint64_t key;
         // a run group (see RunKeys); its members agree on d symbols only when
         // the group's own depth reaches the round's
-        if (R.runs_s && g.depth >= h && run_from(R, sa[g.start]) >= d) {
+        if (R.ends[0] && g.depth >= h && run_from(R, sa[g.start]) >= d) {
             const uint64_t cap = (1ull << R.rbits) - 1;
             const uint64_t lim = dev_lim_at(L, p);
             const uint64_t rl = run_from(R, p);
@@ -1601,22 +1622,47 @@ __global__ void gather_big_kernel(const BigGroup *__restrict__ groups, uint32_t 
             key = ((((((uint64_t)lo << 1) | cls) << R.rbits) | rq) << k2bits) | k2;
         } else {
             const uint64_t k2 = doubling_key(L, rank, p, d, lf, empty_lf);
-            key = ((uint64_t)lo << (R.runs_s ? k2bits + 1 + R.rbits : k2bits)) | k2;
+            key = ((uint64_t)lo << (R.ends[0] ? k2bits + 1 + R.rbits : k2bits)) | k2;
         }
         tkeys[t] = key;
         tvals[t] = p;
     }
 }
 
-// runs_s input: rev[r] = r where text position n - 1 - r ends a run of one
-// symbol (the next symbol differs, or the text ends), else 0.
-__global__ void run_ends_kernel(const void *__restrict__ text, int sym_bytes, uint64_t n,
-                                uint32_t *__restrict__ rev) {
-    for (uint64_t r = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; r < n;
-         r += (uint64_t)gridDim.x * blockDim.x) {
-        const uint64_t q = n - 1 - r;
-        const bool end = q == n - 1 || sym_at(text, sym_bytes, q) != sym_at(text, sym_bytes, q + 1);
-        rev[r] = end ? (uint32_t)r : 0u;
+// The bits of RunKeys::ends[0]: a warp takes 1,024 positions, 32 of them a
+// step, and writes their 32 half words at once.
+__global__ void __launch_bounds__(256)
+    run_ends_kernel(const void *__restrict__ text, int sym_bytes, uint64_t n,
+                    uint32_t *__restrict__ bits) {
+    const uint32_t lane = threadIdx.x & 31;
+    const uint64_t warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+    const uint64_t tiles = (n + 1023) / 1024;
+    for (uint64_t t = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < tiles;
+         t += warps) {
+        uint32_t mine = 0;
+#pragma unroll 8
+        for (uint32_t j = 0; j < 32; j++) {
+            const uint64_t q = t * 1024 + j * 32 + lane;
+            const bool end =
+                q < n && (q + 1 == n || sym_at(text, sym_bytes, q) != sym_at(text, sym_bytes, q + 1));
+            const uint32_t w = __ballot_sync(0xffffffffu, end);
+            if (lane == j) mine = w;
+        }
+        bits[t * 32 + lane] = mine;
+    }
+}
+
+// Summary bits of `words` words: half a word a warp.  The rest of the last
+// word is cleared.
+__global__ void __launch_bounds__(256)
+    run_level_kernel(const uint64_t *__restrict__ in, uint64_t words, uint32_t *__restrict__ out) {
+    const uint64_t halves = 2 * ((words + 63) / 64);
+    const uint64_t warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+    for (uint64_t t = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < halves;
+         t += warps) {
+        const uint64_t i = t * 32 + (threadIdx.x & 31);
+        const uint32_t w = __ballot_sync(0xffffffffu, i < words && in[i] != 0);
+        if ((threadIdx.x & 31) == 0) out[t] = w;
     }
 }
 
@@ -2722,7 +2768,7 @@ __global__ void split_big_kernel(const uint64_t *__restrict__ tkeys,
             // the depth the subgroup's members now agree on (see RunKeys)
             const uint64_t d = g.depth > h ? (uint64_t)g.depth : h;
             uint64_t next_depth = d + h;
-            if (R.runs_s && g.depth >= h && run_from(R, tvals[g.toff]) >= d) {
+            if (R.ends[0] && g.depth >= h && run_from(R, tvals[g.toff]) >= d) {
                 const uint64_t cap = (1ull << R.rbits) - 1;
                 const uint64_t rq = (key >> k2bits) & cap;
                 const bool cls_b = (key >> (k2bits + R.rbits)) & 1ull;
@@ -4043,7 +4089,7 @@ capssa_status core_sort(Ctx &c, const EngineArgs &a, uint32_t **sa_out, eng::Pac
     const uint64_t empty = lf ? empty_lf : 0ull;
     bool ranks_ready = false;
     uint64_t last_groups = 0;    // small groups of the round before
-    uint32_t *runs_s = nullptr;  // run ends, for the run keys of deep rounds
+    uint64_t *run_bits = nullptr;  // run ends, for the run keys of deep rounds
     int cur = 0;
     Counters *hc = group_counts;
     for (;;) {
@@ -4168,22 +4214,33 @@ capssa_status core_sort(Ctx &c, const EngineArgs &a, uint32_t **sa_out, eng::Pac
             // bits fits beside the ordinal and the rank (a masked genome of 40 M
             // symbols, runs up to 50,000, LongerFirst: 12 rounds of doubling and
             // 3.5 ms of refinement without them, 2.2 ms with them)
-            RunKeys R{nullptr, P, n, 0};
+            RunKeys R{{}, P, 0};
             const int rbits = std::min(24, 64 - ord_bits - 1 - k2bits);
             if (!sp && rbits >= 12 && h >= 2 * (uint64_t)geo.k) {
-                if (!runs_s) {  // built once, the first deep round that can use it
-                    runs_s = (uint32_t *)ws_get(c, WS_RUNS, (size_t)n * 4 + 64);
-                    if (!runs_s) return set_err(c, CAPSSA_ENOMEM, "run lengths");
-                    run_ends_kernel<<<grid_for(n, 256), 256, 0, c.stream>>>(a.text, a.sym_bytes,
-                                                                            n, runs_s);
-                    CAPSSA_LAUNCHED(c);
-                    s = scan_u32(c, runs_s, runs_s, n, /*max_op=*/true, /*inclusive=*/true);
-                    if (s != CAPSSA_OK) return s;
+                // levels of 64 bits a word (the lowest in whole tiles)
+                uint64_t words[kRunLevels], at[kRunLevels], sum = 0;
+                for (int l = 0; l < kRunLevels; l++) {
+                    words[l] = l ? (words[l - 1] + 63) / 64 : (n + 1023) / 1024 * 16;
+                    at[l] = sum;
+                    sum += words[l];
                 }
-                R.runs_s = runs_s;
+                const bool build = !run_bits;  // the first deep round that can use it
+                if (build) run_bits = (uint64_t *)ws_get(c, WS_RUNS, sum * 8);
+                if (!run_bits) return set_err(c, CAPSSA_ENOMEM, "run ends");
+                for (int l = 0; l < kRunLevels; l++) R.ends[l] = run_bits + at[l];
                 R.rbits = rbits;
+                if (build) {
+                    run_ends_kernel<<<grid_for(words[0] * 2, 256), 256, 0, c.stream>>>(
+                        a.text, a.sym_bytes, n, (uint32_t *)run_bits);
+                    CAPSSA_LAUNCHED(c);
+                    for (int l = 1; l < kRunLevels; l++) {
+                        run_level_kernel<<<grid_for(words[l - 1], 256), 256, 0, c.stream>>>(
+                            run_bits + at[l - 1], words[l - 1], (uint32_t *)(run_bits + at[l]));
+                        CAPSSA_LAUNCHED(c);
+                    }
+                }
             }
-            const int ord_shift = R.runs_s ? k2bits + 1 + rbits : k2bits;
+            const int ord_shift = R.ends[0] ? k2bits + 1 + rbits : k2bits;
             gather_big_kernel<<<grid_for(big_total, 256), 256, 0, c.stream>>>(
                 G.big[cur], nb, big_total, sa, rank, a.lim, h, lf,
                                                         empty_lf, k2bits, R, keys_a, spare_vals);

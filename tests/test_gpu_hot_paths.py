@@ -454,6 +454,30 @@ def test_run_groups_longer_first(ctx, n, longest):
                           orc.build_in_memory(t, None, orc.Limits(n, ends, True)))
 
 
+@pytest.mark.parametrize("dtype", [np.uint8, np.uint32])
+@pytest.mark.parametrize("tail", [1, 64, 4097])
+def test_run_ends_found_across_words_and_levels(ctx, dtype, tail):
+    """Runs of one symbol that end at, before and after the edges of 64, 4,096
+    and 262,144 positions (a word of run ends and of its summaries), up to the
+    text's own end; both boundary orders."""
+    rng = np.random.default_rng(tail)
+    parts = []
+    for L in [62, 63, 64, 65, 127, 128, 4095, 4096, 4097, 8193, 262143, 262145, 600001]:
+        parts += [np.full(L, 2), rng.integers(0, 4, rng.integers(1, 200))]
+    for q in range(300):  # many runs of the same lengths
+        parts += [np.full(40 + q % 7, 2), rng.integers(0, 4, 3)]
+    parts += [rng.integers(0, 2, 500), np.full(tail, 2)]
+    t = np.concatenate(parts).astype(dtype)
+    n = len(t)
+    assert np.array_equal(ctx.build_in_memory(t), orc.build_in_memory(t))
+    ends = np.unique(np.concatenate([rng.integers(1, n, 40), [n]]))
+    for lf in (True, False):
+        lp = capssa.SegmentedText(n, ends, capssa.BoundaryRank.LONGER_FIRST if lf
+                                  else capssa.BoundaryRank.SHORTER_FIRST)
+        got = ctx.build_in_memory(t, lp, capssa.Opts(tie_order=capssa.TieOrder.REFERENCE))
+        assert np.array_equal(got, orc.build_in_memory(t, None, orc.Limits(n, ends, lf)))
+
+
 # ---------------------------------------------------------------- keys whose padding shows the end
 
 @pytest.mark.parametrize("sigma,dtype", [(5, np.uint8), (6, np.uint8), (7, np.uint8), (9, np.uint8),
