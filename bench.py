@@ -168,10 +168,10 @@ def hbm_peak():
 
 
 def profiled_traffic(n, item_bytes):
-    """DRAM bytes per radix-pass launch from the committed ncu summary for
+    """DRAM bytes per distribution level from the committed ncu summary for
     this record width (captured at 2^26 records, input 4x L2), scaled by
     records per launch (traffic grows linearly with the records)."""
-    p = os.path.join(ROOT, "profiles", "radix_onesweep_pass_%dB.txt" % item_bytes)
+    p = os.path.join(ROOT, "profiles", "record_scatter_%dB.txt" % item_bytes)
     try:
         vals = {}
         for ln in open(p):
@@ -472,7 +472,7 @@ def run_ours(args):
         st = ctx.stats()
         launches += st["kernel_launches"]
         pass_ms.append(st["sort_pass_ms"])
-        passes.append(st["sort_passes"])
+        passes.append(st["sort_passes"] - 1)  # without the sort inside the blocks
         item_bytes = st["sort_item_bytes"] or 12
         rounds = st["refine_rounds"]
         for k in phase:
@@ -487,7 +487,7 @@ def run_ours(args):
     ms_per_step = elapsed_ms / args.steps
     value = job_throughput(n, ws, args.steps, elapsed_ms / 1e3)
 
-    # roofline of the dominant kernel: one onesweep radix pass over the n
+    # roofline of the record sort's distribution kernel: one level over the n
     # suffix records reads and writes each record once (8 B when the
     # position is packed below the key, else a u64 key + a u32 position)
     peak, peak_kind = hbm_peak()
@@ -495,7 +495,7 @@ def run_ours(args):
     alg_bytes = 2.0 * item_bytes * n
     achieved = alg_bytes / (avg_pass_ms / 1e3) / 1e9
     traffic = profiled_traffic(n, item_bytes)
-    roofline = {"kernel": "radix onesweep pass (initial sort of the %d-byte suffix records)"
+    roofline = {"kernel": "scatter_kernel (one distribution level of the %d-byte suffix records)"
                 % item_bytes, "bound": "hbm",
                 "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                 "peak_kind": peak_kind, "traffic": traffic,

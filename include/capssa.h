@@ -150,21 +150,25 @@ typedef struct capssa_stats {
     /* device time per phase of the last suffix sort (CUDA events on the
      * context's stream) */
     double keys_ms;       /* alphabet scan + packed-key build */
-    double sort_ms;       /* initial radix sort, all passes */
+    double sort_ms;       /* initial record sort: every pass, and the groups where its
+                             last step finds them */
     double refine_ms;     /* rank-doubling rounds */
     double finish_ms;     /* bounded-context pass, output ordering and copy */
-    uint32_t sort_passes; /* radix passes executed by the initial sort */
-    uint32_t sort_item_bytes; /* bytes per record the radix passes move: 8 (position packed
+    uint32_t sort_passes; /* passes of the initial sort over the records: radix passes, or
+                             distribution levels and the sort inside the blocks */
+    uint32_t sort_item_bytes; /* bytes per record these passes move: 8 (position packed
                                  below the key) or 12 (key + separate u32 position) */
-    double sort_pass_ms;  /* summed duration of those radix-pass kernels */
+    double sort_pass_ms;  /* summed duration of the radix-pass kernels, or of the levels'
+                             scatter kernels */
     /* sample-sort partition (capssa_build_in_memory_sample_sort_*) */
     double partition_ms;        /* bucket of every suffix (search or prediction + fixup) */
     double train_ms;            /* learned partition: model training */
     uint64_t partition_probes;  /* suffix-vs-splitter comparisons of the partition */
     uint32_t train_samples;     /* learned partition: samples the model trained on */
     float model_loss;           /* learned partition: final mean squared CDF error */
-    uint32_t radix_items;       /* records per thread of the radix passes (for keys alone the context's
-                                   autotuner picks it on its first large sort) */
+    uint32_t radix_items;       /* records per thread of those passes (radix passes over
+                                   packed records: the context's autotuner picks it on its
+                                   first large sort) */
     uint32_t sparse_subset;     /* 1: a subset build sorted only its own positions */
     uint32_t tie_classes;       /* tie classes of the output (CAPSSA_TIES_REFERENCE) */
     uint32_t reserved_u32;
