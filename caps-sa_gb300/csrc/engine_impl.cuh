@@ -45,6 +45,7 @@ constexpr uint64_t kFewLeft = 8;
 // adds cost more (8 M tokens, 153 groups: refinement 0.72 ms for 0.50).
 constexpr int kNarrowSpw = 16;
 constexpr uint32_t kManySmall = 1u << 14;
+constexpr uint64_t kFewLarge = 16;  // pairs per group of 9 and more that build ranks late
 constexpr uint64_t kForkGroups = 1ull << 16;  // rounds of fewer groups stay on one stream
 constexpr uint64_t kDirectMaxH = 4096; // deeper groups fall back to rank doubling
 constexpr int kKeyThreads = 256;
@@ -4150,15 +4151,30 @@ capssa_status core_sort(Ctx &c, const EngineArgs &a, uint32_t **sa_out, eng::Pac
         c.stats.refine_rounds++;
         const int nxt = cur ^ 1;
         // rank doubling reads position-ordered ranks; they are built from the
-        // SA-ordered heads the first time a round needs them
+        // SA-ordered heads the first time a round needs them.  Where nearly all
+        // groups are pairs and threes they are built after that round's direct
+        // kernels, which then have no ranks to write: such a kernel does
+        // little else than its random writes of 4 bytes (round 1 of a masked
+        // genome of 134 M, 9.4 M pairs: 1.08 ms of direct kernels, 1.48 with
+        // ranks to keep; the build 12.70 for 13.10 ms).  The kernels of larger
+        // groups are bound by their ordering and hide the writes (word bytes,
+        // 50 M, 443,000 such groups beside 1.7 M pairs: 14.06 ms late, 13.84
+        // early).
         kt.start(c.stream);
-        if ((nb || cnt[L_DEEP]) && !ranks_ready) {
+        auto build_ranks = [&]() -> capssa_status {
+            if (!(nb || cnt[L_DEEP]) || ranks_ready) return CAPSSA_OK;
             // beyond L2 the sorted keys' buffers (dead once the groups are
             // listed) hold the window pairs and counts
-            s = scatter_u32(c, sa, hd, nn, rank, n, keys_a, (uint32_t *)keys_b);
-            if (s != CAPSSA_OK) return s;
+            const capssa_status rs =
+                scatter_u32(c, sa, hd, nn, rank, n, keys_a, (uint32_t *)keys_b);
+            if (rs != CAPSSA_OK) return rs;
             ranks_ready = true;
             kt.mark(c.stream, "ranks");
+            return CAPSSA_OK;
+        };
+        if (((uint64_t)cnt[L_SMALL] + cnt[L_MEDIUM]) * kFewLarge > cnt[L_PAIR]) {
+            s = build_ranks();
+            if (s != CAPSSA_OK) return s;
         }
         uint32_t *rk = ranks_ready ? rank : nullptr;
         CAPSSA_CUDA(c, cudaMemsetAsync(&G.ctr->half[nxt], 0, sizeof(G.ctr->half[0]), c.stream));
@@ -4228,6 +4244,8 @@ capssa_status core_sort(Ctx &c, const EngineArgs &a, uint32_t **sa_out, eng::Pac
         // every group they resolved, which only refines them (equal ranks
         // still agree through h symbols) and settles the depth-0 groups of
         // early-ended suffixes, whose ranks agree on nothing yet
+        s = build_ranks();
+        if (s != CAPSSA_OK) return s;
         if (cnt[L_DEEP]) {
             gather_small_kernel<<<grid_for(cnt[L_DEEP], 128), 128, 0, c.stream>>>(
                 G.list[L_DEEP][cur], cnt[L_DEEP], sa, rank, a.lim, h, lf, empty_lf, key2);

@@ -454,6 +454,35 @@ def test_run_groups_longer_first(ctx, n, longest):
                           orc.build_in_memory(t, None, orc.Limits(n, ends, True)))
 
 
+@pytest.mark.parametrize("pairs,mediums", [(4000, 0), (4000, 40), (40, 40)])
+@pytest.mark.parametrize("longer_first", [False, True])
+def test_ranks_built_before_and_after_the_direct_kernels(ctx, pairs, mediums, longer_first):
+    """A first round with a group too large for a block (a run) among many
+    pairs and few or many groups of 40: position-ordered ranks are built on
+    either side of the direct kernels, and the run's suffixes are ordered by
+    the ranks of suffixes those kernels have just resolved."""
+    rng = np.random.default_rng(pairs + mediums)
+    parts = []
+    for copies, groups in ((2, pairs), (40, mediums)):
+        for _ in range(groups):
+            unit = rng.integers(0, 4, 40)
+            for _ in range(copies):
+                parts += [unit, rng.integers(0, 4, 3)]
+    ends = [unit for unit in (rng.integers(0, 4, 30) for _ in range(50))]
+    for q in range(300):  # runs that go on with a few repeated texts
+        parts += [np.full(20 + q % 5, 3), ends[q % 50], rng.integers(0, 4, 2)]
+    parts.append(np.full(5000, 3))
+    t = np.concatenate(parts).astype(np.uint8)
+    n = len(t)
+    cuts = np.unique(np.concatenate([rng.integers(1, n, 60), [n]]))
+    lp = capssa.SegmentedText(n, cuts, capssa.BoundaryRank.LONGER_FIRST if longer_first
+                              else capssa.BoundaryRank.SHORTER_FIRST)
+    got = ctx.build_in_memory(t, lp, capssa.Opts(tie_order=capssa.TieOrder.REFERENCE))
+    assert np.array_equal(got, orc.build_in_memory(t, None, orc.Limits(n, cuts, longer_first)))
+    if not longer_first:
+        assert np.array_equal(ctx.build_in_memory(t), orc.build_in_memory(t))
+
+
 @pytest.mark.parametrize("dtype", [np.uint8, np.uint32])
 @pytest.mark.parametrize("tail", [1, 64, 4097])
 def test_run_ends_found_across_words_and_levels(ctx, dtype, tail):
