@@ -2113,6 +2113,16 @@ __device__ __forceinline__ uint32_t pick32(const uint32_t (&A)[N], int q) {
     return v;
 }
 
+// The pairs of member t among those of M members (bit i * M + j, i < j).
+template <int M>
+__device__ __forceinline__ uint64_t pairs_of(int t) {
+    uint64_t m = 0;
+#pragma unroll
+    for (int u = 0; u < M; u++)
+        if (u != t) m |= 1ull << (u < t ? u * M + t : t * M + u);
+    return m;
+}
+
 // Tied groups of 3..4 members: one thread per group, in rounds of four
 // windows (128 DNA symbols): a round loads the next four windows of
 // every member with independent loads (one round trip for the group) and
@@ -2162,7 +2172,9 @@ __global__ void __launch_bounds__(128)
                 uint64_t w[M][4];
 #pragma unroll
                 for (int t = 0; t < M; t++)
-                    if (t < len) windows4_at(P, (uint64_t)pp[t] + base, w[t]);
+                    // (a settled member may have ended: its windows could lie
+                    // past the packed text)
+                    if (und64 & pairs_of<M>(t)) windows4_at(P, (uint64_t)pp[t] + base, w[t]);
 #pragma unroll
                 for (int i = 0; i < M; i++)
 #pragma unroll
@@ -2290,9 +2302,10 @@ __global__ void __launch_bounds__(128)
         for (int x = 1; x < S; x <<= 1) lmin = min(lmin, __shfl_xor_sync(0xffffffffu, lmin, x));
         const bool fast = base + span <= (lmin < horizon ? lmin : horizon);
         const uint64_t step = horizon - base < span ? horizon - base : span;
-        const bool seg_busy = (__ballot_sync(0xffffffffu, und != 0) >> sb) & ((1u << S) - 1u);
         uint64_t w[4] = {0, 0, 0, 0};
-        if (mine && fast && seg_busy) windows4_at(P, (uint64_t)my_p + base, w);
+        // (relations settle in both lanes at once: nobody needs a settled
+        // member's windows, and one that has ended could read past the packed text)
+        if (fast && und) windows4_at(P, (uint64_t)my_p + base, w);
 #pragma unroll
         for (int u = 0; u < S; u++) {
             int r = 0;

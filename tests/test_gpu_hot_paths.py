@@ -361,6 +361,27 @@ def test_members_that_end_inside_a_deep_group(ctx, members, sigma):
         assert np.array_equal(got, orc.build_in_memory(t, None, orc.Limits(n, ends, lf)))
 
 
+@pytest.mark.parametrize("members", [3, 4, 5, 8, 9])
+@pytest.mark.parametrize("sigma,dtype", [(4, np.uint8), (200, np.uint8), (1 << 32, np.uint32)])
+@pytest.mark.parametrize("cut", [20, 300, 4000])
+def test_group_with_a_member_that_ends_with_the_text(ctx, members, sigma, dtype, cut):
+    """Copies of one passage, the last of them cut short by the text's end:
+    that member settles spans before the others part, and windows behind it
+    would lie past the packed text."""
+    rng = np.random.default_rng(members + cut)
+    unit = rng.integers(0, sigma, 9000, dtype=np.uint64)
+    parts = [rng.integers(0, sigma, 9000, dtype=np.uint64)]
+    for i in range(members - 1):
+        parts += [unit, np.array([i % 4], np.uint64)]
+    t = np.concatenate(parts + [unit[:cut]]).astype(dtype)
+    n = len(t)
+    for lf in (False, True):
+        b = capssa.BoundaryRank.LONGER_FIRST if lf else capssa.BoundaryRank.SHORTER_FIRST
+        want = orc.build_in_memory(t, None, orc.Limits(n, None, lf))
+        with capssa.Context(0) as fresh:  # a workspace of this text's size
+            assert np.array_equal(fresh.build_in_memory(t, capssa.PlainText(n, b)), want)
+
+
 @pytest.mark.parametrize("groups", [2000, 17000])
 @pytest.mark.parametrize("sigma", [9, 16, 20, 200])
 def test_groups_of_9_to_32_in_narrow_windows(ctx, groups, sigma):
