@@ -2938,7 +2938,8 @@ __global__ void __launch_bounds__(256, 8)
     for (uint64_t b0 = warp * 32 * kSteps; b0 < m; b0 += stride) {
         if (kRuns && b0 + kSteps * 32 <= m) {
             const uint64_t p0 = (uint64_t)pos[b0], p1 = (uint64_t)pos[b0 + kSteps * 32 - 1];
-            if (p1 == p0 + kSteps * 32 - 1 && p1 < n) {
+            // (p0 < n too: 64-bit positions that run past 2^64 are no run)
+            if (p1 == p0 + kSteps * 32 - 1 && p0 < n && p1 < n) {
                 bool run = true;
 #pragma unroll
                 for (uint32_t j = 0; j < kSteps; j++)

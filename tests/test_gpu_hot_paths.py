@@ -604,3 +604,18 @@ def test_subsets_of_consecutive_positions(ctx, dtype, first, last):
         pos = pos.astype(dtype)
         got = ctx.build_in_memory_for_positions(t, pos)
         assert np.array_equal(got, orc.build_in_memory(t, pos, index=dtype)), len(pos)
+
+
+@pytest.mark.parametrize("before", [0, 256, 300])
+def test_positions_that_wrap_past_2p64_are_refused(ctx, before):
+    """Consecutive 64-bit positions from below 2^64 through 0 (negative signed
+    positions): the same error as for any position beyond the text."""
+    n = 4096
+    t = np.random.default_rng(before).integers(0, 4, n).astype(np.uint8)
+    wrap = np.arange(-200, 800, dtype=np.int64).view(np.uint64)
+    pos = np.concatenate([np.arange(1000, 1000 + before, dtype=np.uint64), wrap])
+    with pytest.raises(ValueError, match="beyond the end of the text"):
+        ctx.build_in_memory_for_positions(t, pos)
+    ok = np.arange(n, dtype=np.uint64)  # the context stays usable
+    assert np.array_equal(ctx.build_in_memory_for_positions(t, ok),
+                          orc.build_in_memory(t, ok, index=np.uint64))
