@@ -76,6 +76,7 @@ capssa_status check_dev_flags(Ctx &c) {
     CAPSSA_CUDA(c, cudaMemcpyAsync(flags_readback(c), c.d_flags, 4, cudaMemcpyDeviceToHost,
                                    c.stream));
     CAPSSA_CUDA(c, cudaStreamSynchronize(c.stream));
+    c.flags_read_at = c.launches;
     return flags_status(c);
 }
 
@@ -338,6 +339,7 @@ struct CallScope {
         c.timed_passes = -1;
         c.timed_finish = false;
         c.waited = false;
+        c.flags_read_at = ~0ull;
         cudaSetDevice(c.device);
         cudaMemsetAsync(c.d_flags, 0, 16, c.stream);
         cudaEventRecord(c.ev0, c.stream);
@@ -378,10 +380,20 @@ struct CallScope {
     }
 };
 
+// Nothing reaches the host from a call whose device waits failed: the flags
+// are read before the first copy, and again where kernels ran since.
+capssa_status flags_before_host(Ctx &c) {
+    return c.flags_read_at == c.launches ? CAPSSA_OK : check_dev_flags(c);
+}
+
 // Deliver a device result to a host or device destination.
 capssa_status stage_out(Ctx &c, void *dst, const void *dsrc, size_t bytes) {
     if (!bytes || dst == dsrc) return CAPSSA_OK;
     bool dev = is_device_ptr(dst);
+    if (!dev) {
+        const capssa_status s = flags_before_host(c);
+        if (s != CAPSSA_OK) return s;
+    }
     auto t0 = std::chrono::steady_clock::now();
     CAPSSA_CUDA(c, cudaMemcpyAsync(dst, dsrc, bytes,
                                    dev ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost,
@@ -408,15 +420,13 @@ struct PartRequest {
     uint64_t *sizes;   // host, p
 };
 
-// Every builder funnels through here.  deliver: the caller passes the device
-// output on to the host itself.
+// Every builder funnels through here.
 template <typename ST>
 capssa_status build_common(Ctx &c, const ST *text, uint64_t n, const void *positions,
                            int pos_bytes, uint64_t m, const capssa_limits *lp,
                            const capssa_opts *opts, void *out_sa, int out_bytes, void *out_lcp,
                            const PartRequest *part = nullptr, uint64_t seg_major_len = 0,
-                           const uint32_t *keep_bits = nullptr, bool in_memory = false,
-                           bool deliver = false) {
+                           const uint32_t *keep_bits = nullptr, bool in_memory = false) {
     if (!text && n) return set_err(c, CAPSSA_EINVAL, "null text");
     if (opts && (opts->tie_order < CAPSSA_TIES_POSITION || opts->tie_order > CAPSSA_TIES_REFERENCE))
         return set_err(c, CAPSSA_EINVAL, "unknown tie order");
@@ -470,6 +480,7 @@ capssa_status build_common(Ctx &c, const ST *text, uint64_t n, const void *posit
         if (done) {
             c.stats.n_suffixes = n;
             c.waited = true;
+            c.flags_read_at = c.launches;  // none of its launches waits
             return out_dev ? CAPSSA_OK : stage_out(c, out_sa, d_out, count * (size_t)out_bytes);
         }
     }
@@ -506,11 +517,6 @@ capssa_status build_common(Ctx &c, const ST *text, uint64_t n, const void *posit
     if (positions && m == 0) return CAPSSA_OK;
     s = engine_build(c, a);
     if (s != CAPSSA_OK) return s;
-    if (!out_dev || (out_lcp && !lcp_dev) || deliver) {
-        // nothing reaches the host from a build whose device waits failed
-        s = check_dev_flags(c);
-        if (s != CAPSSA_OK) return s;
-    }
     if (!out_dev) {
         s = stage_out(c, out_sa, d_out, count * (size_t)out_bytes);
         if (s != CAPSSA_OK) return s;
@@ -549,7 +555,8 @@ uint64_t effective_p(uint64_t n, uint64_t requested, int threads) {
 // each batch copied to pinned memory while the previous one is consumed.
 capssa_status emit_stream(Ctx &c, const uint64_t *d_sa, uint64_t count, capssa_emit_fn emit,
                           void *user) {
-    capssa_status s = CAPSSA_OK;
+    capssa_status s = flags_before_host(c);
+    if (s != CAPSSA_OK) return s;
     const uint64_t batch = 1u << 22;
     if (!c.h_emit) CAPSSA_CUDA(c, cudaMallocHost(&c.h_emit, 2 * batch * 8));
     uint64_t *h = c.h_emit;
@@ -596,8 +603,7 @@ capssa_status sample_sort_common(Ctx &c, const ST *text, uint64_t n, const uint6
                    part_mode(opts),
                    nullptr, nullptr};
     capssa_status s =
-        build_common<ST>(c, text, n, positions, 8, m, lp, opts, d_sa, 8, nullptr, &pr, 0, nullptr,
-                         false, /*deliver=*/true);
+        build_common<ST>(c, text, n, positions, 8, m, lp, opts, d_sa, 8, nullptr, &pr);
     if (s != CAPSSA_OK) return s;
     return emit_stream(c, d_sa, count, emit, user);
 }
@@ -619,7 +625,7 @@ capssa_status ext_mem_common(Ctx &c, const ST *text, uint64_t n, const void *pos
     uint64_t *d_sa = (uint64_t *)ws_get(c, WS_OUT, count * 8 + 64);
     if (!d_sa) return set_err(c, CAPSSA_ENOMEM, "output buffer");
     capssa_status s = build_common<ST>(c, text, n, positions, pos_bytes, m, lp, opts, d_sa, 8,
-                                       nullptr, nullptr, 0, keep_bits, false, /*deliver=*/true);
+                                       nullptr, nullptr, 0, keep_bits);
     if (s != CAPSSA_OK) return s;
     return emit_stream(c, d_sa, count, emit, user);
 }
@@ -1285,7 +1291,9 @@ capssa_status capssa_selftest_bounded_wait(capssa_ctx *ctx, uint32_t polls) {
         return scope.finish(set_err(c, CAPSSA_ECUDA, "self-test word clear"));
     bounded_wait_kernel<<<1, 32, 0, c.stream>>>(word, polls, c.d_flags);
     c.launches++;
-    return scope.finish(CAPSSA_OK);
+    // (a delivery after the wait: refused, so no bytes reach the host)
+    unsigned long long got = 0;
+    return scope.finish(stage_out(c, &got, word, sizeof(got)));
 }
 
 capssa_status capssa_cdf_grad(capssa_ctx *ctx, const float *params, const uint64_t *prefixes,

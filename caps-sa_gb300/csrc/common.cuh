@@ -153,6 +153,8 @@ struct Ctx {
     // the call's last kernel has been waited for, ev1 recorded after it (a small
     // text, which sets no device flags)
     bool waited = false;
+    // launches when the device flags were last read (see stage_out)
+    uint64_t flags_read_at = ~0ull;
     // the last sort produced segment-major order (every segment contiguous)
     bool seg_major_done = false;
     uint64_t *h_emit = nullptr;     // pinned double buffer of the emit stream

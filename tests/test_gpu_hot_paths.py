@@ -619,3 +619,21 @@ def test_positions_that_wrap_past_2p64_are_refused(ctx, before):
     ok = np.arange(n, dtype=np.uint64)  # the context stays usable
     assert np.array_equal(ctx.build_in_memory_for_positions(t, ok),
                           orc.build_in_memory(t, ok, index=np.uint64))
+
+
+# ---------------------------------------------------------------- deliveries to the host
+
+def test_no_result_reaches_the_host_after_a_failed_wait(ctx):
+    """A delivery behind a device wait that gave up is refused before its copy;
+    builds into host buffers read the flags once however many outputs they have."""
+    with pytest.raises(capssa.CapsSaError) as ei:
+        ctx.selftest_bounded_wait(64)
+    assert ei.value.status == capssa.Status.ETIMEOUT
+    assert ctx.stats()["d2h_bytes"] == 0
+    t = np.random.default_rng(1).integers(0, 4, 30000).astype(np.uint8)
+    sa, lcp = ctx.build_in_memory_lcp(t)
+    assert ctx.stats()["d2h_bytes"] == sa.nbytes + lcp.nbytes
+    assert np.array_equal(sa, orc.build_in_memory(t))
+    offs = np.array([0, 10000, 30000], np.uint64)
+    got = ctx.build_batched(t, offs)
+    assert ctx.stats()["d2h_bytes"] == got.nbytes
