@@ -226,14 +226,19 @@ KeyGeom pf_geom(int b, uint64_t n, bool plain, double hbits, int bucket_bits) {
 
 namespace {
 
-bool is_device_ptr(const void *p) {
+bool pointer_attributes(const void *p, cudaPointerAttributes *attr) {
     if (!p) return false;
-    cudaPointerAttributes attr;
-    if (cudaPointerGetAttributes(&attr, p) != cudaSuccess) {
+    if (cudaPointerGetAttributes(attr, p) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }
-    return attr.type == cudaMemoryTypeDevice || attr.type == cudaMemoryTypeManaged;
+    return true;
+}
+
+bool is_device_ptr(const void *p) {
+    cudaPointerAttributes attr;
+    return pointer_attributes(p, &attr) &&
+           (attr.type == cudaMemoryTypeDevice || attr.type == cudaMemoryTypeManaged);
 }
 
 double ms_since(std::chrono::steady_clock::time_point t0) {
@@ -443,15 +448,18 @@ capssa_status build_common(Ctx &c, const ST *text, uint64_t n, const void *posit
     // inside it: only the alphabet, packing and run kernels do (16-byte loads
     // of a u8 text); those of a finite context, a partition plan or the
     // reference's tie order read past the end and need the padded copy, as does
-    // a text that the outputs overlap.  (268 M symbols: 0.08 ms.)
+    // a text that the outputs overlap, and one on another GPU.  (268 M symbols:
+    // 0.08 ms.)
     auto overlaps = [&](const void *p, uint64_t bytes) {
         return p && (uintptr_t)p < (uintptr_t)text + n * sizeof(ST) &&
                (uintptr_t)text < (uintptr_t)p + bytes;
     };
     const uint64_t out_total = (chosen ? m : n) * (uint64_t)out_bytes;
+    cudaPointerAttributes attr;
     if (n && ((uintptr_t)text & 15) == 0 && max_ctx >= n && !part &&
         !(opts && opts->tie_order == CAPSSA_TIES_REFERENCE) && !overlaps(out_sa, out_total) &&
-        !overlaps(out_lcp, out_total) && is_device_ptr(text)) {
+        !overlaps(out_lcp, out_total) && pointer_attributes(text, &attr) &&
+        kernels_reach(attr, c.device)) {
         d_text = const_cast<ST *>(text);
     } else {
         s = stage_text(c, text, n, &d_text);

@@ -190,6 +190,14 @@ capssa_status cuda_err(Ctx &c, cudaError_t e, const char *where);
 // Bytes of the pinned scratch; its last 64 are the device flags' read-back.
 constexpr size_t kScratchBytes = 1 << 16;
 
+// Whether the kernels of a context on `device` can read memory with these
+// attributes where it lies: its own GPU's, and managed memory (another GPU's
+// is reached by copies only, without peer access).
+inline bool kernels_reach(const cudaPointerAttributes &attr, int device) {
+    return attr.type == cudaMemoryTypeManaged ||
+           (attr.type == cudaMemoryTypeDevice && attr.device == device);
+}
+
 // Device flag check: returns CAPSSA_ETIMEOUT / CAPSSA_ENOMEM after a sync.
 capssa_status check_dev_flags(Ctx &c);
 
