@@ -637,3 +637,60 @@ def test_no_result_reaches_the_host_after_a_failed_wait(ctx):
     offs = np.array([0, 10000, 30000], np.uint64)
     got = ctx.build_batched(t, offs)
     assert ctx.stats()["d2h_bytes"] == got.nbytes
+
+
+# ---------------------------------------------------------------- outputs that share the text's memory
+
+def _overlap_text(kind, n):
+    rng = np.random.default_rng(n)
+    t = rng.integers(0, 4, n)
+    if kind == "gives_up":  # a small text too deep for one block
+        t = np.tile(t[:500], n // 500 + 1)[:n]
+    elif kind == "runs":
+        for i in range(30):
+            at = int(rng.integers(0, n - 3000))
+            t[at:at + 2500] = i % 4
+    return t.astype(np.uint8)
+
+
+@pytest.mark.parametrize("kind,n", [("random", 5000), ("gives_up", 8000), ("runs", 200003)])
+@pytest.mark.parametrize("bytes_", [4, 8])
+@pytest.mark.parametrize("where", ["before", "same", "inside", "last_byte", "past"])
+@pytest.mark.parametrize("with_lcp", [False, True])
+def test_outputs_that_overlap_a_device_text(ctx, kind, n, bytes_, where, with_lcp):
+    """The suffix array or the LCP array laid over the text's own bytes, which
+    are then lost, or right behind them: the order is that of the text as it
+    was at the call."""
+    torch = pytest.importorskip("torch")
+    t = _overlap_text(kind, n)
+    want = orc.build_in_memory(t)
+    start = n * bytes_ + 64 & ~15  # of the text in the buffer, 16-byte aligned
+    end = start + n
+    at = {"before": start - (n * bytes_ // 2), "same": start, "inside": start + n // 2,
+          "last_byte": end - 1, "past": end + 15}[where] & ~15
+    buf = torch.zeros(at + (n + 2) * bytes_ + end, dtype=torch.uint8, device="cuda")
+    buf[start:end] = torch.from_numpy(t).cuda()
+    kind_t = torch.int32 if bytes_ == 4 else torch.int64
+    text = buf[start:end]
+    over = buf[at:at + n * bytes_].view(kind_t)
+    torch.cuda.synchronize()
+    if with_lcp:
+        sa = torch.zeros(n, dtype=kind_t, device="cuda")
+        torch.cuda.synchronize()
+        fn = getattr(capssa.lib, "capssa_build_in_memory_lcp_u8_u%d" % (8 * bytes_))
+        assert fn(ctx._h, text.data_ptr(), n, None, 0, None, None, sa.data_ptr(),
+                  over.data_ptr()) == 0
+        lcp = over.cpu().numpy()
+        assert lcp[0] == 0
+        i = np.arange(1, n)
+        w = want.astype(np.int64)
+        # equal for lcp symbols, then different or ended
+        a, b = w[i - 1] + lcp[1:], w[i] + lcp[1:]
+        live = np.maximum(a, b) < n
+        assert (np.maximum(a, b) <= n).all() and (t[a[live]] != t[b[live]]).all()
+        for j in np.random.default_rng(3).choice(i, 200):
+            assert np.array_equal(t[w[j - 1]:w[j - 1] + lcp[j]], t[w[j]:w[j] + lcp[j]])
+    else:
+        sa = over
+        ctx.build_in_memory(text, out=sa)
+    assert np.array_equal(sa.cpu().numpy().astype(np.int64), want.astype(np.int64))
