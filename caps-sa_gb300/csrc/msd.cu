@@ -609,7 +609,17 @@ capssa_status run(Ctx &c, const Plan &pl, uint64_t *ka, uint32_t *va, uint64_t *
     for (int level = first;; level++) {
         // this level's digit
         Digit dg;
-        const int want = level < 0 ? pl.given : level < pl.levels ? pl.bits[level] : kExtraBits;
+        int want = level < 0 ? pl.given : level < pl.levels ? pl.bits[level] : kExtraBits;
+        if (level > first && (uint64_t)nr_bound << want > kFreeBins) {
+            // the ranges there can be, times the digit's values, is a lot of
+            // bins (10,000 texts, one of them of 250 M symbols: up to 9 GB), and
+            // mostly few ranges are left: read their number
+            CAPSSA_CUDA(c, cudaMemcpyAsync(hc, ctr[cur], sizeof(Counters), cudaMemcpyDeviceToHost,
+                                           c.stream));
+            CAPSSA_CUDA(c, cudaStreamSynchronize(c.stream));
+            nr_bound = std::max(1u, std::min(nr_bound, hc->ranges));
+            want = level_bits(n, nr_bound, want);
+        }
         if (key_left > 0) {
             dg.bits = std::min(want, key_left);
             key_left -= dg.bits;

@@ -29,6 +29,17 @@ constexpr int kMaxGiven = 14;  // ... of a given one (a chunk holds 15 bits of d
 // instead (2,048 genomes of 47,000 symbols: 2.83 ms for 3.40 with two levels
 // over both, whose first moved every tile's records to the same few digits).
 Plan plan(uint64_t n, int nbits, int top_bits, uint64_t longest, double eff, bool in_pieces);
+// Digit bits of a level past the first over `ranges` ranges of n records, at
+// most `want`.  Its bins, a word for each digit value of each range, stay
+// within 64 MB or a byte a record, whichever is more.  A range holds over
+// kOneBlock / 2 records, so 8 bits always fit; what a wider digit leaves is up to
+// the levels past the planned ones.
+constexpr uint64_t kFreeBins = 1ull << 24;
+inline int level_bits(uint64_t n, uint64_t ranges, int want) {
+    const uint64_t most = n / 4 > kFreeBins ? n / 4 : kFreeBins;
+    while (want > 1 && ranges << want > most) want--;
+    return want;
+}
 // The pieces of a plan with given bits: piece i ends at record ends[i]
 // (device), and the last at n.
 struct Pieces {

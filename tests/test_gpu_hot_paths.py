@@ -306,6 +306,36 @@ def test_record_sort_of_given_pieces(ctx, sigma, dtype, lens):
             assert np.array_equal(got[offs[i]:offs[i + 1]], orc.build_in_memory(tx)), i
 
 
+def test_workspace_of_one_long_text_among_many(ctx):
+    """10,001 texts, one of them nearly all of the symbols: the levels over the
+    long one need bins for its ranges, not for all there could be."""
+    torch = pytest.importorskip("torch")
+    n = 300000011
+    g = torch.Generator(device="cuda")
+    g.manual_seed(5)
+    cat = torch.randint(0, 4, (n,), generator=g, device="cuda", dtype=torch.uint8)
+    out = torch.empty(n, dtype=torch.int32, device="cuda")
+    lens = np.random.default_rng(5).integers(1, 900, 10000)
+    lens = np.insert(lens, 4321, n - lens.sum())
+    many = np.concatenate([[0], np.cumsum(lens)]).astype(np.uint64)
+    torch.cuda.synchronize()
+    used = []
+    for offs in (np.array([0, 1000, n], np.uint64), many):
+        with capssa.Context(0) as fresh:
+            fresh.build_batched(cat, offs, out=out)
+            used.append(fresh.workspace_bytes())
+    print("workspace: %.2f bytes a symbol, %.2f with many texts" % (used[0] / n, used[1] / n))
+    assert used[1] - used[0] < 0.6 * n
+    a, b = int(many[4321]), int(many[4322])
+    alone = torch.empty(b - a, dtype=torch.int32, device="cuda")
+    ctx.build_in_memory(cat[a:b], out=alone)
+    assert bool((out[a:b] == alone).all())
+    for i in (0, 4320, 4322, 10000):
+        a, b = int(many[i]), int(many[i + 1])
+        assert np.array_equal(out[a:b].cpu().numpy().view(np.uint32),
+                              orc.build_in_memory(cat[a:b].cpu().numpy())), i
+
+
 # ---------------------------------------------------------------- horizons of the direct rounds
 
 @pytest.mark.parametrize("lcp", [255, 256, 257, 600, 2303, 2304, 2305, 5000])

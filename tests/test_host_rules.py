@@ -13,6 +13,7 @@ CSRC = os.path.join(ROOT, "caps-sa_gb300", "csrc")
 PROGRAM = r"""
 #include <cstdio>
 #include "common.cuh"
+#include "msd.cuh"
 using namespace capssa;
 
 int main() {
@@ -28,6 +29,15 @@ int main() {
                 a.device = d;
                 std::printf("%s[%d, %d, %d, %d]", t || d || c ? ", " : "", t, d, c,
                             (int)kernels_reach(a, c));
+            }
+    // bins: records, ranges, bits asked for -> bits taken
+    std::printf("], \"bins\": [");
+    const char *sep = "";
+    for (unsigned long long n = 5000; n < 1ull << 32; n = n * 3 + 1)
+        for (unsigned long long r = 1; r <= n / (msd::kOneBlock / 2 + 1) + 1; r = r * 5 + 2)
+            for (int want = 1; want <= msd::kMaxDigit; want++) {
+                std::printf("%s[%llu, %llu, %d, %d]", sep, n, r, want, msd::level_bits(n, r, want));
+                sep = ", ";
             }
     std::printf("]}\n");
     return 0;
@@ -55,3 +65,15 @@ def test_a_text_is_read_in_place_on_its_own_gpu_only(rules):
     for kind, device, context, reach in rules["reach"]:
         want = kind == 3 or (kind == 2 and device == context)
         assert bool(reach) == want, (kind, device, context)
+
+
+def test_bins_of_a_level_stay_within_a_byte_a_record(rules):
+    """... or 64 MB; eight bits of digit, what the levels past the planned ones
+    take, are never refused, and nothing is cut that fits."""
+    assert len(rules["bins"]) > 500
+    for n, ranges, want, got in rules["bins"]:
+        most = max(n // 4, 1 << 24)
+        assert 1 <= got <= want
+        assert got >= min(want, 8)
+        assert ranges << got <= most
+        assert got == want or ranges << (got + 1) > most
