@@ -2376,10 +2376,11 @@ __global__ void __launch_bounds__(128)
 // settled by direct_cmp (ties by position), the others go on by rounds.  A member's place is the count of members
 // before it, so the relation to its sorted predecessor is already known.
 // Groups deeper than kDirectMaxH are left to rank doubling.
-__global__ void direct_warp_kernel(const uint4 *__restrict__ groups, uint32_t count,
-                                   uint32_t *__restrict__ sa, uint32_t *__restrict__ hd,
-                                   uint32_t *__restrict__ rank, DevLimits L, Packed P, int lf, uint64_t dcap,
-                                   GroupLists G, int nxt) {
+__global__ void __launch_bounds__(128, 6)
+    direct_warp_kernel(const uint4 *__restrict__ groups, uint32_t count,
+                       uint32_t *__restrict__ sa, uint32_t *__restrict__ hd,
+                       uint32_t *__restrict__ rank, DevLimits L, Packed P, int lf, uint64_t dcap,
+                       GroupLists G, int nxt) {
     const uint32_t lane = threadIdx.x & 31;
     const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
     const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
