@@ -48,6 +48,16 @@ constexpr uint32_t kManySmall = 1u << 14;
 constexpr uint64_t kFewLarge = 16;  // pairs per group of 9 and more that build ranks late
 constexpr uint64_t kForkGroups = 1ull << 16;  // rounds of fewer groups stay on one stream
 constexpr uint64_t kDirectMaxH = 4096; // deeper groups fall back to rank doubling
+// Groups of 33..kMediumMax members take about twice the steps for every
+// doubling of their depth, which a few of them are worth: ranks for a text of 64 M
+// cost 0.9 ms, and 1 in 20 of its suffixes in such groups, 40 copies of a passage
+// a group, went on to depth 4,096 in 8.7 ms where leaving at 512 made it 9.8.  But
+// where a quarter of the suffixes are in them, rank doubling orders them all in
+// little more than that each round, and those past kManyMediumH symbols go
+// there: 1,000 copies of a 30,000-symbol text, one substitution in 10,000, took
+// 643 ms to 4,096 symbols and take 119; 50 copies of 262,144 symbols 74 and 22.
+constexpr uint64_t kManyMedium = 4;    // suffixes per member of such groups
+constexpr uint64_t kManyMediumH = 512;
 constexpr int kKeyThreads = 256;
 constexpr int kKeyPer = 8;          // positions per thread in the key kernel
 constexpr int kKeyTile = kKeyThreads * kKeyPer;
@@ -67,6 +77,7 @@ enum GroupList : int {
     L_TINY8 = 5,   // 5..8 members: eight lanes
     kLists = 6     // larger groups: the radix (rank doubling) path
 };
+constexpr int kMembers = kLists;  // counter of the block kernels' L_MEDIUM members
 constexpr uint32_t kTinyMax = 8;
 constexpr uint32_t kTiny4 = 4;
 constexpr int kPairBurst = 4;  // windows the pair kernel loads in its first round trip
@@ -78,7 +89,7 @@ struct Counters {
         unsigned long long big_packed;  // (ordinal << 40) | element total
     } half[2];
 };
-static_assert(kLists <= 8, "a counter per list");
+static_assert(kMembers < 8, "a counter per list, and the members'");
 constexpr unsigned long long kBigOrdUnit = 1ull << 40;
 constexpr unsigned long long kBigTotMask = kBigOrdUnit - 1;
 
@@ -596,6 +607,7 @@ struct GroupLists {
     uint4 *list[kLists][2];  // (start, len, depth, 0)
     BigGroup *big[2];
     Counters *ctr;
+    uint32_t medium_h;  // depth past which L_MEDIUM's sizes go to rank doubling
 };
 
 // The lists are kernel parameters: indexing them with a runtime value would
@@ -612,13 +624,14 @@ __device__ __forceinline__ BigGroup *big_ptr(const GroupLists &G, int q) {
 
 // List of a still-tied group whose members agree on `depth` symbols
 // (kLists = the radix path).
-__device__ __forceinline__ int list_of(uint32_t len, uint64_t depth) {
+__device__ __forceinline__ int list_of(uint32_t len, uint64_t depth,
+                                       uint64_t medium_h = kDirectMaxH) {
     if (len <= kSmallMax && depth > kDirectMaxH) return L_DEEP;
     if (len == 2) return L_PAIR;
     if (len <= kTiny4) return L_TINY;
     if (len <= kTinyMax) return L_TINY8;
     if (len <= kSmallMax) return L_SMALL;
-    if (len <= kMediumMax && depth <= kDirectMaxH) return L_MEDIUM;
+    if (len <= kMediumMax && depth <= medium_h) return L_MEDIUM;
     return kLists;
 }
 
@@ -661,7 +674,7 @@ __device__ __forceinline__ uint32_t warp_append(uint32_t *counter) {
 // Route a still-tied group to the next round's list (any thread, any time).
 __device__ __forceinline__ void append_group(const GroupLists &G, int nxt, uint32_t start,
                                              uint32_t len, uint64_t depth) {
-    int l = list_of(len, depth);
+    int l = list_of(len, depth, G.medium_h);
     if (l == kLists) {
         append_big(G, nxt, start, len, depth);
         return;
@@ -2507,7 +2520,7 @@ __global__ void __launch_bounds__(THREADS)
     __shared__ uint32_t s_wmax[THREADS / 32];
     __shared__ uint2 s_own[kGather ? kQueue : 1];
     uint2 *s_q = kGather ? s_own : reinterpret_cast<uint2 *>(sw);
-    __shared__ uint32_t s_qn, s_cnt[kLists], s_base[kLists];
+    __shared__ uint32_t s_qn, s_cnt[kMembers + 1], s_base[kMembers + 1];
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t spw = (uint32_t)P.spw;
     const uint32_t full = lf ? 0u : spw;  // st of a member with a whole window
@@ -2525,7 +2538,7 @@ __global__ void __launch_bounds__(THREADS)
     auto flush = [&]() {
         __syncthreads();
         const uint32_t nq = s_qn;
-        if (tid < kLists) s_cnt[tid] = 0;
+        if (tid <= kMembers) s_cnt[tid] = 0;
         __syncthreads();
         constexpr int kQPer = (int)((kQueue + THREADS - 1) / THREADS);
         uint32_t at[kQPer];
@@ -2533,12 +2546,15 @@ __global__ void __launch_bounds__(THREADS)
         for (int j = 0; j < kQPer; j++) {
             const uint32_t q = j * THREADS + tid;
             if (q < nq) {
-                const int l = list_of(s_q[q].y & 0xFFFu, s_q[q].y >> 12);
+                const uint32_t n2 = s_q[q].y & 0xFFFu;
+                const int l = list_of(n2, s_q[q].y >> 12, G.medium_h);
                 if (l < kLists) at[j] = atomicAdd(&s_cnt[l], 1u);
+                if (l == L_MEDIUM) atomicAdd(&s_cnt[kMembers], n2);
             }
         }
         __syncthreads();
-        if (tid < kLists && s_cnt[tid]) s_base[tid] = atomicAdd(&G.ctr->half[nxt].n[tid], s_cnt[tid]);
+        if (tid <= kMembers && s_cnt[tid])
+            s_base[tid] = atomicAdd(&G.ctr->half[nxt].n[tid], s_cnt[tid]);
         if (tid == 0) s_qn = 0;
         __syncthreads();
 #pragma unroll
@@ -2546,7 +2562,7 @@ __global__ void __launch_bounds__(THREADS)
             const uint32_t q = j * THREADS + tid;
             if (q < nq) {
                 const uint32_t start = s_q[q].x, n2 = s_q[q].y & 0xFFFu, dep = s_q[q].y >> 12;
-                const int l = list_of(n2, dep);
+                const int l = list_of(n2, dep, G.medium_h);
                 if (l < kLists)
                     list_ptr(G, l, nxt)[s_base[l] + at[j]] = group_entry(start, n2, dep);
                 else
@@ -4038,6 +4054,7 @@ capssa_status core_sort(Ctx &c, const EngineArgs &a, uint32_t **sa_out, eng::Pac
         }
     G.big[0] = (BigGroup *)cursor;
     G.big[1] = G.big[0] + big_cap;
+    G.medium_h = (uint32_t)kDirectMaxH;
     CAPSSA_CUDA(c, cudaMemsetAsync(G.ctr, 0, sizeof(Counters), c.stream));
     // packed positions are unpacked into vals_a, or straight into a u32 output
     // of a full build, which then needs no final copy
@@ -4201,6 +4218,11 @@ capssa_status core_sort(Ctx &c, const EngineArgs &a, uint32_t **sa_out, eng::Pac
             (uint64_t)cnt[L_PAIR] + cnt[L_TINY] + cnt[L_TINY8] + cnt[L_SMALL];
         const uint64_t dcap = n_groups < last_groups / kFewLeft ? kDirectCapFew : kDirectCap;
         last_groups = n_groups;
+        // (the members that the round before queued; from then on, or what
+        // rank doubling leaves tied would come back.  A subset's order has no
+        // ranks to double)
+        if (!sp && hc->half[cur].n[kMembers] * kManyMedium >= N)
+            G.medium_h = (uint32_t)kManyMediumH;
         // ... unless the round is small: then the forks and joins cost more than
         // they overlap
         const bool wide = n_groups + cnt[L_MEDIUM] >= kForkGroups;

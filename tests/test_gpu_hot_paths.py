@@ -412,6 +412,30 @@ def test_group_with_a_member_that_ends_with_the_text(ctx, members, sigma, dtype,
             assert np.array_equal(fresh.build_in_memory(t, capssa.PlainText(n, b)), want)
 
 
+@pytest.mark.parametrize("copies", [33, 300, 2048])
+@pytest.mark.parametrize("share", [1.0, 0.35, 0.2])
+@pytest.mark.parametrize("sigma,dtype", [(4, np.uint8), (100, np.uint8), (60000, np.uint32)])
+def test_deep_medium_groups_of_much_and_little_of_the_text(ctx, copies, share, sigma, dtype):
+    """Groups of 33 to 2,048 members that agree on hundreds to thousands of
+    symbols: all of the text, over and under the quarter of it that decides
+    where they go on, some members ended by a segment on the way."""
+    rng = np.random.default_rng(copies + sigma)
+    length = {33: 6500, 300: 1500, 2048: 800}[copies]
+    unit = rng.integers(0, sigma, length)
+    t = np.tile(unit, copies)
+    hit = rng.random(len(t)) < 0.0004
+    t[hit] = (t[hit] + 1) % sigma
+    t = np.concatenate([t, rng.integers(0, sigma, int(len(t) * (1 / share - 1)))]).astype(dtype)
+    n = len(t)
+    assert np.array_equal(ctx.build_in_memory(t), orc.build_in_memory(t))
+    ends = np.unique(np.concatenate([rng.integers(1, n, 40), [n]]))
+    for lf in (True, False):
+        lp = capssa.SegmentedText(n, ends, capssa.BoundaryRank.LONGER_FIRST if lf
+                                  else capssa.BoundaryRank.SHORTER_FIRST)
+        got = ctx.build_in_memory(t, lp, capssa.Opts(tie_order=capssa.TieOrder.REFERENCE))
+        assert np.array_equal(got, orc.build_in_memory(t, None, orc.Limits(n, ends, lf)))
+
+
 @pytest.mark.parametrize("groups", [2000, 17000])
 @pytest.mark.parametrize("sigma", [9, 16, 20, 200])
 def test_groups_of_9_to_32_in_narrow_windows(ctx, groups, sigma):
