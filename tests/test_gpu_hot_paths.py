@@ -504,6 +504,43 @@ def test_small_texts_too_deep_for_one_block(ctx, make):
     assert np.array_equal(ctx.build_in_memory(t), orc.build_in_memory(t))
 
 
+@pytest.mark.parametrize("lcp", [1, 20, 21, 22, 31, 32, 33, 63, 64, 65, 159, 160, 161, 319, 320, 321])
+@pytest.mark.parametrize("sigma,dtype", [(2, np.uint8), (4, np.uint8), (6, np.uint8),
+                                         (200, np.uint8), (1 << 32, np.uint32)])
+def test_small_texts_with_ties_at_window_edges(ctx, lcp, sigma, dtype):
+    """Suffixes that part, or end, just before, at and after the 64 bits
+    compared first and the 256 compared then."""
+    rng = np.random.default_rng(lcp)
+    unit = rng.integers(0, sigma, lcp, dtype=np.uint64)
+    parts = []
+    for i in range(3):
+        parts += [rng.integers(0, sigma, 40, dtype=np.uint64), unit, np.array([i % 2], np.uint64)]
+    t = np.concatenate(parts + [rng.integers(0, sigma, 40, dtype=np.uint64), unit]).astype(dtype)
+    n = len(t)
+    for lf in (False, True):
+        b = capssa.BoundaryRank.LONGER_FIRST if lf else capssa.BoundaryRank.SHORTER_FIRST
+        assert np.array_equal(ctx.build_in_memory(t, capssa.PlainText(n, b)),
+                              orc.build_in_memory(t, None, orc.Limits(n, None, lf)))
+
+
+@pytest.mark.parametrize("n", [700, 1000, 2000, 4000, 8000])
+@pytest.mark.parametrize("sigma,dtype", [(4, np.uint8), (200, np.uint8), (1 << 32, np.uint32)])
+@pytest.mark.parametrize("make", ["halves", "run", "period"])
+def test_small_texts_around_the_work_of_one_block(ctx, n, sigma, dtype, make):
+    """Comparisons below and above what one block takes on, known from the bins
+    alone (runs, short periods) or only on the way (equal halves)."""
+    rng = np.random.default_rng(n)
+    t = rng.integers(0, sigma, n, dtype=np.uint64)
+    if make == "halves":
+        t[n // 2:] = t[:n - n // 2]
+    elif make == "run":
+        t[100:100 + 400] = t[0]
+    else:
+        t = t[np.arange(n) % 5]
+    t = t.astype(dtype)
+    assert np.array_equal(ctx.build_in_memory(t), orc.build_in_memory(t))
+
+
 # ---------------------------------------------------------------- run groups, longer first
 
 @pytest.mark.parametrize("n,longest", [(1 << 17, 900), (1 << 20, 3000), (1 << 20, 70000)])
