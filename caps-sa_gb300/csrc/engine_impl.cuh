@@ -2485,7 +2485,8 @@ __global__ void __launch_bounds__(128, 6)
 // window is padded low (ShorterFirst) or high (LongerFirst) and ordered by
 // the symbols it still had, as the key records are.  The group leaves once it
 // is settled, or when its subgroups agree on twice the round's depth (what
-// rank doubling needs), and the subgroups then queue by their own size.
+// rank doubling needs) or `reach` symbols past it, and the subgroups then queue
+// by their own size.
 // Ordering: by counting inside 32 slots, then merges of doubling runs by
 // binary search, in which only subgroups that span both runs take part (a
 // bitonic network over the same windows: 20 ms where the large instantiation now
@@ -2502,7 +2503,7 @@ __global__ void __launch_bounds__(THREADS)
     direct_medium_kernel(const uint4 *__restrict__ groups, uint32_t count,
                          uint32_t *__restrict__ sa, uint32_t *__restrict__ hd,
                          uint32_t *__restrict__ rank, DevLimits L, Packed P, int lf,
-                         uint64_t round_h, GroupLists G, int nxt) {
+                         uint64_t round_h, uint64_t reach, GroupLists G, int nxt) {
     constexpr int kPer = (int)(MAXM / THREADS);
     static_assert(MAXM % THREADS == 0 && MAXM <= 2048, "slots per thread; lengths below 2^12");
     // subgroups to append, (start, length | depth << 12): the small
@@ -2576,7 +2577,8 @@ __global__ void __launch_bounds__(THREADS)
         const uint32_t len = g.y;
         if (len <= kLo || len > MAXM) continue;  // the other instantiation's
         const uint64_t h = g.z;
-        const uint64_t target = 2 * (h > round_h ? h : round_h);
+        const uint64_t from = h > round_h ? h : round_h;
+        const uint64_t target = from + (from > reach ? from : reach);
         uint64_t d = h;
 #pragma unroll
         for (int j = 0; j < kPer; j++) {
@@ -4254,7 +4256,7 @@ capssa_status core_sort(Ctx &c, const EngineArgs &a, uint32_t **sa_out, eng::Pac
         if (P.spw <= kNarrowSpw && cnt[L_SMALL] >= kManySmall) {
             direct_medium_kernel<kTinyMax, kSmallMax, 32>
                 <<<std::min<unsigned>(cnt[L_SMALL], c.sm_count * 32), 32, 0, side()>>>(
-                    G.list[L_SMALL][cur], cnt[L_SMALL], sa, hd, rk, a.lim, P, lf, h, G, nxt);
+                    G.list[L_SMALL][cur], cnt[L_SMALL], sa, hd, rk, a.lim, P, lf, h, 0, G, nxt);
             CAPSSA_LAUNCHED(c);
         } else if (cnt[L_SMALL]) {
             direct_warp_kernel<<<grid_for((uint64_t)cnt[L_SMALL] * 32, 128), 128, 0, side()>>>(
@@ -4264,12 +4266,17 @@ capssa_status core_sort(Ctx &c, const EngineArgs &a, uint32_t **sa_out, eng::Pac
         if (cnt[L_MEDIUM]) {
             // one list, two kernels: each takes the groups of its sizes
             const unsigned mg = std::min<unsigned>(cnt[L_MEDIUM], c.sm_count * 16);
+            // few groups, a block each at once: a round's launches and read-back
+            // cost more than what ends earlier in shallower steps, so they go at
+            // least as far as the other kernels do (1,000 symbols of period 3:
+            // 0.63 ms, 0.55 now; 8,000 skewed ones 0.57 and 0.51)
+            const uint64_t reach = cnt[L_MEDIUM] <= (uint32_t)c.sm_count ? kDirectCap : 0;
             direct_medium_kernel<kSmallMax, kMedSmall, 128><<<mg, 128, 0, side()>>>(
-                G.list[L_MEDIUM][cur], cnt[L_MEDIUM], sa, hd, rk, a.lim, P, lf, h, G, nxt);
+                G.list[L_MEDIUM][cur], cnt[L_MEDIUM], sa, hd, rk, a.lim, P, lf, h, reach, G, nxt);
             CAPSSA_LAUNCHED(c);
             direct_medium_kernel<kMedSmall, kMediumMax, 512>
                 <<<std::min<unsigned>(mg, c.sm_count * 4), 512, 0, c.stream>>>(
-                    G.list[L_MEDIUM][cur], cnt[L_MEDIUM], sa, hd, rk, a.lim, P, lf, h, G, nxt);
+                    G.list[L_MEDIUM][cur], cnt[L_MEDIUM], sa, hd, rk, a.lim, P, lf, h, reach, G, nxt);
             CAPSSA_LAUNCHED(c);
         }
         for (int i = 0; i < forked; i++) {
