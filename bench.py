@@ -167,21 +167,51 @@ def hbm_peak():
         return 6800.0, "fallback"
 
 
-def profiled_traffic(n, item_bytes):
-    """DRAM bytes per distribution level from the committed ncu summary for
-    this record width (captured at 2^26 records, input 4x L2), scaled by
-    records per launch (traffic grows linearly with the records)."""
-    p = os.path.join(ROOT, "profiles", "record_scatter_%dB.txt" % item_bytes)
-    try:
-        vals = {}
-        for ln in open(p):
-            if ":" in ln:
-                k, v = ln.split(":", 1)
-                vals[k.strip()] = v.strip().split()[0]
-        per_rec = float(vals["dram_bytes_per_record"])
-        return per_rec * n
-    except Exception:
+# ncu summaries of a distribution level and of a radix pass, by record width
+PROFILES = {("scatter_kernel", 8): "record_scatter_8B.txt",
+            ("onesweep_kernel", 12): "radix_onesweep_pass_12B.txt"}
+
+
+def profiled_traffic(kernel, n, item_bytes):
+    """DRAM bytes per launch from the committed ncu summary for this kernel and
+    record width (captured on inputs of 4x L2), scaled by records per launch
+    (traffic grows linearly with the records); None where no summary is held."""
+    name = PROFILES.get((kernel, item_bytes))
+    if name is None:
         return None
+    with open(os.path.join(ROOT, "profiles", name)) as f:
+        for ln in f:
+            if ln.startswith("dram_bytes_per_record:"):
+                return float(ln.split()[1]) * n
+    return None
+
+
+def sort_roofline(n, steps):
+    """The record sort's passes of the timed steps (their stats) against the
+    copy peak: a distribution level, or a radix pass where keys are skewed.  A
+    pass over the n suffix records reads and writes each once (8 B when the
+    position is packed below the key, else a u64 key + a u32 position).  None
+    where no pass ran (texts that one block sorts)."""
+    passes = sum(st["timed_passes"] for st in steps)
+    if not passes:
+        return None
+    item_bytes = steps[-1]["sort_item_bytes"]
+    levels = steps[-1]["timed_passes"] < steps[-1]["sort_passes"]
+    kernel = "scatter_kernel" if levels else "onesweep_kernel"
+    what = "one distribution level" if levels else "one radix pass"
+    peak, peak_kind = hbm_peak()
+    avg_ms = sum(st["sort_pass_ms"] for st in steps) / passes
+    alg_bytes = 2.0 * item_bytes * n
+    achieved = alg_bytes / (avg_ms / 1e3) / 1e9
+    phases = ("keys_ms", "sort_ms", "refine_ms", "finish_ms")
+    return {"kernel": "%s (%s of the %d-byte suffix records)" % (kernel, what, item_bytes),
+            "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
+            "frac": achieved / peak, "peak_kind": peak_kind,
+            "traffic": profiled_traffic(kernel, n, item_bytes),
+            "algorithmic_bytes_per_launch": alg_bytes, "avg_launch_ms": avg_ms,
+            "launches_per_step": passes / len(steps),
+            "phase_ms": {k: sum(st[k] for st in steps) / len(steps) for k in phases},
+            "refine_rounds": steps[-1]["refine_rounds"]}
 
 
 # ------------------------------------------------------------------ CPU baseline
@@ -462,21 +492,11 @@ def run_ours(args):
     torch.cuda.synchronize()
     ev0 = torch.cuda.Event(enable_timing=True)
     ev1 = torch.cuda.Event(enable_timing=True)
-    launches = 0
-    pass_ms, passes, phase = [], [], {"keys_ms": 0, "sort_ms": 0, "refine_ms": 0, "finish_ms": 0}
-    item_bytes = 12
-    rounds = 0
+    step_stats = []
     ev0.record(stream)
     for _ in range(args.steps):
         ctx.build_in_memory(t_dev, out=sa_dev)
-        st = ctx.stats()
-        launches += st["kernel_launches"]
-        pass_ms.append(st["sort_pass_ms"])
-        passes.append(st["sort_passes"] - 1)  # without the sort inside the blocks
-        item_bytes = st["sort_item_bytes"] or 12
-        rounds = st["refine_rounds"]
-        for k in phase:
-            phase[k] += st[k] / args.steps
+        step_stats.append(ctx.stats())
     ev1.record(stream)
     torch.cuda.synchronize()
     if dist is not None:
@@ -487,21 +507,8 @@ def run_ours(args):
     ms_per_step = elapsed_ms / args.steps
     value = job_throughput(n, ws, args.steps, elapsed_ms / 1e3)
 
-    # roofline of the record sort's distribution kernel: one level over the n
-    # suffix records reads and writes each record once (8 B when the
-    # position is packed below the key, else a u64 key + a u32 position)
-    peak, peak_kind = hbm_peak()
-    avg_pass_ms = sum(pass_ms) / max(1, sum(passes))
-    alg_bytes = 2.0 * item_bytes * n
-    achieved = alg_bytes / (avg_pass_ms / 1e3) / 1e9
-    traffic = profiled_traffic(n, item_bytes)
-    roofline = {"kernel": "scatter_kernel (one distribution level of the %d-byte suffix records)"
-                % item_bytes, "bound": "hbm",
-                "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                "peak_kind": peak_kind, "traffic": traffic,
-                "algorithmic_bytes_per_launch": alg_bytes, "avg_launch_ms": avg_pass_ms,
-                "launches_per_step": sum(passes) / len(passes),
-                "phase_ms": phase, "refine_rounds": rounds}
+    launches = sum(st["kernel_launches"] for st in step_stats)
+    roofline = sort_roofline(n, step_stats)
 
     e2e = None
     if not args.no_e2e:

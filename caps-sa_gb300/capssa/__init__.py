@@ -124,7 +124,7 @@ class _Stats(C.Structure):
                 ("train_ms", C.c_double), ("partition_probes", C.c_uint64),
                 ("train_samples", C.c_uint32), ("model_loss", C.c_float),
                 ("radix_items", C.c_uint32), ("sparse_subset", C.c_uint32),
-                ("tie_classes", C.c_uint32), ("reserved_u32", C.c_uint32),
+                ("tie_classes", C.c_uint32), ("timed_passes", C.c_uint32),
                 ("tie_order_ms", C.c_double)]
 
 

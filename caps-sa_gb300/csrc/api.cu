@@ -374,7 +374,8 @@ struct CallScope {
             c.stats.sort_ms = ms(c.pev[1], c.pev[2]);
             c.stats.refine_ms = ms(c.pev[2], c.pev[3]);
             c.stats.sort_pass_ms = 0;
-            for (int i = 0; i < c.timed_passes && i < 16; i++)
+            c.stats.timed_passes = (uint32_t)std::min(c.timed_passes, 16);
+            for (int i = 0; i < (int)c.stats.timed_passes; i++)
                 c.stats.sort_pass_ms += ms(c.kev[2 * i], c.kev[2 * i + 1]);
         }
         if (c.timed_finish) c.stats.finish_ms = ms(c.pev[4], c.pev[5]);

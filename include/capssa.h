@@ -171,7 +171,9 @@ typedef struct capssa_stats {
                                    first large sort) */
     uint32_t sparse_subset;     /* 1: a subset build sorted only its own positions */
     uint32_t tie_classes;       /* tie classes of the output (CAPSSA_TIES_REFERENCE) */
-    uint32_t reserved_u32;
+    uint32_t timed_passes;      /* kernels that sort_pass_ms adds up: all sort_passes of a radix
+                                   sort, one fewer of a distribution (its last step sorts
+                                   inside the blocks), 0 where neither ran */
     double tie_order_ms;        /* device time of the reference tie order */
 } capssa_stats;
 

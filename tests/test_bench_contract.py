@@ -57,3 +57,29 @@ def test_reference_arm_other_ranks_exit_without_work():
     lines, status = _run({"RANK": "1", "LOCAL_RANK": "1", "WORLD_SIZE": "2"})
     assert status["rc"] == 0
     assert lines == []
+
+
+def _step(**over):
+    st = {"timed_passes": 2, "sort_passes": 3, "sort_item_bytes": 8, "sort_pass_ms": 2.0,
+          "keys_ms": 0.5, "sort_ms": 5.0, "refine_ms": 4.0, "finish_ms": 0.1, "refine_rounds": 2}
+    st.update(over)
+    return st
+
+
+def test_roofline_of_the_sort_that_ran():
+    """Distribution levels, radix passes, and builds in which no pass ran."""
+    import bench
+    n = 1 << 20
+    r = bench.sort_roofline(n, [_step(), _step(sort_pass_ms=4.0)])
+    assert r["kernel"].startswith("scatter_kernel") and r["launches_per_step"] == 2
+    assert r["avg_launch_ms"] == 1.5
+    assert abs(r["achieved"] - 16.0 * n / 1.5e-3 / 1e9) < 1e-6
+    assert r["traffic"] > 14 * n and r["phase_ms"]["sort_ms"] == 5.0
+    r = bench.sort_roofline(n, [_step(timed_passes=6, sort_passes=6, sort_item_bytes=12)])
+    assert r["kernel"].startswith("onesweep_kernel") and r["launches_per_step"] == 6
+    assert r["algorithmic_bytes_per_launch"] == 24 * n and r["traffic"] > 24 * n
+    assert bench.sort_roofline(n, [_step(sort_item_bytes=12)])["traffic"] is None
+    small = _step(timed_passes=0, sort_passes=0, sort_item_bytes=0, sort_pass_ms=0.0)
+    assert bench.sort_roofline(4096, [small]) is None
+    inside = _step(timed_passes=0, sort_passes=1, sort_pass_ms=0.0)
+    assert bench.sort_roofline(2000, [inside]) is None
