@@ -144,7 +144,8 @@ __global__ void __launch_bounds__(256)
 }
 
 __global__ void __launch_bounds__(256) iota_kernel(uint32_t *__restrict__ out, uint32_t n) {
-    for (uint32_t i = blockIdx.x * 256 + threadIdx.x; i < n; i += gridDim.x * 256) out[i] = i;
+    for (uint64_t i = blockIdx.x * 256ull + threadIdx.x; i < n; i += gridDim.x * 256ull)
+        out[i] = (uint32_t)i;
 }
 
 // One tile of a range at a time: ranks by digit in shared memory, a place in
@@ -170,7 +171,7 @@ __global__ void __launch_bounds__(kThreads, 2)
     __shared__ uint32_t s_w[kThreads / 32];
     const uint32_t R = 1u << dg.bits;
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const uint32_t nt = tiles ? ctr->tiles : (n + T - 1) / T;
+    const uint32_t nt = tiles ? ctr->tiles : pieces_of(n, T);
     for (uint32_t t = blockIdx.x; t < nt; t += gridDim.x) {
         Tile tl;
         if (tiles) {
@@ -283,7 +284,7 @@ __global__ void __launch_bounds__(256)
             const uint32_t len = end - start;
             if (last) {
                 // one key: a run entry and its pieces, or pieces to sort alone
-                const uint32_t nc = (len + kChunk - 1) / kChunk;
+                const uint32_t nc = pieces_of(len, kChunk);
                 uint32_t at = atomicAdd(n_chunks, nc + (runs ? 1 : 0));
                 if (runs) chunks[at++] = make_uint4(start, in_b, len, kRunWhole);
                 for (uint32_t q = 0; q < nc; q++)
@@ -291,7 +292,7 @@ __global__ void __launch_bounds__(256)
                         make_uint4(start + q * kChunk, min(kChunk, len - q * kChunk) | in_b,
                                    runs ? start : d, runs ? kRunPiece : chunk_key(1, dg));
             } else {
-                const uint32_t nt = (len + tile_recs - 1) / tile_recs;
+                const uint32_t nt = pieces_of(len, tile_recs);
                 const uint32_t id = atomicAdd(&next->ranges, 1u);
                 const uint32_t at = atomicAdd(&next->tiles, nt);
                 next_ranges[id] = Range{start, len};

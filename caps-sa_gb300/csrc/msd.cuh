@@ -64,6 +64,11 @@ struct Chunks {
 // first index, kRunPiece) and one (start, kInB or 0, run length, kRunWhole).
 constexpr uint32_t kRunPiece = 0x80000000u, kRunWhole = 0xC0000000u;
 
+// Pieces of at most `per` in n (up to the largest n: n + per - 1 would wrap).
+__host__ __device__ __forceinline__ uint32_t pieces_of(uint32_t n, uint32_t per) {
+    return n / per + (n % per ? 1u : 0u);
+}
+
 struct Digit {  // `bits` bits at `shift` of the key, or of the position
     int shift, bits, from_val;
 };

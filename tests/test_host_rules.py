@@ -39,6 +39,15 @@ int main() {
                 std::printf("%s[%llu, %llu, %d, %d]", sep, n, r, want, msd::level_bits(n, r, want));
                 sep = ", ";
             }
+    // pieces: n, at most this many in each -> pieces
+    std::printf("], \"pieces\": [");
+    sep = "";
+    for (unsigned per : {1u, 2560u, 6144u, 8192u})
+        for (unsigned n : {1u, 2559u, 2560u, 2561u, 8192u, 8193u, 4294959104u, 4294959105u,
+                           4294961152u, 4294964736u, 4294967294u, 4294967295u}) {
+            std::printf("%s[%u, %u, %u]", sep, n, per, msd::pieces_of(n, per));
+            sep = ", ";
+        }
     std::printf("]}\n");
     return 0;
 }
@@ -77,3 +86,9 @@ def test_bins_of_a_level_stay_within_a_byte_a_record(rules):
         assert got >= min(want, 8)
         assert ranges << got <= most
         assert got == want or ranges << (got + 1) > most
+
+
+def test_pieces_of_the_largest_counts(rules):
+    """Up to 2^32 - 1 records: none are lost to a wrapped sum."""
+    for n, per, got in rules["pieces"]:
+        assert got == -(-n // per)
