@@ -1594,8 +1594,10 @@ __global__ void gather_big_kernel(const BigGroup *__restrict__ groups, uint32_t 
                                   const uint32_t *__restrict__ rank, DevLimits L, uint64_t h,
                                   int lf, uint64_t empty_lf, int k2bits, RunKeys R,
                                   uint64_t *__restrict__ tkeys, uint32_t *__restrict__ tvals) {
-    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < total;
-         t += gridDim.x * blockDim.x) {
+    // (64-bit strides: past 2^31 members a 32-bit one would wrap and visit some twice)
+    for (uint64_t t64 = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t64 < total;
+         t64 += (uint64_t)gridDim.x * blockDim.x) {
+        const uint32_t t = (uint32_t)t64;
         uint32_t lo = 0, hi = nb;  // last group with toff <= t
         while (hi - lo > 1) {
             const uint32_t mid = (lo + hi) >> 1;
@@ -2780,8 +2782,10 @@ __global__ void split_big_kernel(const uint64_t *__restrict__ tkeys,
                                  uint32_t *__restrict__ rank, int lf,
                                  uint64_t empty, uint64_t h, GroupLists G, int nxt) {
     const uint64_t k2mask = (k2bits >= 64) ? ~0ull : ((1ull << k2bits) - 1);
-    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < total;
-         t += gridDim.x * blockDim.x) {
+    // (64-bit strides: past 2^31 members a 32-bit one would wrap and visit some twice)
+    for (uint64_t t64 = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t64 < total;
+         t64 += (uint64_t)gridDim.x * blockDim.x) {
+        const uint32_t t = (uint32_t)t64;
         uint64_t key = tkeys[t];
         uint32_t ord = (uint32_t)(key >> ord_shift);
         if (ord >= n_groups) continue;  // unreachable unless a sort step failed (flagged)
