@@ -3914,9 +3914,10 @@ capssa_status core_sort(Ctx &c, const EngineArgs &a, uint32_t **sa_out, eng::Pac
     // and 6.0 ms.
     const bool use_msd = N <= msd::kOneBlock || entropy >= 0.9 * b;
     // short suffixes of the flagless geometry; the MSD sort, whose levels do
-    // not depend on the key's width, takes them along with a flag bit
+    // not depend on the key's width, takes them along with a flag bit (there is
+    // always room: the key without it saves a whole radix pass)
     const uint64_t n_short = geo.flagless ? (uint64_t)geo.k - 1 : 0;
-    const bool flag_short = geo.flagless && use_msd && geo.total + 1 + geo.vbits <= 64;
+    const bool flag_short = geo.flagless && use_msd;
     if (flag_short) {
         geo.lbits = geo.flag_len = 1;
         geo.total++;
@@ -4088,9 +4089,8 @@ capssa_status core_sort(Ctx &c, const EngineArgs &a, uint32_t **sa_out, eng::Pac
         c.stats.radix_items = msd::records_per_thread(false);
     } else if (use_msd) {
         s = msd::sort(c, plan, keys_a, vbits ? nullptr : vals_a, keys_b, vbits ? nullptr : vals_b,
-                      (uint32_t)n_rec, vbits, sort_bits, bits_for(n - 1),
-                      geo.flag_len == 0 || geo.flag_len == 3, !sp,
-                      counts, given, &passes);
+                      (uint32_t)n_rec, vbits, sort_bits, bits_for(n - 1), !sp, counts, given,
+                      &passes);
         c.stats.radix_items = msd::records_per_thread(vbits == 0);
     } else {
         s = vbits ? radix::sort_keys(c, keys_a, keys_b, (uint32_t)n_rec, vbits, vbits + sort_bits,

@@ -745,16 +745,16 @@ uint32_t *count_buffer(Ctx &c) {
 }
 
 capssa_status sort(Ctx &c, const Plan &pl, uint64_t *ka, uint32_t *va, uint64_t *kb, uint32_t *vb,
-                   uint32_t n, int low, int nbits, int pos_bits, bool pos_order, bool gen_vals,
+                   uint32_t n, int low, int nbits, int pos_bits, bool gen_vals,
                    uint32_t *counts, const Pieces &given, int *levels_out) {
     if (n == 0) {
         *levels_out = 0;
         return CAPSSA_OK;
     }
-    return va ? run<true>(c, pl, ka, va, kb, vb, n, low, nbits, pos_bits, pos_order, gen_vals,
-                          counts, given, levels_out, nullptr)
-              : run<false>(c, pl, ka, nullptr, kb, nullptr, n, low, nbits, pos_bits, pos_order,
-                           false, counts, given, levels_out, nullptr);
+    return va ? run<true>(c, pl, ka, va, kb, vb, n, low, nbits, pos_bits, /*pos_order=*/true,
+                          gen_vals, counts, given, levels_out, nullptr)
+              : run<false>(c, pl, ka, nullptr, kb, nullptr, n, low, nbits, pos_bits,
+                           /*pos_order=*/true, false, counts, given, levels_out, nullptr);
 }
 
 capssa_status distribute(Ctx &c, const Plan &pl, uint64_t *ka, uint64_t *kb, uint32_t n, int low,

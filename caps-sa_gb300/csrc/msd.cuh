@@ -118,13 +118,11 @@ capssa_status distribute(Ctx &c, const Plan &pl, uint64_t *ka, uint64_t *kb, uin
 // position.  vals null: each u64 record carries its position in the low bits
 // (the whole record is the order).  Otherwise u64 keys with u32 positions.
 // Records in (ka, va), scratch (kb, vb); sorted into (ka, va).  counts: the
-// 2^bits[0] digit counts of level 0 (device; overwritten).  pos_order false:
-// the order of equal keys is left open (it is then whatever is cheapest).
-// gen_vals: the input values are not read, value i is i.  levels_out: planned
-// levels run.
+// 2^bits[0] digit counts of level 0 (device; overwritten).  gen_vals: the input
+// values are not read, value i is i.  levels_out: planned levels run.
 capssa_status sort(Ctx &c, const Plan &pl, uint64_t *ka, uint32_t *va, uint64_t *kb, uint32_t *vb,
-                   uint32_t n, int low, int nbits, int pos_bits, bool pos_order,
-                   bool gen_vals, uint32_t *counts, const Pieces &given, int *levels_out);
+                   uint32_t n, int low, int nbits, int pos_bits, bool gen_vals,
+                   uint32_t *counts, const Pieces &given, int *levels_out);
 
 // Records a thread handles in a distribution tile (stats.radix_items).
 constexpr uint32_t records_per_thread(bool pairs) { return pairs ? 12u : 16u; }
