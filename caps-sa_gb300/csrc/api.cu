@@ -76,7 +76,7 @@ capssa_status check_dev_flags(Ctx &c) {
     CAPSSA_CUDA(c, cudaMemcpyAsync(flags_readback(c), c.d_flags, 4, cudaMemcpyDeviceToHost,
                                    c.stream));
     CAPSSA_CUDA(c, cudaStreamSynchronize(c.stream));
-    c.flags_read_at = c.launches;
+    c.flags_due = false;
     return flags_status(c);
 }
 
@@ -344,7 +344,7 @@ struct CallScope {
         c.timed_passes = -1;
         c.timed_finish = false;
         c.waited = false;
-        c.flags_read_at = ~0ull;
+        c.flags_due = false;
         cudaSetDevice(c.device);
         cudaMemsetAsync(c.d_flags, 0, 16, c.stream);
         cudaEventRecord(c.ev0, c.stream);
@@ -387,9 +387,9 @@ struct CallScope {
 };
 
 // Nothing reaches the host from a call whose device waits failed: the flags
-// are read before the first copy, and again where kernels ran since.
+// are read before the first copy, and again where kernels that wait ran since.
 capssa_status flags_before_host(Ctx &c) {
-    return c.flags_read_at == c.launches ? CAPSSA_OK : check_dev_flags(c);
+    return c.flags_due ? check_dev_flags(c) : CAPSSA_OK;
 }
 
 // Deliver a device result to a host or device destination.
@@ -489,7 +489,6 @@ capssa_status build_common(Ctx &c, const ST *text, uint64_t n, const void *posit
         if (done) {
             c.stats.n_suffixes = n;
             c.waited = true;
-            c.flags_read_at = c.launches;  // none of its launches waits
             return out_dev ? CAPSSA_OK : stage_out(c, out_sa, d_out, count * (size_t)out_bytes);
         }
     }
@@ -1298,7 +1297,7 @@ capssa_status capssa_selftest_bounded_wait(capssa_ctx *ctx, uint32_t polls) {
     if (!word) return scope.finish(set_err(c, CAPSSA_ENOMEM, "self-test word"));
     if (cudaMemsetAsync(word, 0, 64, c.stream) != cudaSuccess)
         return scope.finish(set_err(c, CAPSSA_ECUDA, "self-test word clear"));
-    bounded_wait_kernel<<<1, 32, 0, c.stream>>>(word, polls, c.d_flags);
+    bounded_wait_kernel<<<1, 32, 0, c.stream>>>(word, polls, error_flag(c));
     c.launches++;
     // (a delivery after the wait: refused, so no bytes reach the host)
     unsigned long long got = 0;

@@ -153,8 +153,8 @@ struct Ctx {
     // the call's last kernel has been waited for, ev1 recorded after it (a small
     // text, which sets no device flags)
     bool waited = false;
-    // launches when the device flags were last read (see stage_out)
-    uint64_t flags_read_at = ~0ull;
+    // a kernel that may set the error flag was launched since it was last read
+    bool flags_due = false;
     // the last sort produced segment-major order (every segment contiguous)
     bool seg_major_done = false;
     uint64_t *h_emit = nullptr;     // pinned double buffer of the emit stream
@@ -196,6 +196,12 @@ constexpr size_t kScratchBytes = 1 << 16;
 inline bool kernels_reach(const cudaPointerAttributes &attr, int device) {
     return attr.type == cudaMemoryTypeManaged ||
            (attr.type == cudaMemoryTypeDevice && attr.device == device);
+}
+
+// The error flag, for the launch of a kernel that may set it.
+inline int *error_flag(Ctx &c) {
+    c.flags_due = true;
+    return c.d_flags;
 }
 
 // Device flag check: returns CAPSSA_ETIMEOUT / CAPSSA_ENOMEM after a sync.

@@ -291,7 +291,7 @@ void launch_words(Ctx &c, const uint64_t *ki, const uint32_t *vi, uint64_t *ko, 
                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     const unsigned tiles = ((uint64_t)n + kThreads * IT - 1) / (kThreads * IT);
     onesweep_kernel<MODE, IT, W><<<tiles, kThreads, sm, c.stream>>>(
-        ki, vi, ko, vo, n, shift, offsets, (W *)status, tile_counter, c.d_flags, val_base);
+        ki, vi, ko, vo, n, shift, offsets, (W *)status, tile_counter, error_flag(c), val_base);
 }
 
 template <int MODE, int IT>

@@ -326,10 +326,10 @@ capssa_status select_bits(Ctx &c, const uint32_t *sa, uint64_t n, const uint32_t
     CAPSSA_CUDA(c, cudaMemsetAsync(status, 0, tiles * 8 + 64, c.stream));
     if (out_bytes == 8)
         select_kernel<uint64_t><<<(unsigned)tiles, kScanThreads, 0, c.stream>>>(
-            sa, n, bits, off, (uint64_t *)out, status, counter, c.d_flags);
+            sa, n, bits, off, (uint64_t *)out, status, counter, error_flag(c));
     else
         select_kernel<uint32_t><<<(unsigned)tiles, kScanThreads, 0, c.stream>>>(
-            sa, n, bits, off, (uint32_t *)out, status, counter, c.d_flags);
+            sa, n, bits, off, (uint32_t *)out, status, counter, error_flag(c));
     CAPSSA_LAUNCHED(c);
     return CAPSSA_OK;
 }
@@ -345,16 +345,16 @@ capssa_status scan_u32(Ctx &c, const uint32_t *in, uint32_t *out, uint64_t n, bo
     CAPSSA_CUDA(c, cudaMemsetAsync(status, 0, tiles * 8 + 64, c.stream));
     if (max_op && inclusive)
         scan_kernel<true, true><<<(unsigned)tiles, kScanThreads, 0, c.stream>>>(in, out, n, status,
-                                                                               counter, c.d_flags);
+                                                                               counter, error_flag(c));
     else if (max_op)
         scan_kernel<true, false><<<(unsigned)tiles, kScanThreads, 0, c.stream>>>(
-            in, out, n, status, counter, c.d_flags);
+            in, out, n, status, counter, error_flag(c));
     else if (inclusive)
         scan_kernel<false, true><<<(unsigned)tiles, kScanThreads, 0, c.stream>>>(
-            in, out, n, status, counter, c.d_flags);
+            in, out, n, status, counter, error_flag(c));
     else
         scan_kernel<false, false><<<(unsigned)tiles, kScanThreads, 0, c.stream>>>(
-            in, out, n, status, counter, c.d_flags);
+            in, out, n, status, counter, error_flag(c));
     CAPSSA_LAUNCHED(c);
     return CAPSSA_OK;
 }

@@ -634,7 +634,7 @@ capssa_status reference_tie_order(Ctx &c, const TieArgs &t) {
     const unsigned gS = grid_for(S, 256);
     resolve_kernel<<<gS, 256, 0, c.stream>>>(K, S, slo, shi, pred, idxf, start, dep);
     CAPSSA_LAUNCHED(c);
-    chase_kernel<<<gS, 256, 0, c.stream>>>(S, dep, start, c.d_flags);
+    chase_kernel<<<gS, 256, 0, c.stream>>>(S, dep, start, error_flag(c));
     CAPSSA_LAUNCHED(c);
     if (t.out_bytes == 8)
         place_kernel<uint64_t><<<gM, 256, 0, c.stream>>>(K, start, melem, (uint64_t *)t.out);
