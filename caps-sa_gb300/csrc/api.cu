@@ -618,8 +618,8 @@ capssa_status sample_sort_common(Ctx &c, const ST *text, uint64_t n, const uint6
 
 // build_ext_mem* (src/ext_mem.rs:279-553): the same suffix order streamed
 // to `emit`.  The reference spills partition buckets to temp files to bound
-// host RAM; here the whole working set (under 50 bytes per suffix, so under
-// 200 GB for the largest supported text) lives in device memory and the
+// host RAM; here the whole working set (about 100 bytes per suffix, so
+// texts of about 2.5 G symbols) lives in device memory and the
 // host holds only the text and the two emit batches, so there is nothing
 // to spill and no partition plan to compute.
 template <typename ST>

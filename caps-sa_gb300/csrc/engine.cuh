@@ -14,7 +14,12 @@
 //     out of the sort and placed afterwards); the position rides below the
 //     key when it fits, and a segment index above it in segment-major order.
 //     Key order never contradicts suffix_cmp_with (src/lcp.rs:184-201);
-//  3. stable LSD radix sort of the records;
+//  3. the records sorted: distribution by leading digits (msd.cuh) for spread
+//     symbols, stable LSD radix passes (radix.cuh) for skewed ones.  The
+//     distribution is not stable: where suffixes can tie completely (length
+//     field or padding codes) it orders the position bits too; with a flag,
+//     where they cannot, its last step leaves tied groups in any order and
+//     finds them on the way (finish_chunks_kernel);
 //  4. the groups still tied are resolved by size class: direct comparison
 //     on a bit-packed copy of the text for groups of up to 2048 members and
 //     depths up to 4096 symbols, rank doubling for the rest (a suffix p of
@@ -25,7 +30,7 @@
 // Boundary orders: ShorterFirst (the default boundary_order) leaves suffixes
 // that end together with equal content tied; their output order is
 // ascending position.  LongerFirst (STAR) orders them by position, which the
-// stable sorts produce directly.
+// record sorts produce directly.
 #pragma once
 
 #include "common.cuh"
@@ -33,7 +38,8 @@
 namespace capssa {
 
 struct EngineArgs {
-    const void *text;      // device, padded with >= 64 zero bytes
+    const void *text;      // device, padded with >= 64 zero bytes unless it is the
+                           // caller's own buffer (see build_common)
     int sym_bytes;         // 1, 2, 4
     uint64_t n;
     DevLimits lim;

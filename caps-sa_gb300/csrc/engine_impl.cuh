@@ -3907,11 +3907,17 @@ capssa_status core_sort(Ctx &c, const EngineArgs &a, uint32_t **sa_out, eng::Pac
     const uint64_t N = sp ? sp->m : n;
     // Distribution by leading digits (msd.cuh) for spread keys, stable LSD
     // passes (radix.cuh) for skewed ones, whose leading digits hold little of
-    // their information and leave long pieces level after level: at an
-    // entropy of 0.64 of the code width (a word text, 50 M records of 12
-    // bytes) the MSD levels took 7.7 ms and the LSD passes 3.2 ms, at 0.7 (a
-    // masked genome, 134 M) 7.3 and 7.2 ms, at 1 (DNA, 268 M of 8 bytes) 4.5
-    // and 6.0 ms.
+    // their information and leave long pieces level after level.  The line lies
+    // where four symbols cross, at either record width (whole builds, LSD / MSD
+    // in ms, by the entropy as a share of the code width):
+    //                                 0.75         0.88         0.92         1
+    //   268 M of 4 symbols, 8 B   14.4 / 25.7  12.3 / 12.8  12.1 / 11.1   8.0 / 6.6
+    //   629 M of 4 symbols, 12 B  34.3 / 61.3  29.0 / 31.9  28.1 / 28.0  27.6 / 22.4
+    //   67 M in segments, 8 B      4.6 /  7.7   3.7 /  3.9   3.7 /  3.5   3.0 / 2.4
+    //   67 M of 256 values, 12 B   4.2 /  4.0   4.2 /  2.9   4.2 /  2.8   4.2 / 2.2
+    //   16 M of 32,768, 12 B       1.3 /  1.1   1.5 /  1.0   1.5 /  1.0   1.5 / 0.8
+    // Wide alphabets of independent symbols cross earlier, real ones do not: 50 M
+    // word bytes (0.64) take 13.5 and 17.0 ms, 8 M tokens 1.36 and 1.60.
     const bool use_msd = N <= msd::kOneBlock || entropy >= 0.9 * b;
     // short suffixes of the flagless geometry; the MSD sort, whose levels do
     // not depend on the key's width, takes them along with a flag bit (there is
@@ -3929,7 +3935,7 @@ capssa_status core_sort(Ctx &c, const EngineArgs &a, uint32_t **sa_out, eng::Pac
     c.stats.key_symbols = geo.k;
     c.stats.key_bits_per_symbol = geo.b;
 
-    // ---- 2+3. composite keys of every position, stable radix sort
+    // ---- 2+3. composite keys of every position, record sort
     const uint32_t nn = (uint32_t)N;
     uint64_t *keys_a = (uint64_t *)ws_get(c, WS_KEYS_A, (size_t)N * 8);
     uint64_t *keys_b = (uint64_t *)ws_get(c, WS_KEYS_B, (size_t)N * 8);
@@ -4694,7 +4700,7 @@ inline capssa_status pf_report(Ctx &c, const EngineArgs &a, const PfRun &pf) {
 
 // Subsets far smaller than the text (m * kSparseRatio <= n) are sorted on
 // their own: the distinct chosen positions become records of their own and
-// go through the same radix sort and refinement, so the work is O(m) plus
+// go through the same record sort and refinement, so the work is O(m) plus
 // one n / 8-byte bitmap.  Repeated positions, deep ties (a group needing
 // rank doubling) or any other case leave *res null and the caller sorts the
 // whole text instead.  On success *res holds the m positions in order (the
@@ -4737,8 +4743,9 @@ capssa_status sparse_subset(Ctx &c, const EngineArgs &a, const uint32_t **res,
     }
     const uint64_t count = m - n_empty;  // chosen positions below n
     if (count == 0) return CAPSSA_OK;
-    // the chosen positions, ascending (a stable sort then keeps every tie
-    // class in ascending position, as the whole-text path does)
+    // the chosen positions, ascending (the stable passes then keep every tie
+    // class in that order, and the distribution orders the position bits where
+    // there can be one, as on the whole-text path)
     uint32_t *wc = (uint32_t *)ws_get(c, WS_MISC, nw * 4 + 64);
     uint32_t *pos = (uint32_t *)ws_get(c, WS_MISC2, count * 4 + 64);
     if (!wc || !pos) return set_err(c, CAPSSA_ENOMEM, "subset positions");

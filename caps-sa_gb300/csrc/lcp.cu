@@ -1,5 +1,6 @@
-// lcp.cu — LCP-based kernels: batched LcpDispatch::lcp / suffix_cmp_with, the bounded-context run flags, and the merge-path
-// version of the reference's LCP-enhanced two-way merge.
+// lcp.cu — LCP-based kernels: batched LcpDispatch::lcp / suffix_cmp_with, the
+// bounded-context run flags, and the merge-path version of the reference's
+// LCP-enhanced two-way merge.
 #include <algorithm>
 
 #include "lcp.cuh"

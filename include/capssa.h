@@ -148,7 +148,8 @@ typedef struct capssa_stats {
     uint64_t h2d_bytes;
     uint64_t d2h_bytes;
     /* device time per phase of the last suffix sort (CUDA events on the
-     * context's stream) */
+     * context's stream).  Plain texts of up to 8,192 symbols that one block
+     * sorts have no phases: these and the key's and the sort's fields are 0 */
     double keys_ms;       /* alphabet scan + packed-key build */
     double sort_ms;       /* initial record sort: every pass, and the groups where its
                              last step finds them */
