@@ -4279,7 +4279,9 @@ capssa_status core_sort(Ctx &c, const EngineArgs &a, uint32_t **sa_out, eng::Pac
             // few groups, a block each at once: a round's launches and read-back
             // cost more than what ends earlier in shallower steps, so they go at
             // least as far as the other kernels do (1,000 symbols of period 3:
-            // 0.63 ms, 0.55 now; 8,000 skewed ones 0.57 and 0.51)
+            // 0.63 ms, 0.55 now; 8,000 skewed ones 0.57 and 0.51).  With 500
+            // groups the windows count: 60 copies of a 500-symbol text take 1.19 ms
+            // as it is, 1.44 with this reach
             const uint64_t reach = cnt[L_MEDIUM] <= (uint32_t)c.sm_count ? kDirectCap : 0;
             direct_medium_kernel<kSmallMax, kMedSmall, 128><<<mg, 128, 0, side()>>>(
                 G.list[L_MEDIUM][cur], cnt[L_MEDIUM], sa, hd, rk, a.lim, P, lf, h, reach, G, nxt);

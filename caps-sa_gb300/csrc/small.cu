@@ -17,7 +17,7 @@
 // where the bins alone show it, else when the count passes kWork.  A bound of 384
 // windows for each thread, as before, let all of them run to it: 8,000 symbols in
 // two equal halves took 0.86 ms, twice the 0.40 of the general path they then
-// took, and 1,000 equal symbols 0.71 ms; 0.37 and 0.57 now.
+// took, and 1,000 equal symbols 0.71 ms; 0.37 and 0.52 now.
 #include "small.cuh"
 
 namespace capssa {
